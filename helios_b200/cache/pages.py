@@ -100,6 +100,7 @@ class RequestPages:
     # per group: first logical page still held behind the kept first pages (0: none given back yet)
     first_held: List[int] = field(default_factory=list)
     version: int = 0                                 # counts the changes of ``tables``
+    serial: int = 0                                  # which admission of the layout this is: ids come again
     arrays: dict = field(default_factory=dict)       # group -> (version, tables[group] as int32 array)
 
 
@@ -116,6 +117,7 @@ class CacheLayout:
         self.max_slots = max_slots
         self.watermark = watermark
         self._free_slots: Deque[int] = deque(range(max_slots))
+        self._admissions = 0
         self.requests: Dict[Hashable, RequestPages] = {}
 
     # ------------------------------------------------------------------ sizes
@@ -182,7 +184,9 @@ class CacheLayout:
             raise OutOfPages("no free request slot")
         slot = self._free_slots.popleft()
         n = len(self.groups)
-        self.requests[request_id] = RequestPages(slot, 0, [[] for _ in range(n)], [0] * n)
+        self._admissions += 1
+        self.requests[request_id] = RequestPages(slot, 0, [[] for _ in range(n)], [0] * n,
+                                                 serial=self._admissions)
         return slot
 
     def pages_needed(self, request_id: Hashable, n_new: int) -> List[int]:

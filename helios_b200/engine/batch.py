@@ -111,7 +111,8 @@ def _fill_decode(layout, entries, cache, pad_page, rows_kept, token_ids, positio
     """``fill_meta`` for a captured decode step (one token a request, one row a request): whole
     arrays at once instead of slices per request, and a block-table row is written again only
     when its request or that request's table has changed since this buffer was last filled
-    (``rows_kept``: row -> (request, table version)); with hundreds of requests the per-request
+    (``rows_kept``: row -> (admission, table version): an id that ended and was admitted again
+    is another request, whose table may have got to the same version); with hundreds of requests the per-request
     work of the general path costs more than the step."""
     S, n_real = layout.S, len(entries)
     requests = cache.requests
@@ -121,7 +122,7 @@ def _fill_decode(layout, entries, cache, pad_page, rows_kept, token_ids, positio
         lengths.append(req.length)
         slot_of.append(req.slot)
         seqs.append(SeqSlice(e.request_id, req.slot, req.length, 1, i))
-        key = (e.request_id, req.version)
+        key = (req.serial, req.version)
         if rows_kept.get(i) != key:
             rows_kept[i] = key
             for g, t in enumerate(tables):

@@ -137,3 +137,27 @@ def test_corruption_is_detected():
     lay.table("b", 0)[0] = lay.table("a", 0)[0]      # the same page in two tables
     with pytest.raises(CacheInvariantError):
         lay.check_invariants()
+
+
+def test_decode_rows_follow_an_id_that_was_admitted_again():
+    """A captured decode step keeps the block-table rows of its staging buffer from fill to fill;
+    a request that ended and came back under its old id has other pages at the same version."""
+    import numpy as np
+
+    from helios_b200.engine.batch import MetaLayout, StepEntry, fill_meta
+
+    layout = CacheLayout([GroupLayout(None, 12)], page_size=4, max_slots=2)
+    meta = MetaLayout(1, 1, 1, [4])
+    host, kept = np.zeros(meta.total, dtype=np.int32), {}
+    seen = []
+    for _ in range(2):
+        layout.admit("a")
+        layout.extend("a", 6)
+        layout.commit("a", 6)
+        layout.extend("a", 1)
+        fill_meta(meta, host, [StepEntry("a", (1,), (0,))], layout, [12], 4, rows_kept=kept)
+        row = meta.host_views(host)[8][:2].tolist()
+        assert row == layout.table("a", 0)
+        seen.append(row)
+        layout.release("a")
+    assert seen[0] != seen[1]
