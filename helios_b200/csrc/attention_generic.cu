@@ -1,4 +1,4 @@
-// Attention over the paged cache for any batch of tokens: one warp per
+// Attention over the paged cache for any batch of tokens: one block per
 // (token, query head).  It serves the float32 path and every size the tiled
 // bfloat16 kernels do not take.  A token at position p sees the keys at
 // positions lo..p of its own request, lo = max(0, p - window + 1) with a
@@ -15,10 +15,18 @@
 // of `pool` tokens behind the window (`pooled`: a key and a value a block in pages of their own,
 // block b seen if (b + 1) * pool <= p - window + 1); a constant `factor` on the output.
 //
-// Scores, softmax and the weighted sum are float32.  The keys are walked in
-// runs of 32 from `lo`, so the order of every sum depends on the token's
-// position alone: not on how the request was cut into steps, nor on the rest of
-// the batch.
+// Scores, softmax and the weighted sum are float32.  The keys are walked in runs of 32 from
+// `lo`; the runs are dealt to the block's eight warps in turn, and the warps' sums are merged
+// in order, so the order of every sum depends on the token's position alone: not on how the
+// request was cut into steps, nor on the rest of the batch.
+//
+// Bound by the latency of its loads: a decode step has a few dozen rows of some hundred keys.
+// So a row has a block of eight warps, and a run's loads are independent: eight lanes share a
+// key (four elements a lane and load, the key's dot product finished by three shuffles), a
+// warp's four groups of eight lanes walk eight keys of the run each, and values the same way.
+// In chains, 14 heads of 64 on 2 KV heads, float32, one warp a row with a key a lane / this:
+// 3 decode rows of 313 keys 132 / 8.1 µs, 24 of 1,000 420 / 29, one of 4,096 1,676 / 49;
+// prompts of 37, 128 and 301 tokens 345 / 99, one of 2,048 8,646 / 1,455.
 #include "common.cuh"
 
 // Keys and values that stand for whole blocks of tokens; all null / 0: none.
@@ -31,105 +39,195 @@ struct PooledPages {
   int pool;
 };
 
-constexpr int ATTN_WARPS = 4;
+constexpr int ATTN_WARPS = 8;
 constexpr int ATTN_MAX_HD = 256;
 
-template <typename T>
-__global__ void attention_generic_kernel(
+// four neighbouring elements of a row of `n`, as float; zeros behind its end
+template <typename T, bool VEC>
+__device__ __forceinline__ float4 load_four(const T* row, int d, int n) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (VEC) {
+    if (d < n) {
+      if constexpr (sizeof(T) == 4) {
+        v = *reinterpret_cast<const float4*>(row + d);
+      } else {
+        const uint2 raw = *reinterpret_cast<const uint2*>(row + d);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+        v = make_float4(a.x, a.y, b.x, b.y);
+      }
+    }
+  } else {
+    if (d < n) v.x = to_float(row[d]);
+    if (d + 1 < n) v.y = to_float(row[d + 1]);
+    if (d + 2 < n) v.z = to_float(row[d + 2]);
+    if (d + 3 < n) v.w = to_float(row[d + 3]);
+  }
+  return v;
+}
+
+// NJ: 32 * NJ >= hd, vd.  VEC: rows of keys and values are whole 4-element pieces.
+template <typename T, int NJ, bool VEC>
+__global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
     T* __restrict__ out, const T* __restrict__ q, int q_stride,
     const T* __restrict__ k_pages, const T* __restrict__ v_pages,
     const int* __restrict__ block_table, int bt_stride, const int* __restrict__ seq_of_token,
-    const int* __restrict__ positions, int n_rows, int nh, int nkv, int hd, int vd, int page_size,
+    const int* __restrict__ positions, int nh, int nkv, int hd, int vd, int page_size,
     int window, float scale, const float* __restrict__ slopes, int sink,
     const T* __restrict__ gate, int gate_stride, const float* __restrict__ bias_table, int bias_rows,
     const float* __restrict__ sink_values, int keep_first, int gate_wide, PooledPages<T> pooled,
     int out_stride, float factor) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float q_smem[ATTN_WARPS][ATTN_MAX_HD];
+  __shared__ float part_acc[ATTN_WARPS][32 * NJ];
+  __shared__ float part_m[ATTN_WARPS], part_l[ATTN_WARPS];
+  constexpr int KEYS = NJ <= 4 ? 8 / NJ : 1;         // keys a group has in flight: eight loads a lane
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * ATTN_WARPS + warp;
-  if (row >= n_rows) return;
-  const int t = row / nh, h = row - t * nh;
+  const int group = lane >> 3, gl = lane & 7;
+  const int t = blockIdx.x / nh, h = blockIdx.x - t * nh;
   const int kvh = h / (nh / nkv);
   const int pos = positions[t];
   const int* token_table = block_table + (size_t)seq_of_token[t] * bt_stride;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
 
-  float* qs = q_smem[warp];
+  // this lane's pieces of a row: elements 4 (8 j + gl) .. + 3
+  float4 qr[NJ], acc[NJ];
   const T* qrow = q + (size_t)t * q_stride + (size_t)h * hd;
-  for (int d = lane; d < hd; d += 32) qs[d] = to_float(qrow[d]);
-  __syncwarp();
-
-  constexpr int ND = ATTN_MAX_HD / 32;
-  float acc[ND];
 #pragma unroll
-  for (int i = 0; i < ND; ++i) acc[i] = 0.f;
+  for (int j = 0; j < NJ; ++j) {
+    qr[j] = load_four<T, false>(qrow, 4 * (8 * j + gl), hd);
+    acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   float m = -INFINITY, l = 0.f;
   const float slope = slopes ? slopes[h] : 0.f;
 
   // three stretches of keys: the means of the blocks behind the window, the first tokens a
   // window keeps (those it has passed), then the window itself; each in runs of 32 from its own
   // first key
+  int run = 0;                                         // runs of the row so far
   for (int stretch = pooled.pool > 0 ? -1 : 0; stretch < 2; ++stretch) {
     const int first = stretch <= 0 ? 0 : lo;
     const int last = stretch < 0 ? lo / pooled.pool - 1 : stretch == 0 ? min(keep_first, lo) - 1 : pos;
     const int* table = stretch < 0 ? pooled.table + (size_t)seq_of_token[t] * pooled.table_stride : token_table;
     const T* kp = stretch < 0 ? pooled.k : k_pages;
     const T* vp = stretch < 0 ? pooled.v : v_pages;
-    for (int base = first; base <= last; base += 32) {
+    const int runs = last >= first ? (last - first) / 32 + 1 : 0;
+    for (int r = (warp - run % ATTN_WARPS + ATTN_WARPS) % ATTN_WARPS; r < runs; r += ATTN_WARPS) {
+      const int base = first + 32 * r;
       const int key = base + lane;
       const bool valid = key <= last;
-      int page = 0;
+      // the key's place in the pages, in rows
+      size_t place = 0;
+      if (valid) place = ((size_t)table[key / page_size] * nkv + kvh) * page_size + key % page_size;
       float score = -INFINITY;
+#pragma unroll 1
+      for (int i0 = 0; i0 < 8; i0 += KEYS) {           // the group's keys 8 group + i
+        float4 kv[KEYS][NJ];
+#pragma unroll
+        for (int u = 0; u < KEYS; ++u) {
+          const size_t at = __shfl_sync(0xffffffffu, (unsigned long long)place, 8 * group + i0 + u);
+          const int n = base + 8 * group + i0 + u <= last ? hd : 0;
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) kv[u][j] = load_four<T, VEC>(kp + at * hd, 4 * (8 * j + gl), n);
+        }
+#pragma unroll
+        for (int u = 0; u < KEYS; ++u) {
+          float dot = 0.f;
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) {
+            dot = fmaf(qr[j].x, kv[u][j].x, dot);
+            dot = fmaf(qr[j].y, kv[u][j].y, dot);
+            dot = fmaf(qr[j].z, kv[u][j].z, dot);
+            dot = fmaf(qr[j].w, kv[u][j].w, dot);
+          }
+          dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+          dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+          dot += __shfl_xor_sync(0xffffffffu, dot, 4);
+          if (gl == i0 + u) score = dot;
+        }
+      }
       if (valid) {
-        page = table[key / page_size];
-        const T* kr = kp + (((size_t)page * nkv + kvh) * page_size + key % page_size) * hd;
-        float dot = 0.f;
-        for (int d = 0; d < hd; ++d) dot = fmaf(qs[d], to_float(kr[d]), dot);
-        score = dot * scale - slope * (float)(pos - key);
+        score = score * scale - slope * (float)(pos - key);
         if (bias_table) score += bias_table[(size_t)min(pos - key, bias_rows - 1) * nh + h];
+      } else {
+        score = -INFINITY;
       }
       const float m_new = fmaxf(m, warp_max(score));
-      const float p = valid ? expf(score - m_new) : 0.f;
+      const float p = score == -INFINITY ? 0.f : expf(score - m_new);
       const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
       l = l * corr + warp_sum(p);
       m = m_new;
 #pragma unroll
-      for (int i = 0; i < ND; ++i) acc[i] *= corr;
-      const int n_valid = min(32, last - base + 1);
-      for (int j = 0; j < n_valid; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, p, j);
-        const int pagej = __shfl_sync(0xffffffffu, page, j);
-        const T* vr = vp + (((size_t)pagej * nkv + kvh) * page_size + (base + j) % page_size) * vd;
+      for (int j = 0; j < NJ; ++j) {
+        acc[j].x *= corr;
+        acc[j].y *= corr;
+        acc[j].z *= corr;
+        acc[j].w *= corr;
+      }
+#pragma unroll 1
+      for (int i0 = 0; i0 < 8; i0 += KEYS) {
+        float4 kv[KEYS][NJ];
+        float pj[KEYS];
 #pragma unroll
-        for (int i = 0; i < ND; ++i) {
-          const int d = lane + 32 * i;
-          if (d < vd) acc[i] = fmaf(pj, to_float(vr[d]), acc[i]);
+        for (int u = 0; u < KEYS; ++u) {
+          const size_t at = __shfl_sync(0xffffffffu, (unsigned long long)place, 8 * group + i0 + u);
+          pj[u] = __shfl_sync(0xffffffffu, p, 8 * group + i0 + u);
+          const int n = base + 8 * group + i0 + u <= last ? vd : 0;
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) kv[u][j] = load_four<T, VEC>(vp + at * vd, 4 * (8 * j + gl), n);
         }
+#pragma unroll
+        for (int u = 0; u < KEYS; ++u)
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) {
+            acc[j].x = fmaf(pj[u], kv[u][j].x, acc[j].x);
+            acc[j].y = fmaf(pj[u], kv[u][j].y, acc[j].y);
+            acc[j].z = fmaf(pj[u], kv[u][j].z, acc[j].z);
+            acc[j].w = fmaf(pj[u], kv[u][j].w, acc[j].w);
+          }
       }
     }
+    run += runs;
+  }
+
+  // the four groups' sums, then the warps' in order
+  auto groups_sum = [](float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v + __shfl_xor_sync(0xffffffffu, v, 16);
+  };
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const float4 a = make_float4(groups_sum(acc[j].x), groups_sum(acc[j].y), groups_sum(acc[j].z), groups_sum(acc[j].w));
+    if (group == 0) *reinterpret_cast<float4*>(&part_acc[warp][4 * (8 * j + gl)]) = a;
+  }
+  if (lane == 0) { part_m[warp] = m; part_l[warp] = l; }
+  __syncthreads();
+  const int d = threadIdx.x;
+  if (d >= vd) return;
+  m = -INFINITY;
+#pragma unroll
+  for (int w = 0; w < ATTN_WARPS; ++w) m = fmaxf(m, part_m[w]);
+  l = 0.f;
+  float y = 0.f;
+#pragma unroll
+  for (int w = 0; w < ATTN_WARPS; ++w) {
+    if (w >= run) break;                               // the warps behind the last run have seen no key
+    const float f = part_m[w] == -INFINITY ? 0.f : expf(part_m[w] - m);
+    l = fmaf(part_l[w], f, l);
+    y = fmaf(part_acc[w][d], f, y);
   }
   if (sink) {                       // a key without a value: it adds exp(s - m) to the sum only (s = 0 unless given)
     const float sv = sink_values ? sink_values[h] : 0.f;
     const float m_new = fmaxf(m, sv);
     const float corr = expf(m - m_new);
     l = l * corr + expf(sv - m_new);
-#pragma unroll
-    for (int i = 0; i < ND; ++i) acc[i] *= corr;
+    y *= corr;
   }
   float inv = factor / l;
   if (gate && !gate_wide) inv /= 1.f + expf(-to_float(gate[(size_t)t * gate_stride + h]));
-  T* orow = out + (size_t)t * out_stride + (size_t)h * vd;
-#pragma unroll
-  for (int i = 0; i < ND; ++i) {
-    const int d = lane + 32 * i;
-    if (d < vd) {
-      float y = acc[i] * inv;
-      if (gate && gate_wide) y /= 1.f + expf(-to_float(gate[(size_t)t * gate_stride + (size_t)h * vd + d]));
-      orow[d] = from_float<T>(y);
-    }
-  }
+  y *= inv;
+  if (gate && gate_wide) y /= 1.f + expf(-to_float(gate[(size_t)t * gate_stride + (size_t)h * vd + d]));
+  out[(size_t)t * out_stride + (size_t)h * vd + d] = from_float<T>(y);
 }
 
 HB_EXPORT int hb_attention_generic(void* out, const void* q, int q_stride, const void* k_pages,
@@ -147,15 +245,25 @@ HB_EXPORT int hb_attention_generic(void* out, const void* q, int q_stride, const
       page_size <= 0 || keep_first < 0 || pool < 0 || out_stride < nh * vd ||
       (pool > 0 && (window <= 0 || !pooled_k || !pooled_v || !pooled_table)) || (bias_table != nullptr && bias_rows <= 0))
     return HB_BAD_ARGUMENT;
-  const int n_rows = T * nh;
-  const int blocks = (n_rows + ATTN_WARPS - 1) / ATTN_WARPS;
+  if ((long)T * nh > 0x7fffffffL) return HB_BAD_ARGUMENT;
+  const int most = hd > vd ? hd : vd;
+#define HB_GENERIC_LAUNCH(NJ, VEC)                                                                             \
+    hb_launch(attention_generic_kernel<TA, NJ, VEC>, dim3((unsigned)(T * nh)), dim3(ATTN_WARPS * 32), 0, stream,  \
+        (TA*)out, (const TA*)q, q_stride, (const TA*)k_pages, (const TA*)v_pages, block_table,                 \
+        bt_stride, seq_of_token, positions, nh, nkv, hd, vd, page_size, window, scale,                         \
+        slopes, sink, (const TA*)gate, gate_stride, bias_table, bias_rows, sink_values, keep_first,            \
+        gate_wide,                                                                                             \
+        PooledPages<TA>{(const TA*)pooled_k, (const TA*)pooled_v, pooled_table, pooled_table_stride, pool},    \
+        out_stride, factor)
   HB_DISPATCH_DTYPE(act_dt, TA,
-    hb_launch(attention_generic_kernel<TA>, dim3(blocks), dim3(ATTN_WARPS * 32), 0, stream, 
-        (TA*)out, (const TA*)q, q_stride, (const TA*)k_pages, (const TA*)v_pages, block_table,
-        bt_stride, seq_of_token, positions, n_rows, nh, nkv, hd, vd, page_size, window, scale,
-        slopes, sink, (const TA*)gate, gate_stride, bias_table, bias_rows, sink_values, keep_first,
-        gate_wide,
-        PooledPages<TA>{(const TA*)pooled_k, (const TA*)pooled_v, pooled_table, pooled_table_stride, pool},
-        out_stride, factor));
+    const uintptr_t addresses = reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages) |
+                                (pool > 0 ? reinterpret_cast<uintptr_t>(pooled_k) | reinterpret_cast<uintptr_t>(pooled_v) : 0);
+    const bool vec = hd % 4 == 0 && vd % 4 == 0 && addresses % (4 * sizeof(TA)) == 0;
+    if (!vec) HB_GENERIC_LAUNCH(8, false);
+    else if (most <= 32) HB_GENERIC_LAUNCH(1, true);
+    else if (most <= 64) HB_GENERIC_LAUNCH(2, true);
+    else if (most <= 128) HB_GENERIC_LAUNCH(4, true);
+    else HB_GENERIC_LAUNCH(8, true));
+#undef HB_GENERIC_LAUNCH
   return hb_check_launch();
 }

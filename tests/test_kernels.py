@@ -563,3 +563,18 @@ def test_tcgen05_attention_refuses_sizes_it_does_not_take():
     with pytest.raises(ops().KernelError):
         ops().attention_prefill_tc(case.qkv, case.k_pages, case.v_pages, case.table, tiles, case.cu_tokens,
                                    case.start_pos, 6, 2, 96, 16, None, 0.125)
+
+
+# ---------------------------------------------------------------------- generic attention, runs dealt to warps
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd", [(2, 1, 4), (3, 3, 20), (4, 2, 33), (7, 1, 64), (2, 2, 100), (4, 1, 130), (2, 1, 255), (1, 1, 256)])
+def test_generic_attention_at_the_edges_of_runs_and_head_sizes(nh, nkv, hd, dtype):
+    """Contexts around a run (32 keys), around one run a warp (256) and beyond, with and without a
+    window, whole and odd head sizes."""
+    scale = 1.0 / math.sqrt(hd)
+    seqs = [(before, 1) for before in (0, 1, 30, 31, 32, 254, 255, 256, 300, 700)] + [(250, 9)]
+    case = make_paged_case(seqs, nh, nkv, hd, 8, dtype, DEV, seed=hd)
+    for window in (None, 1, 31, 33, 290):
+        got = ops().attention_generic(case.qkv, case.k_pages, case.v_pages, case.table, case.seq_of_token,
+                                      case.positions, nh, nkv, hd, 8, window, scale)
+        torch.testing.assert_close(got.cpu().double(), dense_attention(case, scale, window), **tol(dtype))
