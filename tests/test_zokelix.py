@@ -705,3 +705,51 @@ def test_greedy_generation_through_the_scheduler(zk_folders, name, dtype):
                 assert dtype == "bfloat16", f"token {t} instead of {best} after {len(toks)} tokens"
                 assert float(logits[best] - logits[t]) <= 0.03 * float(logits.abs().max())
             toks.append(t)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dk,dv", [(4, 4), (24, 30), (32, 128), (36, 40), (64, 132), (100, 17), (128, 128), (130, 20), (256, 8)])
+def test_delta_rule_a_token_a_step_is_the_walk_over_all_tokens_bit_for_bit(dk, dv):
+    """float32: the kernel for steps of single tokens (values in whole 16-byte pieces; the walk
+    otherwise) and the walk at both column widths leave the same outputs and states, and both are
+    the plain scan's."""
+    from types import SimpleNamespace
+    from helios_b200.csrc import ops
+
+    dev, heads, n, S = "cuda", 2, 21, 3
+    g = torch.Generator().manual_seed(dk + dv)
+    C = heads * (2 * dk + dv)
+    qkv, beta = torch.randn(S, n, C, generator=g), torch.randn(S, n, heads, generator=g) + 2
+    a = torch.randn(S, n, heads * dk, generator=g) - 2
+    a_log, dt_bias = torch.randn(heads, generator=g) * 0.3, torch.randn(heads * dk, generator=g) * 0.3
+    stride = -(-heads * dk * dv // 4) * 4
+
+    def run(rows, lens, state, slots):
+        cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).int().to(dev)
+        ctx = SimpleNamespace(cu_tokens=cu, slots=torch.tensor(slots, dtype=torch.int32, device=dev), num_seqs=len(lens))
+        return ops.delta_rule(ctx, rows(qkv), (0, heads * dk, 2 * heads * dk), rows(beta), rows(a), a_log.to(dev),
+                              dt_bias.to(dev), state[:, :heads * dk * dv], heads, heads, dk, dv)
+
+    whole = torch.zeros(S, stride, device=dev)
+    want = run(lambda t: t.reshape(S * n, -1).to(dev), [n] * S, whole, [0, 1, 2]).view(S, n, -1)
+    # many requests: the wide blocks (the same three again and again)
+    many = torch.zeros(240, stride, device=dev)
+    got = run(lambda t: t.repeat(80, 1, 1).reshape(240 * n, -1).to(dev), [n] * 240, many, list(range(240)))
+    assert torch.equal(got.view(80, S, n, -1), want.expand(80, S, n, -1)) and torch.equal(many.view(80, S, -1), whole.expand(80, S, -1))
+    # a token a step, other slots
+    state = torch.zeros(4, stride, device=dev)
+    for t in range(n):
+        got = run(lambda x: x[:, t].contiguous().to(dev), [1] * S, state, [3, 0, 2])
+        assert torch.equal(got, want[:, t])
+    assert torch.equal(state[[3, 0, 2]], whole) and not state[1].any()
+    for s in range(S):
+        x = qkv[s].double()
+        for h in range(heads):
+            q, k = x[:, h * dk:(h + 1) * dk], x[:, (heads + h) * dk:(heads + h + 1) * dk]
+            q = q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * dk ** -0.5
+            k = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+            v = x[:, 2 * heads * dk + h * dv:2 * heads * dk + (h + 1) * dv]
+            gd = torch.exp(-torch.exp(a_log[h].double()) * torch.nn.functional.softplus(
+                a[s, :, h * dk:(h + 1) * dk].double() + dt_bias[h * dk:(h + 1) * dk].double()))
+            o = pz.delta_scan(q, k, v, torch.sigmoid(beta[s, :, h].double()), gd)
+            assert (want[s, :, h * dv:(h + 1) * dv].cpu().double() - o).abs().max() < 2e-5
