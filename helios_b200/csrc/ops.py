@@ -525,6 +525,12 @@ def silu_mul(gate_up: torch.Tensor) -> torch.Tensor:
 
 
 # ------------------------------------------------------------------ matrix products
+#: rows of x up to which the float32 product streams the weight through the kernel for few rows
+#: (eight at a time).  Tiles / rows, microseconds at 16 rows and at 32: 9,728 x 896 73 / 33 and 72 / 56;
+#: 896 x 4,864 193 / 46 and 194 / 84; 151,936 x 896 479 / 364 and, at 32, the tiles are ahead
+GEMM_F32_FEW_ROWS = 16
+
+
 def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x [M, K] times weight [N, K] transposed (+ bias [N]) on the float32 FMA pipes."""
     _check(x, "x", torch.float32, 2)
@@ -539,8 +545,10 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
             raise KernelError(f"bias has {bias.numel()} entries for {N} outputs")
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     f = _fn("gemm_f32", "hb_gemm_f32",
-            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
-    _run(f(_p(out), _p(x), _p(weight), _p(bias), M, N, K, K, K, N, _stream()), "gemm_f32")
+            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+             c_void_p])
+    _run(f(_p(out), _p(x), _p(weight), _p(bias), M, N, K, K, K, N, GEMM_F32_FEW_ROWS, sm_count(x.device), _stream()),
+         "gemm_f32")
     return out
 
 

@@ -565,6 +565,25 @@ def test_tcgen05_attention_refuses_sizes_it_does_not_take():
                                    case.start_pos, 6, 2, 96, 16, None, 0.125)
 
 
+# ---------------------------------------------------------------------- float32 products of few rows
+@pytest.mark.parametrize("K", [4, 16, 20, 124, 128, 132, 512, 900, 4096, 4868, 19000])
+@pytest.mark.parametrize("M,N", [(1, 1), (1, 1201), (2, 130), (3, 37), (4, 600), (5, 64), (8, 9), (9, 33), (16, 5), (17, 40)])
+def test_gemm_f32_of_few_rows_is_the_tiled_product_bit_for_bit(M, N, K, monkeypatch):
+    """Edges of runs (16), of blocks of runs (128), of a warp's piece (512) and of a row's place in
+    shared memory; both kernels add in the same order, and a row alone is the row in the batch."""
+    g = torch.Generator().manual_seed(M * N + K)
+    x, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
+    got = ops().linear_f32(x.to(DEV), w.to(DEV), b.to(DEV))
+    want = x.double() @ w.double().T + b.double()
+    # |error| <= (additions an element goes through) * eps * sum |x||w|; sums of 16, of 8, of K / 128
+    bound = (26 + K / 128) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs()) + 1e-30
+    assert ((got.cpu().double() - want).abs() <= bound).all()
+    alone = ops().linear_f32(x[M - 1:].contiguous().to(DEV), w.to(DEV), b.to(DEV))
+    assert torch.equal(got[M - 1:], alone)
+    monkeypatch.setattr(ops(), "GEMM_F32_FEW_ROWS", 0)
+    assert torch.equal(ops().linear_f32(x.to(DEV), w.to(DEV), b.to(DEV)), got)
+
+
 # ---------------------------------------------------------------------- generic attention, runs dealt to warps
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("nh,nkv,hd", [(2, 1, 4), (3, 3, 20), (4, 2, 33), (7, 1, 64), (2, 2, 100), (4, 1, 130), (2, 1, 255), (1, 1, 256)])
