@@ -526,8 +526,8 @@ def silu_mul(gate_up: torch.Tensor) -> torch.Tensor:
 
 # ------------------------------------------------------------------ matrix products
 #: rows of x up to which the float32 product streams the weight through the kernel for few rows
-#: (eight at a time).  Tiles / rows, microseconds at 16 rows and at 32: 9,728 x 896 73 / 33 and 72 / 56;
-#: 896 x 4,864 193 / 46 and 194 / 84; 151,936 x 896 479 / 364 and, at 32, the tiles are ahead
+#: (eight at a time).  Tiles / rows, microseconds, at 16 rows: 9,728 x 896 46 / 35; 896 x 4,864
+#: 59 / 45; 1,152 x 896 14.5 / 8; at 24 rows 46 / 47, 59 / 64 and 14.5 / 14
 GEMM_F32_FEW_ROWS = 16
 
 
