@@ -173,10 +173,23 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, int V, in
 // on a row instead of one; three such blocks fit an SM.  Sums keep a fixed order: a
 // thread's elements in index order, the block's threads by `block_sum`, the cluster's blocks
 // by rank; the draw walks the row in index order as the kernel above does.
+//
+// A threshold search costs a pass over the row and two exchanges within the cluster per four bits,
+// sixteen for a row with top-k and top-p, though the tokens that matter are a few hundred.  So
+// one pass counts (and weighs) the values above SC_LEVELS levels below the maximum, in steps of
+// the temperature; the threshold lies between the highest level that holds k values, or more than
+// p of the mass, and the next.  Up to three more passes narrow that interval to an eighth each,
+// until it holds at most SC_LIST values; these go to the first block's shared memory, which sorts
+// them and reads the threshold off the sorted list.  Rows that stay wider (masses of equal
+// values, thresholds below the lowest level) keep the search.  128,256 values a row, µs a launch,
+// search / list: 64 rows N(0, 4) of mixed options 166 / 50, all top-k 50 and top-p 0.9 265 / 68,
+// one row 81 / 25; top-p 0.95 of 64 rows N(0, 1), 60,000 tokens kept, 452 / 146.
 constexpr int SC_THREADS = 512;
 constexpr int SC_CLUSTER = 8;
 constexpr int SC_MOST = 40;          // elements a thread keeps: rows of up to 8 * 512 * 40 values
 constexpr int SC_WARPS = SC_THREADS / 32;
+constexpr int SC_LEVELS = 6;
+constexpr int SC_LIST = 1024;        // two values a thread; a block's shared memory still fits an SM three times
 
 __device__ __forceinline__ float key_float(uint32_t k) {   // inverse of float_key
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
@@ -196,6 +209,71 @@ __device__ __forceinline__ float sc_peer_f32(const float* mine, uint32_t rank) {
                : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
   return v;
+}
+
+__device__ __forceinline__ void sc_store_peer_u32(const uint32_t* mine, uint32_t rank, uint32_t v) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote)
+               : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(v) : "memory");
+}
+
+// The threshold of a row, given the `count` <= SC_LIST values around it in `list` (unsorted, all of
+// an interval): sorts them, the largest first, and returns what the searches below find.  All
+// threads of one block.  k: the place in the list top-k keeps to, 0 off; p < 1: top-p of the mass
+// `all`, of which `above` lies above the list, or, with top-k, of what that keeps (then nothing is
+// above the list).  scratch: SC_WARPS floats and a word.
+__device__ uint32_t sc_sorted_threshold(uint32_t* list, int count, int k, float p, float all, float above,
+                                        float inv_t, float mx_t, float* scratch, uint32_t* word) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int n = 2;
+  while (n < count) n *= 2;
+  for (int i = count + tid; i < n; i += SC_THREADS) list[i] = 0u;
+  for (int size = 2; size <= n; size *= 2)
+    for (int half = size / 2; half > 0; half /= 2) {
+      __syncthreads();
+      const int i = 2 * half * (tid / half) + tid % half;          // pairs (i, i + half), n / 2 of them
+      if (tid < n / 2) {
+        const uint32_t a = list[i], b = list[i + half];
+        if ((a < b) == ((i & size) == 0)) { list[i] = b; list[i + half] = a; }
+      }
+    }
+  __syncthreads();
+  uint32_t thr = 1;
+  if (k > 0) thr = list[min(k, count) - 1];
+  if (p < 1.f) {
+    // the kept values' masses, two neighbours a thread, added up from the largest down
+    const int i = 2 * tid;
+    const uint32_t k0 = i < count ? list[i] : 0u, k1 = i + 1 < count ? list[i + 1] : 0u;
+    const float e0 = k0 >= thr ? expf(key_float(k0) * inv_t - mx_t) : 0.f;
+    const float e1 = k1 >= thr ? expf(key_float(k1) * inv_t - mx_t) : 0.f;
+    float incl = e0 + e1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) scratch[warp] = incl;
+    if (tid == 0) *word = 0u;
+    __syncthreads();
+    float before = __shfl_up_sync(0xffffffffu, incl, 1), total = 0.f;
+    if (lane == 0) before = 0.f;
+    before += above;
+    for (int w = 0; w < SC_WARPS; ++w) {
+      if (w < warp) before += scratch[w];
+      total += scratch[w];
+    }
+    const float want = p * (k > 0 ? total : all);
+    // the largest value down to which the mass exceeds the share
+    if (k0 >= thr && before + e0 > want) atomicMax(word, k0);
+    else if (k1 >= thr && before + e0 + e1 > want) atomicMax(word, k1);
+    __syncthreads();
+    // (nothing: the whole list's mass rounds to the share; it stays as it is)
+    const uint32_t found = *word;
+    if (found == 0u && k <= 0) thr = list[count - 1];
+    if (found > thr) thr = found;
+  }
+  return thr;
 }
 
 // Fifteen sums over the whole cluster, the same in every thread of every block afterwards:
@@ -241,7 +319,8 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
   __shared__ float total[16];
   __shared__ uint32_t s_key[SC_WARPS];
   __shared__ int s_idx[SC_WARPS];
-  __shared__ float x_f[4];                 // what a block shows its peers: key, index, total, pick
+  __shared__ float x_f[5];                 // what a block shows its peers: key, index, total, pick, threshold
+  __shared__ uint32_t list[SC_LIST];       // of the first block: the row's largest values
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = sc_rank();
   const int row = blockIdx.x / SC_CLUSTER;
@@ -303,10 +382,131 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
   int slot = 0;
   float acc[15];
 
+  // ---- the values above a level, sorted (see above); not for a maximum that is no number or infinite
+  const int k_row = top_k[row], k_on = (k_row > 0 && k_row < V) ? k_row : 0;
+  const float p_on = top_p[row];
+  uint32_t sorted_thr = 0;
+  if ((k_on > 0 || p_on < 1.f) && !(p_on < 0.f) && fabsf(key_float(bk)) < INFINITY && inv_t < INFINITY) {
+    constexpr float depth[SC_LEVELS] = {1.f, 2.f, 4.f, 7.f, 12.f, 24.f};
+    uint32_t level[SC_LEVELS];
+#pragma unroll
+    for (int j = 0; j < SC_LEVELS; ++j) level[j] = float_key(key_float(bk) - depth[j] * temp);
+#pragma unroll
+    for (int j = 0; j < 15; ++j) acc[j] = 0.f;
+    // [0, 6): masses above the levels; 6: of everything; [7, 13): counts
+#pragma unroll 4
+    for (int i = 0; i < EPT; ++i) {
+      const uint32_t c = key[i];
+      float e = 0.f;
+      if (k_on == 0 && c >= 1u) acc[SC_LEVELS] += e = expf(key_float(c) * inv_t - mx_t);
+      if (c >= level[SC_LEVELS - 1]) {
+#pragma unroll
+        for (int j = 0; j < SC_LEVELS; ++j)
+          if (c >= level[j]) {
+            acc[j] += e;
+            acc[SC_LEVELS + 1 + j] += 1.f;
+          }
+      }
+    }
+    sc_sum15(acc, warp_part, block_part, total, slot);
+    // lo: the highest level that satisfies the row (holds k values, or more than p of the mass);
+    // up: the level above it, which does not; with the mass and count above them
+    const float everything = acc[SC_LEVELS];
+    const bool whole = k_on > 0 && p_on < 1.f;             // the list starts at the maximum
+    auto satisfies = [&](float mass, float count) { return k_on > 0 ? count >= (float)k_on : mass > p_on * everything; };
+    uint32_t lo = 0, up = 0xffffffffu;
+    float lo_count = 0.f, up_mass = 0.f, up_count = 0.f;
+    bool settled = false;
+#pragma unroll
+    for (int j = 0; j < SC_LEVELS; ++j)
+      if (!settled) {
+        const float count = acc[SC_LEVELS + 1 + j];
+        settled = satisfies(acc[j], count);
+        if (settled) { lo = level[j]; lo_count = count; }
+        else { up = level[j]; up_mass = acc[j]; up_count = count; }
+      }
+    // too many in between: seven values between the two, a few times
+    bool fits = false;
+    for (int round = 0; settled; ++round) {
+      fits = lo_count - (whole ? 0.f : up_count) <= (float)SC_LIST;
+      if (fits || round == 4) break;
+      slot ^= 1;
+      const float v0 = key_float(lo), step = (key_float(up == 0xffffffffu ? bk : up) - v0) * 0.125f;
+#pragma unroll
+      for (int j = 0; j < 15; ++j) acc[j] = 0.f;
+#pragma unroll 4
+      for (int i = 0; i < EPT; ++i) {
+        const uint32_t c = key[i];
+        if (c >= lo && c < up) {
+          const float v = key_float(c), e = k_on == 0 ? expf(v * inv_t - mx_t) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 7; ++j)
+            if (v >= fmaf(step, (float)(j + 1), v0)) {
+              acc[j] += e;
+              acc[7 + j] += 1.f;
+            }
+        }
+      }
+      sc_sum15(acc, warp_part, block_part, total, slot);
+      const float base_mass = up_mass, base_count = up_count;
+      const uint32_t old_lo = lo, old_up = up;
+      bool raised = false;
+#pragma unroll
+      for (int j = 6; j >= 0; --j) {                        // from the highest cut down
+        const uint32_t cut = float_key(fmaf(step, (float)(j + 1), v0));
+        if (raised || cut <= old_lo || cut >= old_up) continue;
+        raised = satisfies(base_mass + acc[j], base_count + acc[7 + j]);
+        if (raised) { lo = cut; lo_count = base_count + acc[7 + j]; }
+        else { up = cut; up_mass = base_mass + acc[j]; up_count = base_count + acc[7 + j]; }
+      }
+    }
+    if (fits) {                                              // the same in every thread of the cluster
+      const uint32_t list_up = whole ? 0xffffffffu : up;
+      const float above_count = whole ? 0.f : up_count, above_mass = whole ? 0.f : up_mass;
+      int kept = 0;
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) kept += key[i] >= lo && key[i] < list_up ? 1 : 0;
+      int incl = kept;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane == 31) s_idx[warp] = incl;
+      __syncthreads();
+      int at = incl - kept;
+      for (int w = 0; w < warp; ++w) at += s_idx[w];
+      if (tid == SC_THREADS - 1) x_f[2] = __int_as_float(at + kept);
+      sc_cluster_sync();
+      int count = 0;
+      for (uint32_t r = 0; r < SC_CLUSTER; ++r) {
+        const int n = __float_as_int(sc_peer_f32(&x_f[2], r));
+        if (r < rank) at += n;
+        count += n;
+      }
+      if (kept > 0 && count <= SC_LIST) {
+        for (int i = 0; i < EPT; ++i)
+          if (key[i] >= lo && key[i] < list_up) sc_store_peer_u32(&list[at++], 0, key[i]);
+      }
+      sc_cluster_sync();
+      if (rank == 0 && count > 0 && count <= SC_LIST) {
+        const uint32_t found = sc_sorted_threshold(list, count, k_on > 0 ? k_on - (int)above_count : 0, p_on, everything,
+                                                   above_mass, inv_t, mx_t, total, &s_key[0]);
+        if (tid == 0) x_f[4] = __uint_as_float(found);
+      } else if (rank == 0 && tid == 0) {
+        x_f[4] = 0.f;                                        // (cannot be: the counts are exact)
+      }
+      sc_cluster_sync();
+      sorted_thr = __float_as_uint(sc_peer_f32(&x_f[4], 0));
+    }
+    slot ^= 1;
+  }
+  const bool search = sorted_thr == 0;
+
   // ---- top-k: the largest key c with #(key >= c) >= k, four bits a pass
   uint32_t thr = 1;                        // keeps every value, and none of the padding
-  const int k = top_k[row];
-  if (k > 0 && k < V) {
+  const int k = k_on;
+  if (k > 0 && search) {
     uint32_t cand = 0;
     for (int shift = 28; shift >= 0; shift -= 4) {
 #pragma unroll
@@ -331,8 +531,8 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
     if (cand > thr) thr = cand;
   }
   // ---- top-p over what top-k kept: the largest key c with mass(key >= c) > p * Z
-  const float pp = top_p[row];
-  if (pp < 1.f) {
+  const float pp = p_on;
+  if (pp < 1.f && search) {
 #pragma unroll
     for (int j = 0; j < 15; ++j) acc[j] = 0.f;
 #pragma unroll
@@ -363,6 +563,8 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
     }
     if (cand > thr) thr = cand;
   }
+
+  if (!search) thr = sorted_thr;
 
   // ---- inverse CDF in index order: a thread's kept mass, its place among the block's
   // threads (a scan in thread order), the block's place among the blocks (by rank)
@@ -464,7 +666,7 @@ static int launch_sample_cluster(int* out, const float* logits, int R, int V, in
 // draw but none has a top-k or top-p, 2 some have (-1: unknown, taken as 2), 3: the one-block
 // kernel whatever the rows.  Measured in chains at 128,256 values, one block / cluster, µs:
 // argmax 10 / 6 at 8 rows, 16 / 15 at 64, 24 / 58 at 256; temperature 57 / 13, 84 / 31,
-// 95 / 106; top-k 50 and top-p 0.9: 672 / 91, 1,000 / 262, 1,620 / 855.
+// 95 / 106; top-k 50 and top-p 0.9: 672 / 30, 1,000 / 68, 1,620 / 215.
 HB_EXPORT int hb_sample(int* out, const float* logits, int R, int V, int ld, const float* temperature,
                         const int* top_k, const float* top_p, const unsigned long long* seed,
                         const unsigned long long* offset, int kind, cudaStream_t stream) {

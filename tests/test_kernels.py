@@ -486,6 +486,62 @@ def test_temperature_top_k_top_p_follow_the_reference_rules(V, one_block):
             assert near < 1e-4, f"row {i}: got {got[i]}, reference {want}, u={u}"
 
 
+def _sampling_row(kind, V, g):
+    """A row at an edge of the sorted list of the cluster kernel: its longest (1,024 values), one
+    more, none (a spread row), ties at the k-th value, nearly everything masked out."""
+    if kind == "spread":
+        return torch.randn(V, generator=g) * 0.05
+    if kind == "masked":
+        row = torch.full((V,), float("-inf"))
+        row[torch.randperm(V, generator=g)[:3]] = torch.tensor([1.0, 2.0, 2.5])
+        return row
+    if kind == "ties":
+        row = torch.randn(V, generator=g) - 10
+        row[torch.randperm(V, generator=g)[:300]] = 3.0
+        row[torch.randperm(V, generator=g)[:4]] = 5.0
+        return row
+    n = int(kind)                              # n values within a unit of the maximum, the rest far below
+    row = torch.randn(V, generator=g) * 0.5 - 60
+    row[torch.randperm(V, generator=g)[:n]] = torch.rand(n, generator=g) * 0.5 + 4
+    return row
+
+
+@pytest.mark.parametrize("V", [4096, 40003, 163840])
+@pytest.mark.parametrize("kind", ["1", "2", "3", "31", "512", "1023", "1024", "1025", "1500", "spread", "masked", "ties"])
+def test_sampling_from_the_sorted_list_follows_the_reference_rules(kind, V):
+    g = torch.Generator().manual_seed(V)
+    options = [(1.0, 0, 0.9), (0.7, 0, 0.2), (1.0, 40, 1.0), (1.3, 1, 1.0), (0.9, 200, 0.8), (1.0, 1000, 0.999), (1.0, 1, 0.3),
+               (0.5, 0, 0.0), (1.0, 0, 1.0 - 2.0 ** -20), (1.0, V - 1, 0.5)]
+    logits = torch.stack([_sampling_row(kind, V, g) for _ in options])
+    temps, ks, ps = map(list, zip(*options))
+    seeds, offsets = list(range(7, 7 + len(options))), [5 * i for i in range(len(options))]
+    got = _sample(logits, temps, ks, ps, seeds, offsets)
+    if kind == "ties":                         # all of equal values stay or go: the rule of the other kernel
+        assert got == _sample(logits, temps, ks, ps, seeds, offsets, kind="one_block")
+        return
+    for i in range(len(options)):
+        u = ops().philox_uniform(seeds[i], offsets[i])
+        want = plain_model.sample_reference(logits[i], temps[i], ks[i], ps[i], u)
+        if got[i] != want:                     # a draw, or the share itself, that falls on a rounding of the mass
+            kept = torch.softmax(logits[i].double() / temps[i], -1)
+            if ks[i]:
+                kept = torch.where(logits[i] < torch.topk(logits[i], ks[i]).values[-1], 0.0, kept)
+            cum = torch.cumsum(torch.sort(kept, descending=True).values, 0) / kept.sum()
+            share = float((cum - ps[i]).abs().min()) if ps[i] < 1 else 1.0
+            near = min(abs(u - x) for x in _boundaries(logits[i], temps[i], ks[i], ps[i], got[i], want))
+            assert kept[got[i]] > 0 and min(near, share) < 1e-6, f"row {i}: got {got[i]}, reference {want}, u={u}"
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan"), -float("inf")])
+def test_rows_without_a_finite_maximum_end(bad):
+    """Rows of infinities and NaN have no distribution; the kernel returns some id of the vocabulary."""
+    logits = torch.randn(4, 9000, generator=torch.Generator().manual_seed(2))
+    logits[0, 77] = logits[1, 78] = bad
+    logits[2:] = bad
+    got = _sample(logits, [1.0] * 4, [5, 0, 50, 0], [1.0, 0.9, 0.9, 0.5], [1] * 4, [0] * 4)
+    assert all(0 <= t < 9000 for t in got)
+
+
 def _boundaries(logits, temp, k, p, a, b):
     l = logits.double() / temp
     if k > 0:
