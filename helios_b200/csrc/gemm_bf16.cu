@@ -747,6 +747,12 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(args.out) + (size_t)t * args.ldo + n0);
             dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
             dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+          } else if (args.out_f32 && n0 + 16 <= args.N && (args.ldo & 3) == 0) {
+            // (one value a store instead: every store of a warp begins 32 sectors of which it fills an
+            // eighth; the head of 151,936 x 896 at 200 tokens took 278 µs so, against 95)
+            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(args.out) + (size_t)t * args.ldo + n0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dst[i] = make_float4(val[4 * i], val[4 * i + 1], val[4 * i + 2], val[4 * i + 3]);
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {

@@ -212,3 +212,12 @@ def test_two_products_with_the_norm_between_them_folded_in():
         ops().linear_bf16(torch.zeros(40, H, dtype=torch.bfloat16, device=DEV), wo.to(DEV),
                           residual=torch.zeros(40, H, device=DEV))
     ops().check_kernel_errors()
+
+
+@pytest.mark.parametrize("T", [129, 255, 257])
+@pytest.mark.parametrize("N", [16, 250, 252, 255, 256, 260, 1001])
+def test_float32_output_of_the_two_sm_kernel_at_odd_widths(T, N):
+    """Rows that are and are not whole 16-byte pieces, and a last piece of sixteen columns that is cut."""
+    x, w, _b = _case(T, N, 136, T * N)
+    got = ops().linear_bf16(x.to(DEV), w.to(DEV), plan=(0, 1), two_sm=True, out_dtype=torch.float32)
+    torch.testing.assert_close(got.double().cpu(), x.double() @ w.double().T, atol=2e-3, rtol=1e-3)
