@@ -605,8 +605,11 @@ HB_EXPORT int hb_glu_act(void* out, const void* gate_up, int T, int I, int kind,
 // that norms what a sublayer returns instead of what it reads; `copy` (may be null)
 // receives the new residual row in the activation dtype, which is what the next sublayer
 // reads.  With y == null only the copy is made.
-template <typename TY, typename TC>
-__global__ void __launch_bounds__(256)
+// GROUPS: groups of four neighbouring values a thread keeps between the passes, all loads issued
+// before the first sum (0: any width, value by value, which reads y twice).  Rows of 2,048,
+// bfloat16 y, a launch in a chain, value by value / kept, µs: 4.9 / 2.1 at 64 rows, 21 / 8.6 at 2,048.
+template <typename TY, typename TC, int GROUPS>
+__global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_add_kernel(float* __restrict__ residual, const TY* __restrict__ y,
                    const float* __restrict__ weight, TC* __restrict__ copy, int H, float eps) {
   pdl_launch_dependents();
@@ -614,11 +617,48 @@ rmsnorm_add_kernel(float* __restrict__ residual, const TY* __restrict__ y,
   __shared__ float scratch[33];
   float* res = residual + (size_t)blockIdx.x * H;
   TC* cp = copy ? copy + (size_t)blockIdx.x * H : nullptr;
+  const TY* yr = y + (size_t)blockIdx.x * H;
+  if constexpr (GROUPS > 0) {
+    float v[GROUPS][4], d[GROUPS][4], w[GROUPS][4];
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+      const int c = (g * NORM_THREADS + threadIdx.x) * 4;
+      if (c < H) {
+        load4(res + c, v[g]);
+        if (y) {
+          load4(yr + c, d[g]);
+          load4(weight + c, w[g]);
+        }
+      }
+    }
+    if (y) {
+      float ss = 0.f;
+#pragma unroll
+      for (int g = 0; g < GROUPS; ++g)
+        if ((g * NORM_THREADS + threadIdx.x) * 4 < H) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) ss = fmaf(d[g][e], d[g][e], ss);
+        }
+      const float rstd = rsqrtf(block_sum(ss, scratch) / (float)H + eps);
+#pragma unroll
+      for (int g = 0; g < GROUPS; ++g)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[g][e] = fmaf(d[g][e] * rstd, w[g][e], v[g][e]);
+    }
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+      const int c = (g * NORM_THREADS + threadIdx.x) * 4;
+      if (c < H) {
+        if (y) store4(res + c, v[g]);
+        if (cp) store4(cp + c, v[g]);
+      }
+    }
+    return;
+  }
   if (y == nullptr) {
     for (int c = threadIdx.x; c < H; c += blockDim.x) cp[c] = from_float<TC>(res[c]);
     return;
   }
-  const TY* yr = y + (size_t)blockIdx.x * H;
   float ss = 0.f;
   for (int c = threadIdx.x; c < H; c += blockDim.x) { const float v = to_float(yr[c]); ss += v * v; }
   const float rstd = rsqrtf(block_sum(ss, scratch) / (float)H + eps);
@@ -633,10 +673,20 @@ HB_EXPORT int hb_rmsnorm_add(float* residual, const void* y, const float* weight
                              int n, int H, float eps, int y_dt, int copy_dt, cudaStream_t stream) {
   if (n <= 0) return HB_OK;
   if (y == nullptr && copy == nullptr) return HB_OK;
+  const bool vec = H % 4 == 0 && H <= NORM_THREADS * NORM_GROUPS * 4 &&
+                   (((uintptr_t)residual | (uintptr_t)y | (uintptr_t)weight | (uintptr_t)copy) & 15) == 0;
+  const int groups = vec ? (H + NORM_THREADS * 4 - 1) / (NORM_THREADS * 4) : 0;
+#define HB_NORM_ADD(G)                                                                                      \
+  hb_launch(rmsnorm_add_kernel<TY, TC, G>, dim3(n), dim3(NORM_THREADS), 0, stream, residual, (const TY*)y,    \
+            weight, (TC*)copy, H, eps)
   HB_DISPATCH_DTYPE(y_dt, TY,
     HB_DISPATCH_DTYPE(copy_dt, TC,
-      hb_launch(rmsnorm_add_kernel<TY, TC>, dim3(n), dim3(256), 0, stream, residual, (const TY*)y,
-                weight, (TC*)copy, H, eps)));
+      if (groups == 0) HB_NORM_ADD(0);
+      else if (groups == 1) HB_NORM_ADD(1);
+      else if (groups == 2) HB_NORM_ADD(2);
+      else if (groups <= 4) HB_NORM_ADD(4);
+      else HB_NORM_ADD(8)));
+#undef HB_NORM_ADD
   return hb_check_launch();
 }
 

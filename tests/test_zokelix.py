@@ -753,3 +753,25 @@ def test_delta_rule_a_token_a_step_is_the_walk_over_all_tokens_bit_for_bit(dk, d
                 a[s, :, h * dk:(h + 1) * dk].double() + dt_bias[h * dk:(h + 1) * dk].double()))
             o = pz.delta_scan(q, k, v, torch.sigmoid(beta[s, :, h].double()), gd)
             assert (want[s, :, h * dv:(h + 1) * dv].cpu().double() - o).abs().max() < 2e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("y_dtype", DTYPES)
+@pytest.mark.parametrize("H", [4, 37, 1020, 1024, 1028, 2052, 4100, 8192, 8196])
+def test_norm_on_an_output_at_the_widths_its_rows_are_kept_at(H, y_dtype):
+    """One to eight groups of four values a thread, and the widths that go value by value; with and
+    without the copy, and the copy alone."""
+    from helios_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(H)
+    dt = torch.float32 if y_dtype == "float32" else torch.bfloat16
+    res, w = torch.randn(5, H, generator=g), torch.rand(H, generator=g) + 0.5
+    y = (torch.randn(5, H, generator=g) * 3).to(dt)
+    yd = y.double()
+    want = res.double() + yd / torch.sqrt((yd * yd).mean(-1, keepdim=True) + 1e-5) * w.double()
+    r = res.cuda()
+    copy = ops.rmsnorm_add(r, y.cuda(), w.cuda(), 1e-5, torch.bfloat16)
+    # a sum of H squares, a root and two products: some H / 256 + 12 roundings, most of them averaged out
+    torch.testing.assert_close(r.cpu().double(), want, atol=4e-6, rtol=4e-6)
+    assert torch.equal(copy, r.to(torch.bfloat16))
+    assert torch.equal(ops.rmsnorm_add(r, None, None, 0.0, torch.bfloat16), copy)
