@@ -196,7 +196,8 @@ HB_EXPORT int hb_causal_conv_silu(void* out, const void* x, int ld, const float*
 // Bound by the chain of a token: products, shuffles, the write.  So the columns of one request
 // are spread over as many SMs as there are (one prompt of 16 heads of 128 x 128: 128 blocks of
 // four warps; with 64 columns a block and four threads a column it was 32 blocks), and the
-// products go two an instruction.  2,048 tokens 1,428 -> 527 µs, of 8 heads of 64 x 64 912 -> 372.
+// products go two an instruction.  2,048 tokens 1,428 -> 447 µs, of 8 heads of 64 x 64 912 -> 314 (with
+// conversions of the next chunk's values, and its beta stored from registers, 527 and 372).
 constexpr int DR_CHUNK = 16;        // tokens staged in shared memory at a time
 constexpr int DR_PARTS = 8;         // threads a column of S is spread over
 // columns of S a block owns: 16, or 32 where 32 still give two blocks an SM (the staged rows
@@ -207,6 +208,10 @@ constexpr int DR_WIDE_BLOCKS = 296;
 __device__ __forceinline__ void dr_cp_async16(void* smem, const void* gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void dr_cp_async8(void* smem, const void* gmem) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
 }
 
 // A warp's norms of one (token, head): 1 / |k|, dk^-1/2 / |q| and k . q of the unit vectors
@@ -333,25 +338,35 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
   for (int idx = threadIdx.x; idx < 2 * DR_CHUNK * 3 * (DK - dkp); idx += THREADS)
     stage_buf[idx / (DK - dkp) * DK + dkp + idx % (DK - dkp)] = 0.f;
 
+  // (nothing here waits for a load: a warp issues in order, and a conversion or a store of what was
+  // just asked for would hold up the tokens of the chunk that is there)
   auto stage = [&](int c0, int b) {
     const int nc = min(DR_CHUNK, n - c0);
-    const int vecs = dkp / 4;
     float* dst = stage_buf + b * DR_CHUNK * ROW;
     const float* src = kqg + ((size_t)(t0 + c0) * heads + h) * 3 * dkp;
-    for (int idx = threadIdx.x; idx < nc * 3 * vecs; idx += THREADS) {
-      const int r = idx / vecs, v = idx - r * vecs, j = r / 3;      // r = 3 j + (k, q or g)
-      dr_cp_async16(dst + r * DK + v * 4, src + (size_t)j * heads * 3 * dkp + (r - 3 * j) * dkp + v * 4);
+    const size_t token_step = (size_t)heads * 3 * dkp;
+    if (dkp == DK) {
+      for (int idx = threadIdx.x; idx < nc * (ROW / 4); idx += THREADS) {
+        const int j = idx / (ROW / 4), v = idx % (ROW / 4);
+        dr_cp_async16(dst + j * ROW + v * 4, src + j * token_step + v * 4);
+      }
+    } else {
+      const int vecs = dkp / 4;
+      for (int idx = threadIdx.x; idx < nc * 3 * vecs; idx += THREADS) {
+        const int r = idx / vecs, v = idx - r * vecs, j = r / 3;    // r = 3 j + (k, q or g)
+        dr_cp_async16(dst + r * DK + v * 4, src + j * token_step + (r - 3 * j) * dkp + v * 4);
+      }
     }
-    for (int j = threadIdx.x; j < 2 * nc; j += THREADS)
-      bs[2 * b * DR_CHUNK + j] = beta[2 * ((size_t)(t0 + c0 + (j >> 1)) * heads + h) + (j & 1)];
+    for (int j = threadIdx.x; j < nc; j += THREADS)
+      dr_cp_async8(bs + 2 * (b * DR_CHUNK + j), beta + 2 * ((size_t)(t0 + c0 + j) * heads + h));
   };
   // the column's thread `part` fetches the values of tokens part, part + DR_PARTS, ... of a chunk
-  float v_next[VT];
+  T v_next[VT];
   auto fetch_v = [&](int c0) {
 #pragma unroll
     for (int jj = 0; jj < VT; ++jj) {
       const int j = DR_PARTS * jj + part;
-      v_next[jj] = (c0 + j < n) ? to_float(v_col[(size_t)(t0 + c0 + j) * qkv_ld]) : 0.f;
+      v_next[jj] = v_col[(size_t)(t0 + min(c0 + j, n - 1)) * qkv_ld];
     }
   };
 
@@ -368,7 +383,7 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
     const int nc = min(DR_CHUNK, n - c0);
     asm volatile("cp.async.wait_group 0;\n" ::);
 #pragma unroll
-    for (int jj = 0; jj < VT; ++jj) vs[(b * DR_CHUNK + DR_PARTS * jj + part) * COLS + lcol] = v_next[jj];
+    for (int jj = 0; jj < VT; ++jj) vs[(b * DR_CHUNK + DR_PARTS * jj + part) * COLS + lcol] = to_float(v_next[jj]);
     __syncthreads();
     if (c0 + DR_CHUNK < n) {
       stage(c0 + DR_CHUNK, b ^ 1);
