@@ -189,7 +189,7 @@ HB_EXPORT int hb_causal_conv_silu(void* out, const void* x, int ld, const float*
 // beta = sigmoid(b), all float32, left as kqg [T, heads, 3, dkp] (dkp = dk rounded up to 4;
 // the padding holds k = q = 0, g = 1) and (beta, k . q) [T, heads, 2].  `delta_rule` then walks each
 // request's tokens in order: a block owns 16 (or 32) columns of one head's S, eight threads one
-// column in registers (an eighth of its dk rows each); the staged rows of 16 tokens arrive in
+// column (or two) in registers (an eighth of its dk rows each); the staged rows of 16 tokens arrive in
 // shared memory by 16-byte cp.async one chunk ahead, the values of the next chunk wait in
 // registers, and the two sums over dk run as four partial sums a thread and three shuffles
 // (their order depends on dk alone, not on the step or the batch).
@@ -200,9 +200,14 @@ HB_EXPORT int hb_causal_conv_silu(void* out, const void* x, int ld, const float*
 // conversions of the next chunk's values, and its beta stored from registers, 527 and 372).
 constexpr int DR_CHUNK = 16;        // tokens staged in shared memory at a time
 constexpr int DR_PARTS = 8;         // threads a column of S is spread over
-// columns of S a block owns: 16, or 32 where 32 still give two blocks an SM (the staged rows
-// then serve twice the columns)
+// Columns of S a block owns, and columns a thread has a share of.  Where every block has an SM of its
+// own, 16 and one: a token's chain bounds the walk, and is shortest so.  With several blocks an SM its
+// shared-memory path does (a 16-byte load takes four cycles whatever it broadcasts; 212 of 345 cycles
+// a token), and a row's piece is read once for two columns; 32 columns a block where that leaves two
+// blocks an SM.  One column a thread / two, µs: one request of 2,048 tokens 447 / 498; 3 of 700 328 /
+// 284; 24 of 40 150 / 110; 64 of 8 130 / 103.
 constexpr int DR_COLS = 16, DR_COLS_WIDE = 32;
+constexpr int DR_SMS = 148;
 constexpr int DR_WIDE_BLOCKS = 296;
 
 __device__ __forceinline__ void dr_cp_async16(void* smem, const void* gmem) {
@@ -296,9 +301,10 @@ __device__ __forceinline__ float dr_hi(uint64_t v) { return __uint_as_float((uin
 // v at qkv[t, v_off + h * dv + col].  S of a slot at state + slot * state_stride,
 // [heads, dk, dv].  o [T, heads * dv] float32.  A column of S is held by DR_PARTS neighbouring
 // threads: thread `part` keeps the rows 4 (DR_PARTS m + part) .. + 3, and the two sums over dk
-// are finished with shuffles.  COLS changes which block owns a column, never a sum's order.
-template <typename T, int DK, int COLS>
-__global__ void __launch_bounds__(COLS * DR_PARTS)
+// are finished with shuffles.  A thread has W (1 or 2) columns.  COLS and W change which block and
+// thread own a column, never a sum's order.
+template <typename T, int DK, int COLS, int W>
+__global__ void __launch_bounds__(COLS * DR_PARTS / W)
 delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const float* __restrict__ beta,
                   const T* __restrict__ qkv, int qkv_ld, int v_off, float* __restrict__ state,
                   long state_stride, const int* __restrict__ cu_tokens, const int* __restrict__ slots,
@@ -309,7 +315,7 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
   // time; the blocks of a dependent released at the start would wait beside them as long.
   pdl_wait();
   extern __shared__ __align__(16) float dr_sm[];
-  constexpr int THREADS = COLS * DR_PARTS, STEP = 4 * DR_PARTS;
+  constexpr int THREADS = COLS * DR_PARTS / W, STEP = 4 * DR_PARTS;
   constexpr int G = DK / STEP;                      // float4 groups a thread holds
   constexpr int VT = DR_CHUNK / DR_PARTS;           // values of a chunk a thread fetches
   constexpr int ROW = 3 * DK;                       // staged floats a token: k, q, g of DK rows each
@@ -319,21 +325,25 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
   float* vs = bs + 4 * DR_CHUNK;                    // [2][CHUNK][COLS]
   const int s = blockIdx.x, h = blockIdx.y;
   const int part = threadIdx.x % DR_PARTS, lcol = threadIdx.x / DR_PARTS;
-  const int col = blockIdx.z * COLS + lcol;
-  const bool live = col < dv;
+  const int col = blockIdx.z * COLS + W * lcol;
+  bool live[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) live[w] = col + w < dv;
   const int t0 = cu_tokens[s], n = cu_tokens[s + 1] - t0;
   float* S_g = state + (size_t)slots[s] * state_stride + (size_t)h * dk * dv;
-  const T* v_col = qkv + v_off + (size_t)h * dv + (live ? col : 0);
+  const T* v_head = qkv + v_off + (size_t)h * dv;
 
-  uint64_t S[G][2];
+  uint64_t S[W][G][2];
 #pragma unroll
   for (int m = 0; m < G; ++m)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int i = STEP * m + 4 * part + 2 * e;
-      S[m][e] = dr_pack((live && i < dk) ? S_g[(size_t)i * dv + col] : 0.f,
-                        (live && i + 1 < dk) ? S_g[(size_t)(i + 1) * dv + col] : 0.f);
-    }
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        const int i = STEP * m + 4 * part + 2 * e;
+        S[w][m][e] = dr_pack((live[w] && i < dk) ? S_g[(size_t)i * dv + col + w] : 0.f,
+                             (live[w] && i + 1 < dk) ? S_g[(size_t)(i + 1) * dv + col + w] : 0.f);
+      }
   // the staged rows behind dkp hold nothing: k = q = g = 0 there, once for all tokens
   for (int idx = threadIdx.x; idx < 2 * DR_CHUNK * 3 * (DK - dkp); idx += THREADS)
     stage_buf[idx / (DK - dkp) * DK + dkp + idx % (DK - dkp)] = 0.f;
@@ -360,13 +370,14 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
     for (int j = threadIdx.x; j < nc; j += THREADS)
       dr_cp_async8(bs + 2 * (b * DR_CHUNK + j), beta + 2 * ((size_t)(t0 + c0 + j) * heads + h));
   };
-  // the column's thread `part` fetches the values of tokens part, part + DR_PARTS, ... of a chunk
-  T v_next[VT];
+  // the columns' thread `part` fetches the values of tokens part, part + DR_PARTS, ... of a chunk
+  T v_next[VT][W];
   auto fetch_v = [&](int c0) {
 #pragma unroll
     for (int jj = 0; jj < VT; ++jj) {
-      const int j = DR_PARTS * jj + part;
-      v_next[jj] = v_col[(size_t)(t0 + min(c0 + j, n - 1)) * qkv_ld];
+      const T* v = v_head + (size_t)(t0 + min(c0 + DR_PARTS * jj + part, n - 1)) * qkv_ld;
+#pragma unroll
+      for (int w = 0; w < W; ++w) v_next[jj][w] = v[live[w] ? col + w : 0];
     }
   };
 
@@ -378,12 +389,14 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
   int b = 0;
   float* o_next = o + (size_t)t0 * heads * dv + (size_t)h * dv + col;
   const size_t o_step = (size_t)heads * dv;
-  const bool writes = live && part == 0;
   for (int c0 = 0; c0 < n; c0 += DR_CHUNK) {
     const int nc = min(DR_CHUNK, n - c0);
     asm volatile("cp.async.wait_group 0;\n" ::);
 #pragma unroll
-    for (int jj = 0; jj < VT; ++jj) vs[(b * DR_CHUNK + DR_PARTS * jj + part) * COLS + lcol] = to_float(v_next[jj]);
+    for (int jj = 0; jj < VT; ++jj)
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        vs[(b * DR_CHUNK + DR_PARTS * jj + part) * COLS + W * lcol + w] = to_float(v_next[jj][w]);
     __syncthreads();
     if (c0 + DR_CHUNK < n) {
       stage(c0 + DR_CHUNK, b ^ 1);
@@ -392,10 +405,10 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
     asm volatile("cp.async.commit_group;\n" ::);
     const float* rows = stage_buf + b * DR_CHUNK * ROW + 4 * part;
     const float* bq = bs + 2 * b * DR_CHUNK;
-    const float* vc = vs + b * DR_CHUNK * COLS + lcol;
+    const float* vc = vs + b * DR_CHUNK * COLS + W * lcol;
     // a token's row pieces are read one token ahead, so that the chain of a token is the
     // products, the shuffles and the write alone
-    struct Token { ulonglong2 k[G], q[G], g[G]; float2 bq; float v; };
+    struct Token { ulonglong2 k[G], q[G], g[G]; float2 bq; float v[W]; };
     auto fetch = [&](Token& x, int j) {
       const float* r = rows + j * ROW;
 #pragma unroll
@@ -405,38 +418,55 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
         x.g[m] = *reinterpret_cast<const ulonglong2*>(r + 2 * DK + STEP * m);
       }
       x.bq = *reinterpret_cast<const float2*>(bq + 2 * j);
-      x.v = vc[j * COLS];
+      if constexpr (W == 2) {
+        const float2 v = *reinterpret_cast<const float2*>(vc + j * COLS);
+        x.v[0] = v.x;
+        x.v[1] = v.y;
+      } else {
+        x.v[0] = vc[j * COLS];
+      }
     };
     // one pass: S <- g (.) S with the sums S^T k and S^T q; then u, the read-out
     // o = S^T q + u (k . q) (what S^T q is after the write), and the write S += k u, which
     // nothing waits for until the next token's pass
     auto token = [&](const Token& x, Token& ahead, int j_ahead) {
-      uint64_t d01 = 0, d23 = 0, e01 = 0, e23 = 0;
+      uint64_t d01[W] = {}, d23[W] = {}, e01[W] = {}, e23[W] = {};
 #pragma unroll
-      for (int m = 0; m < G; ++m) {
-        S[m][0] = dr_mul2(S[m][0], x.g[m].x);
-        S[m][1] = dr_mul2(S[m][1], x.g[m].y);
-        d01 = dr_fma2(S[m][0], x.k[m].x, d01);
-        d23 = dr_fma2(S[m][1], x.k[m].y, d23);
-        e01 = dr_fma2(S[m][0], x.q[m].x, e01);
-        e23 = dr_fma2(S[m][1], x.q[m].y, e23);
-      }
+      for (int m = 0; m < G; ++m)
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          S[w][m][0] = dr_mul2(S[w][m][0], x.g[m].x);
+          S[w][m][1] = dr_mul2(S[w][m][1], x.g[m].y);
+          d01[w] = dr_fma2(S[w][m][0], x.k[m].x, d01[w]);
+          d23[w] = dr_fma2(S[w][m][1], x.k[m].y, d23[w]);
+          e01[w] = dr_fma2(S[w][m][0], x.q[m].x, e01[w]);
+          e23[w] = dr_fma2(S[w][m][1], x.q[m].y, e23[w]);
+        }
       fetch(ahead, j_ahead);
-      float dot = (dr_lo(d01) + dr_hi(d01)) + (dr_lo(d23) + dr_hi(d23));
-      float rd = (dr_lo(e01) + dr_hi(e01)) + (dr_lo(e23) + dr_hi(e23));
+      float dot[W], rd[W], u[W];
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        dot[w] = (dr_lo(d01[w]) + dr_hi(d01[w])) + (dr_lo(d23[w]) + dr_hi(d23[w]));
+        rd[w] = (dr_lo(e01[w]) + dr_hi(e01[w])) + (dr_lo(e23[w]) + dr_hi(e23[w]));
+      }
 #pragma unroll
       for (int p = 1; p < DR_PARTS; p *= 2) {
-        dot += __shfl_xor_sync(0xffffffffu, dot, p);
-        rd += __shfl_xor_sync(0xffffffffu, rd, p);
-      }
-      const float u = x.bq.x * (x.v - dot);
-      const uint64_t uu = dr_pack(u, u);
 #pragma unroll
-      for (int m = 0; m < G; ++m) {
-        S[m][0] = dr_fma2(x.k[m].x, uu, S[m][0]);
-        S[m][1] = dr_fma2(x.k[m].y, uu, S[m][1]);
+        for (int w = 0; w < W; ++w) dot[w] += __shfl_xor_sync(0xffffffffu, dot[w], p);
+#pragma unroll
+        for (int w = 0; w < W; ++w) rd[w] += __shfl_xor_sync(0xffffffffu, rd[w], p);
       }
-      if (writes) *o_next = fmaf(u, x.bq.y, rd);
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        u[w] = x.bq.x * (x.v[w] - dot[w]);
+        const uint64_t uu = dr_pack(u[w], u[w]);
+#pragma unroll
+        for (int m = 0; m < G; ++m) {
+          S[w][m][0] = dr_fma2(x.k[m].x, uu, S[w][m][0]);
+          S[w][m][1] = dr_fma2(x.k[m].y, uu, S[w][m][1]);
+        }
+        if (live[w] && part == 0) o_next[w] = fmaf(u[w], x.bq.y, rd[w]);
+      }
       o_next += o_step;
     };
     Token x0, x1;
@@ -450,16 +480,18 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
     b ^= 1;
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
-  if (live) {
 #pragma unroll
-    for (int m = 0; m < G; ++m)
+  for (int w = 0; w < W; ++w)
+    if (live[w]) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int i = STEP * m + 4 * part + 2 * e;
-        if (i < dk) S_g[(size_t)i * dv + col] = dr_lo(S[m][e]);
-        if (i + 1 < dk) S_g[(size_t)(i + 1) * dv + col] = dr_hi(S[m][e]);
-      }
-  }
+      for (int m = 0; m < G; ++m)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int i = STEP * m + 4 * part + 2 * e;
+          if (i < dk) S_g[(size_t)i * dv + col + w] = dr_lo(S[w][m][e]);
+          if (i + 1 < dk) S_g[(size_t)(i + 1) * dv + col + w] = dr_hi(S[w][m][e]);
+        }
+    }
 }
 
 // Steps of single tokens (decode), bound by reading and writing the states once: a block owns
@@ -612,24 +644,26 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
     hb_launch(delta_prepare_kernel<TA>, dim3((n_rows + 3) / 4), dim3(128), 0, stream, kqg, beta,
               (const TA*)qkv, qkv_ld, q_off, k_off, (const TA*)beta_raw, beta_ld, (const TA*)a_raw, a_ld,
               a_log, dt_bias, n_rows, heads, kv_heads, dk, dkp));
+  const bool alone = (long)n_seqs * heads * ((dv + DR_COLS - 1) / DR_COLS) <= DR_SMS;
   const int cols = dk <= 128 && (long)n_seqs * heads * ((dv + DR_COLS_WIDE - 1) / DR_COLS_WIDE) >= DR_WIDE_BLOCKS ? DR_COLS_WIDE : DR_COLS;
   dim3 grid(n_seqs, heads, (dv + cols - 1) / cols);
-#define HB_DR_LAUNCH_COLS(DKMAX, COLS)                                                            \
+#define HB_DR_LAUNCH_COLS(DKMAX, COLS, W)                                                            \
   HB_DISPATCH_DTYPE(act_dt, TA,                                                                   \
     const size_t smem = (2 * DR_CHUNK * 3 * DKMAX + 4 * DR_CHUNK + 2 * DR_CHUNK * COLS) * sizeof(float); \
     if (smem > 48 * 1024)                                                                         \
-      cudaFuncSetAttribute(delta_rule_kernel<TA, DKMAX, COLS>,                                    \
+      cudaFuncSetAttribute(delta_rule_kernel<TA, DKMAX, COLS, W>,                                 \
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-    delta_rule_kernel<TA, DKMAX, COLS><<<grid, dim3(COLS * DR_PARTS), smem, stream>>>(            \
+    delta_rule_kernel<TA, DKMAX, COLS, W><<<grid, dim3(COLS * DR_PARTS / W), smem, stream>>>(              \
         o, (const float*)kqg, (const float*)beta, (const TA*)qkv, qkv_ld, v_off, state,           \
         state_stride, cu_tokens, slots, heads, dk, dkp, dv))
 #define HB_DR_LAUNCH(DKMAX)                                                                       \
-  if (cols == DR_COLS) HB_DR_LAUNCH_COLS(DKMAX, DR_COLS);                                         \
-  else HB_DR_LAUNCH_COLS(DKMAX, DR_COLS_WIDE)
+  if (alone) HB_DR_LAUNCH_COLS(DKMAX, DR_COLS, 1);                                                \
+  else if (cols == DR_COLS) HB_DR_LAUNCH_COLS(DKMAX, DR_COLS, 2);                                 \
+  else HB_DR_LAUNCH_COLS(DKMAX, DR_COLS_WIDE, 2)
   if (dk <= 32) { HB_DR_LAUNCH(32); }
   else if (dk <= 64) { HB_DR_LAUNCH(64); }
   else if (dk <= 128) { HB_DR_LAUNCH(128); }
-  else HB_DR_LAUNCH_COLS(256, DR_COLS);
+  else HB_DR_LAUNCH_COLS(256, DR_COLS, 1);
 #undef HB_DR_LAUNCH_COLS
 #undef HB_DR_LAUNCH
   return hb_check_launch();
