@@ -322,7 +322,7 @@ HB_EXPORT int hb_latent_attention(void* out, const void* q_lat, long ql_t, long 
 // `latent_attention_merge` puts them together.
 #include "attention_mma.cuh"
 
-constexpr int LM_ROWS = 32, LM_KEYS = 32, LM_MAXNT = 16, LM_SPAD = 36, LM_PPAD = 40;
+constexpr int LM_KEYS = 32, LM_MAXNT = 16, LM_SPAD = 36, LM_PPAD = 40;
 
 // The factor on a row's accumulator: 1 / l, the sum relative to the maximum m (log2 domain), with the
 // sink's share in the sum where there is one.
@@ -336,8 +336,11 @@ __device__ __forceinline__ float latent_finish(float m, float l, const float* si
 // NTQ = rank / 32: the 8-column tiles of the latent a warp owns, a template parameter so that the
 // loops over them unroll without predicates (with a run-time count, integer arithmetic and
 // branches were most of the executed instructions and the tensor pipe a twentieth).
-template <int NTQ>
-__global__ void __launch_bounds__(256)
+// ROWS: query rows a block, 32 (two groups of four warps) or 16 (one): steps of single tokens with at
+// most 16 heads fill one group only, and without the other's rows two blocks fit an SM (16 heads, rows
+// of 576, with the merge, µs: 64 requests of 1,000 rows 53 -> 40, of 2,000 97 -> 69, 160 of 800 113 -> 93).
+template <int NTQ, int ROWS>
+__global__ void __launch_bounds__(8 * ROWS)
 latent_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_acc,
                             float* __restrict__ part_ml,
                             const __nv_bfloat16* __restrict__ q_lat, long ql_t, long ql_h,
@@ -353,14 +356,14 @@ latent_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__
   extern __shared__ __align__(16) unsigned char lm_smem[];
   const int D = rank + rot, RS = D + 8;
   __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lm_smem);      // [32][RS]
-  __nv_bfloat16* k_s = q_s + LM_ROWS * RS;                             // [2][32][RS]
+  __nv_bfloat16* k_s = q_s + ROWS * RS;                             // [2][32][RS]
   float* s_s = reinterpret_cast<float*>(k_s + 2 * LM_KEYS * RS);       // [32][LM_SPAD]
-  int* row_pos = reinterpret_cast<int*>(s_s + LM_ROWS * LM_SPAD);      // [32]
-  int* row_out = row_pos + LM_ROWS;                                    // [32]: token * heads + head, -1 for none
-  float* corr_s = reinterpret_cast<float*>(row_out + LM_ROWS);         // [32]
-  float* m_s = corr_s + LM_ROWS;                                       // [32]
-  float* l_s = m_s + LM_ROWS;                                          // [32]
-  __nv_bfloat16* p_s = reinterpret_cast<__nv_bfloat16*>(l_s + LM_ROWS);  // [32][LM_PPAD]
+  int* row_pos = reinterpret_cast<int*>(s_s + ROWS * LM_SPAD);      // [32]
+  int* row_out = row_pos + ROWS;                                    // [32]: token * heads + head, -1 for none
+  float* corr_s = reinterpret_cast<float*>(row_out + ROWS);         // [32]
+  float* m_s = corr_s + ROWS;                                       // [32]
+  float* l_s = m_s + ROWS;                                          // [32]
+  __nv_bfloat16* p_s = reinterpret_cast<__nv_bfloat16*>(l_s + ROWS);  // [32][LM_PPAD]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rg = warp >> 2, cq = warp & 3, g = lane >> 2, t4 = lane & 3;
@@ -379,7 +382,7 @@ latent_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__
   const int per = (n_kt - kt_first + n_splits - 1) / n_splits;
   const int kt_lo = kt_first + split * per, kt_hi = min(n_kt, kt_lo + per);
 
-  if (tid < LM_ROWS) {
+  if (tid < ROWS) {
     const int lt = tid / heads_per_block, h = h0 + tid % heads_per_block;
     const bool ok = lt < tokens_per_tile && t_first + lt < n_tok && h < heads;
     row_pos[tid] = ok ? start_pos[seq] + t_first + lt : -1;
@@ -390,7 +393,7 @@ latent_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__
   // tokens with 16 heads or fewer fill one group only)
   const bool group_live = row_out[rg * 16] >= 0;
   // a warp copies 4 query rows (index arithmetic once a row, not once a value)
-  for (int r = warp; r < LM_ROWS; r += 8) {
+  for (int r = warp; r < ROWS; r += ROWS / 4) {
     __nv_bfloat16* dst = q_s + r * RS;
     if (row_out[r] >= 0) {
       const int tg = row_out[r] / heads, h = row_out[r] - tg * heads;
@@ -404,7 +407,7 @@ latent_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__
   }
 
   // Lane r finds the row of key kt * 32 + r (its page from the block table); warp w then
-  // copies rows 4 w .. 4 w + 3 in 16-byte pieces, the row's start handed over by shuffles:
+  // copies its rows (4, or 8, from 4 w or 8 w on) in 16-byte pieces, the row's start handed over by shuffles:
   // no division per piece.  Rows beyond the last key, and before the first, are zero-filled.
   const int vec_per_row = D / 8;
   auto load_tile = [&](int kt, int buf) {
@@ -417,8 +420,8 @@ latent_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__
       row_off = ((long long)table[pg] * page_size + in_pg) * D;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = 4 * warp + i;
+    for (int i = 0; i < LM_KEYS / (ROWS / 4); ++i) {
+      const int r = LM_KEYS / (ROWS / 4) * warp + i;
       const long long off = __shfl_sync(0xffffffffu, row_off, r);
       const __nv_bfloat16* src = pages + (off < 0 ? 0 : off);
       __nv_bfloat16* drow = dst + r * RS;
@@ -626,35 +629,40 @@ HB_EXPORT int hb_latent_attention_mma(void* out, float* part_acc, float* part_ml
                                       const int* start_pos, int n_tokens, int heads,
                                       int heads_per_block, int tokens_per_tile, int rank, int rot,
                                       int page_size, float scale, int n_splits, int window, const float* sink,
-                                      cudaStream_t stream) {
+                                      int rows, cudaStream_t stream) {
   if (n_tiles <= 0 || n_tokens <= 0) return HB_OK;
   if (rank <= 0 || rank % 32 || rank > 32 * LM_MAXNT || rot < 0 || rot % 16 || heads <= 0 ||
-      heads_per_block <= 0 || heads_per_block > LM_ROWS || tokens_per_tile <= 0 ||
-      tokens_per_tile * heads_per_block > LM_ROWS || page_size <= 0 || n_splits <= 0 ||
+      (rows != 16 && rows != 32) || heads_per_block <= 0 || heads_per_block > rows || tokens_per_tile <= 0 ||
+      tokens_per_tile * heads_per_block > rows || page_size <= 0 || n_splits <= 0 ||
       n_splits > 32 || (n_splits > 1 && (part_acc == nullptr || part_ml == nullptr)))
     return HB_BAD_ARGUMENT;
   const int RS = rank + rot + 8;
-  const size_t smem = (size_t)3 * LM_ROWS * RS * 2 + (size_t)LM_ROWS * LM_SPAD * 4 + 5 * LM_ROWS * 4 +
-                      (size_t)LM_ROWS * LM_PPAD * 2;
+  const size_t smem = (size_t)(rows + 2 * LM_KEYS) * RS * 2 + (size_t)rows * LM_SPAD * 4 + 5 * rows * 4 +
+                      (size_t)rows * LM_PPAD * 2;
   if (smem > 220 * 1024) return HB_BAD_ARGUMENT;
   const int head_groups = (heads + heads_per_block - 1) / heads_per_block;
   int page_shift = -1;                               // log2 of a page size that is a power of two
   for (int b = 0; b < 31; ++b)
     if ((1 << b) == page_size) page_shift = b;
-  static size_t smem_set[LM_MAXNT + 1] = {};
-#define HB_LM_LAUNCH(N)                                                                              \
-  case N:                                                                                            \
-    if (smem > 48 * 1024 && smem > smem_set[N]) {                                                    \
-      if (cudaFuncSetAttribute(latent_attention_mma_kernel<N>,                                       \
+  static size_t smem_set[2][LM_MAXNT + 1] = {};
+#define HB_LM_LAUNCH_ROWS(N, R)                                                                      \
+  {                                                                                                  \
+    if (smem > 48 * 1024 && smem > smem_set[R == 16][N]) {                                           \
+      if (cudaFuncSetAttribute(latent_attention_mma_kernel<N, R>,                                    \
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
         return HB_LAUNCH_FAILED;                                                                     \
-      smem_set[N] = smem;                                                                            \
+      smem_set[R == 16][N] = smem;                                                                   \
     }                                                                                                \
-    hb_launch(latent_attention_mma_kernel<N>, dim3(n_tiles, head_groups, n_splits), dim3(256), smem, \
+    hb_launch(latent_attention_mma_kernel<N, R>, dim3(n_tiles, head_groups, n_splits), dim3(8 * R), smem, \
               stream, (__nv_bfloat16*)out, part_acc, part_ml, (const __nv_bfloat16*)q_lat, ql_t, ql_h, \
               (const __nv_bfloat16*)q_rot, qr_t, qr_h, (const __nv_bfloat16*)pages, block_table,     \
               bt_stride, q_tiles, cu_tokens, start_pos, heads, heads_per_block, tokens_per_tile, rank, \
               rot, page_size, page_shift, scale * 1.4426950408889634f, n_splits, window, sink);      \
+  }
+#define HB_LM_LAUNCH(N)                                                                              \
+  case N:                                                                                            \
+    if (rows == 16) HB_LM_LAUNCH_ROWS(N, 16)                                                         \
+    else HB_LM_LAUNCH_ROWS(N, 32)                                                                    \
     break;
   switch (rank / 32) {
     HB_LM_LAUNCH(1) HB_LM_LAUNCH(2) HB_LM_LAUNCH(3) HB_LM_LAUNCH(4) HB_LM_LAUNCH(5) HB_LM_LAUNCH(6)
@@ -663,6 +671,7 @@ HB_EXPORT int hb_latent_attention_mma(void* out, float* part_acc, float* part_ml
     default: return HB_BAD_ARGUMENT;
   }
 #undef HB_LM_LAUNCH
+#undef HB_LM_LAUNCH_ROWS
   if (n_splits > 1) {
     const int n_rows = n_tokens * heads;
     hb_launch(latent_attention_merge_kernel, dim3((n_rows + 3) / 4), dim3(128), 0, stream,

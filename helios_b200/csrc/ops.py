@@ -1974,18 +1974,32 @@ def latent_attention(ctx, q_lat: torch.Tensor, q_rot: torch.Tensor, pages: torch
             raise KernelError(f"{sink_values.numel()} sink values for {H} heads")
     out = torch.empty((T, H, rank), dtype=q_lat.dtype, device=q_lat.device)
     if LATENT_ATTENTION_TENSOR_CORES and q_lat.dtype == torch.bfloat16 and rank % 32 == 0 and rot % 16 == 0:
-        # 32 query rows a block: (token, head) pairs of one request, which share every key
-        hpb = min(H, 32)
-        tpt = max(1, 32 // hpb)
+        # 32 query rows a block: (token, head) pairs of one request, which share every key.  Steps of
+        # single tokens with at most 16 heads take 16 rows (four warps instead of eight, half of which
+        # would have no rows) where two such blocks then fit an SM and there are ranges of keys for more
+        # than the SMs.  32 rows / 16, microseconds: 64 requests of 1,000 rows of 576 53 / 40, 16 of 3,000
+        # 51 / 45, 24 of 1,000 32 / 32, 8 of 1,024 24 / 27; rows of 288, which fit twice as they are,
+        # 64 of 1,000 28 / 33.
+        max_keys = min(ctx.max_context_len, window) if window else ctx.max_context_len
+        row_bytes = 2 * (rank + rot + 8)
+        rows = 16 if T == len(ctx.seqs) and H <= 16 and 96 * row_bytes > 108 * 1024 \
+            and 80 * row_bytes <= 108 * 1024 and T * max(1, max_keys // 256) > sm_count() else 32
+        hpb = min(H, rows)
+        tpt = 1 if rows == 16 else rows // hpb
         tiles = _step_tiles(ctx, tpt, False, q_lat.device)
-        blocks = tiles.shape[0] * -(-H // hpb)
+        # (a captured step's list of tiles is longer than its work; of one token each there are T)
+        n_tiles = T if tpt == 1 and rows == 16 else tiles.shape[0]
+        blocks = n_tiles * -(-H // hpb)
+        slots = 2 * sm_count() if rows == 16 else sm_count()
         n_splits = 1
-        if blocks < sm_count():
+        if blocks < slots:
             keys = min(ctx.max_context_len, window + tpt - 1) if window else ctx.max_context_len
-            # ranges of at least 256 keys, or of 128 where all of those still have an SM each (a range
+            # ranges of at least 256 keys, or of 128 where all of those still have a place each (a range
             # walks its tiles one after the other; 8 requests, 1,024 keys each: 20.6 against 26.3 us)
-            least = 128 if blocks * (keys // 128) <= sm_count() else 256
-            n_splits = max(1, min(32, keys // least, -(-2 * sm_count() // blocks)))
+            least = 128 if blocks * (keys // 128) <= slots else 256
+            # 16 rows: all ranges at once; 32 rows: up to two rounds
+            most = slots // blocks if rows == 16 else -(-2 * slots // blocks)
+            n_splits = max(1, min(32, keys // least, most))
         part_acc = part_ml = None
         if n_splits > 1:
             part_acc = torch.empty((T * H, n_splits, rank), dtype=torch.float32, device=q_lat.device)
@@ -1993,11 +2007,11 @@ def latent_attention(ctx, q_lat: torch.Tensor, q_rot: torch.Tensor, pages: torch
         f = _fn("latent_attention", "hb_latent_attention_mma",
                 [c_void_p, c_void_p, c_void_p, c_void_p, _LONG, _LONG, c_void_p, _LONG, _LONG, c_void_p,
                  c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                 c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p])
+                 c_int, c_int, c_float, c_int, c_int, c_void_p, c_int, c_void_p])
         _run(f(_p(out), _p(part_acc), _p(part_ml), _p(q_lat), q_lat.stride(0), q_lat.stride(1), _p(q_rot),
                q_rot.stride(0), q_rot.stride(1), _p(pages), _p(block_table), block_table.shape[1],
-               _p(tiles), tiles.shape[0], _p(ctx.cu_tokens), _p(ctx.start_pos), T, H, hpb, tpt, rank, rot,
-               page_size, float(scale), n_splits, window, _p(sink_values), _stream()), "latent_attention_mma")
+               _p(tiles), n_tiles, _p(ctx.cu_tokens), _p(ctx.start_pos), T, H, hpb, tpt, rank, rot,
+               page_size, float(scale), n_splits, window, _p(sink_values), rows, _stream()), "latent_attention_mma")
         return out
     f = _fn("latent_attention", "hb_latent_attention",
             [c_void_p, c_void_p, _LONG, _LONG, c_void_p, _LONG, _LONG, c_void_p, c_void_p, c_int, c_void_p,

@@ -775,3 +775,39 @@ def test_norm_on_an_output_at_the_widths_its_rows_are_kept_at(H, y_dtype):
     torch.testing.assert_close(r.cpu().double(), want, atol=4e-6, rtol=4e-6)
     assert torch.equal(copy, r.to(torch.bfloat16))
     assert torch.equal(ops.rmsnorm_add(r, None, None, 0.0, torch.bfloat16), copy)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,rank,rot,count", [(16, 512, 64, 60), (11, 512, 64, 75), (1, 512, 96, 149), (16, 480, 112, 300)])
+@pytest.mark.parametrize("window", [None, 40, 700])
+def test_latent_attention_of_many_single_tokens_takes_sixteen_rows_a_block(heads, rank, rot, count, window):
+    """Rows wide enough that 32 query rows fill an SM, more ranges than SMs: contexts at the edges of
+    key tiles, one and more ranges a request, a window, a sink; against the kernel with a warp a row."""
+    from types import SimpleNamespace
+    from helios_b200.csrc import ops
+    from helios_b200.engine.batch import SeqSlice
+
+    dev, page = "cuda", 16
+    g = torch.Generator().manual_seed(heads + count)
+    lens = [(1, 2, 31, 32, 33, 300, 1000)[i % 7] for i in range(count)]
+    width, n_pages = 63, 200
+    table = torch.stack([torch.randperm(n_pages, generator=g)[:width] for _ in lens]).int()
+    pages = (torch.randn(n_pages, 1, page, rank + rot, generator=g) * 0.5).to(torch.bfloat16).to(dev)
+    q = (torch.randn(count, heads, rank + rot, generator=g) * 0.7).to(torch.bfloat16).to(dev)
+    sink = (torch.randn(heads, generator=g) * 2).to(dev) if window == 700 else None
+    start = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=dev)
+    ctx = SimpleNamespace(seq_of_token=torch.arange(count, dtype=torch.int32, device=dev), positions=start, start_pos=start,
+                          cu_tokens=torch.arange(count + 1, dtype=torch.int32, device=dev), extras={}, num_seqs=count,
+                          seqs=[SeqSlice(None, 0, n - 1, 1, i) for i, n in enumerate(lens)], max_context_len=1000)
+    call = lambda: ops.latent_attention(ctx, q[:, :, :rank], q[:, :, rank:], pages, table.to(dev), rank, rot, page, 0.3,
+                                        window, sink).float()
+    got = call()
+    ops.LATENT_ATTENTION_TENSOR_CORES = False
+    try:
+        want = call()
+    finally:
+        ops.LATENT_ATTENTION_TENSOR_CORES = True
+    assert torch.isfinite(got).all()
+    # weights and results have 8 bits: two results of at most about 1.5 in size, each within 2^-8 of it
+    torch.testing.assert_close(got, want, atol=1.6e-2, rtol=1.6e-2)
+
