@@ -51,7 +51,8 @@ LIBRARIES: Dict[str, str] = {
 }
 _HEADERS = ["common.cuh", "tcgen05.cuh"]
 # further files a library's source includes
-_INCLUDES: Dict[str, List[str]] = {"gemm_bf16_noalloc": ["gemm_bf16.cu", "gemm_bf16_noalloc.h"],
+_INCLUDES: Dict[str, List[str]] = {"gemm_bf16": ["gemv_bf16.cuh"],
+                                   "gemm_bf16_noalloc": ["gemm_bf16.cu", "gemm_bf16_noalloc.h"],
                                    "attention_bf16": ["attention_mma.cuh", "attention_options.cuh", "attention_decode.cuh"],
                                    "attention_pooled": ["attention_mma.cuh", "attention_options.cuh",
                                                         "attention_decode.cuh"],

@@ -912,6 +912,8 @@ int max_clusters(int cluster_size) {
 }  // namespace
 
 #ifndef HB_GEMM_BF16_NO_EXPORTS
+#include "gemv_bf16.cuh"
+
 // Resident clusters of `cluster_size` blocks for the kernel variant a call would use
 // (-1 if the query fails).
 HB_EXPORT int hb_gemm_bf16_max_clusters(int swap_bn, int glu, int cluster_size) {

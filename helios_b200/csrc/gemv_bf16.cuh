@@ -1,0 +1,179 @@
+// Products of one to four tokens with a small weight matrix, on the FMA pipes: y[t, n] = x[t] . w[n],
+// with the epilogues that decode steps use of the tensor-core kernel (same meaning, see there).
+//
+// A step of a small model is a chain of such products, each over in less time than the tensor-core
+// kernel takes around its sums (barriers, tensor memory, copies through shared memory, a cluster's
+// two barriers).  Here a warp takes two rows of w, a lane 16 bytes of a row at a time, straight into
+// registers, and asks for its first rows before the kernel before is done, as the tensor-core
+// kernel does; then x, the sums, one barrier, and 16 features x tokens finish, a thread each.  A block
+// has 16 features: they share a slot of the sums of squares (eight slots to 128 features, as the
+// tensor-core kernel leaves them).  Long rows are split over two warps.  Chains over cold weights,
+// tensor cores / this, µs at one token: 1,152 x 896 4.95 / 2.30, 896 x 896 4.05 / 2.18, 896 x 4,864
+// 6.06 / 5.08, 2,048 x 8,192 9.98 / 8.62.  (Gated units, four rows a warp, were not ahead: 4,864 x 896
+// 6.36 / 7.30; they stay there.)
+#pragma once
+#include "common.cuh"
+
+namespace {
+
+struct GemvArgs {
+  void* out;                   // [T, ldo] bfloat16 or float32
+  const __nv_bfloat16* x;      // [T, ldx]
+  const __nv_bfloat16* w;      // [N or 2 N, ldw]
+  const float* bias;
+  float* residual;
+  const float* norm_weight;
+  float* sumsq_out;            // [T, slots_out]
+  const float* sumsq_in;       // [T, slots_in]
+  int T, N, K, ldx, ldw, ldo, out_f32, slots_in, slots_out;
+  float eps;
+};
+
+constexpr int GEMV_F = 16;     // features a block
+
+__device__ __forceinline__ float gemv_dot8(const uint4& a, const uint4& b, float acc) {
+  const uint32_t u[4] = {a.x, a.y, a.z, a.w}, v[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    acc = fmaf(__uint_as_float(u[i] << 16), __uint_as_float(v[i] << 16), acc);
+    acc = fmaf(__uint_as_float(u[i] & 0xffff0000u), __uint_as_float(v[i] & 0xffff0000u), acc);
+  }
+  return acc;
+}
+
+// TT: tokens (T <= TT); KS: warps that share a row
+template <int TT, int KS>
+__global__ void __launch_bounds__(256 * KS)
+gemv_bf16_kernel(GemvArgs a) {
+  constexpr int ROWS = 2, PRE = 4;               // rows a warp; 256-element steps a register buffer holds
+  __shared__ float part[KS][TT][GEMV_F];
+  __shared__ float scale[TT];
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ks = warp >> 3, f0 = 2 * (warp & 7), n0 = blockIdx.x * GEMV_F;
+  const int steps = (a.K + 255) / 256;
+  uint4 w[2][PRE][ROWS];
+  auto load_w = [&](uint4 (&buf)[PRE][ROWS], int s0) {      // this warp's steps s0 .. s0 + PRE - 1
+#pragma unroll
+    for (int i = 0; i < PRE; ++i) {
+      const int k = ((s0 + i) * KS + ks) * 256 + 8 * lane;
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int n = n0 + f0 + r;
+        buf[i][r] = (k < a.K && n < a.N) ? __ldg(reinterpret_cast<const uint4*>(a.w + (size_t)n * a.ldw + k))
+                                         : make_uint4(0, 0, 0, 0);
+      }
+    }
+  };
+  float acc[ROWS][TT];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+    for (int t = 0; t < TT; ++t) acc[r][t] = 0.f;
+  auto multiply = [&](const uint4 (&buf)[PRE][ROWS], int s0) {
+    uint4 x[PRE][TT];
+#pragma unroll
+    for (int i = 0; i < PRE; ++i) {
+      const int k = ((s0 + i) * KS + ks) * 256 + 8 * lane;
+#pragma unroll
+      for (int t = 0; t < TT; ++t)
+        x[i][t] = (k < a.K && t < a.T) ? __ldcg(reinterpret_cast<const uint4*>(a.x + (size_t)t * a.ldx + k))
+                                       : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < PRE; ++i)
+#pragma unroll
+      for (int t = 0; t < TT; ++t)
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) acc[r][t] = gemv_dot8(buf[i][r], x[i][t], acc[r][t]);
+  };
+  const int mine = (steps - ks + KS - 1) / KS;             // steps of this warp
+  load_w(w[0], 0);
+  load_w(w[1], PRE);
+  pdl_wait();
+  // what a finishing thread needs from memory beyond the sums goes out under them
+  const int et = tid >> 4, ef = tid & 15, en = n0 + ef;
+  const bool finishes = tid < TT * GEMV_F && et < a.T && en < a.N;
+  float old = 0.f, bias_n = 0.f, weight_n = 0.f;
+  if (finishes) {
+    if (a.residual) old = __ldcg(a.residual + (size_t)et * a.N + en);
+    if (a.bias) bias_n = a.bias[en];
+    if (a.norm_weight) weight_n = a.norm_weight[en];
+  }
+  float squares = 0.f;
+  if (a.sumsq_in && warp < a.T) {
+#pragma unroll 4
+    for (int j = lane; j < a.slots_in; j += 32) squares += __ldcg(a.sumsq_in + (size_t)warp * a.slots_in + j);
+  }
+  for (int s = 0; s < mine; s += 2 * PRE) {
+    multiply(w[0], s);
+    if (s + 2 * PRE < mine) load_w(w[0], s + 2 * PRE);
+    if (s + PRE < mine) {
+      multiply(w[1], s + PRE);
+      if (s + 3 * PRE < mine) load_w(w[1], s + 3 * PRE);
+    }
+  }
+  if (a.sumsq_in && warp < a.T) {
+    squares = warp_sum(squares);
+    if (lane == 0) scale[warp] = rsqrtf(squares / (float)a.K + a.eps);
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+    for (int t = 0; t < TT; ++t) {
+      const float v = warp_sum(acc[r][t]);
+      if (lane == 0) part[ks][t][f0 + r] = v;
+    }
+  __syncthreads();
+  if (tid >= TT * GEMV_F) return;                          // whole warps but for TT = 1: half a warp stays
+  float val = 0.f;
+#pragma unroll
+  for (int i = 0; i < KS; ++i) val += part[i][et][ef];
+  if (a.sumsq_in && et < a.T) val *= scale[et];
+  val += bias_n;
+  if (a.residual) {
+    val += old;
+    if (finishes) a.residual[(size_t)et * a.N + en] = val;
+    if (a.norm_weight) {
+      if (finishes) reinterpret_cast<__nv_bfloat16*>(a.out)[(size_t)et * a.ldo + en] = __float2bfloat16_rn(val * weight_n);
+      float sq = finishes ? val * val : 0.f;
+      const uint32_t lanes = TT == 1 ? 0xffffu : 0xffffffffu;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(lanes, sq, o);
+      if (ef == 0 && et < a.T) a.sumsq_out[(size_t)et * a.slots_out + blockIdx.x] = sq;
+    }
+  } else if (finishes) {
+    if (a.out_f32) reinterpret_cast<float*>(a.out)[(size_t)et * a.ldo + en] = val;
+    else reinterpret_cast<__nv_bfloat16*>(a.out)[(size_t)et * a.ldo + en] = __float2bfloat16_rn(val);
+  }
+}
+
+template <int TT>
+int launch_gemv(const GemvArgs& a, cudaStream_t stream) {
+  // with sums of squares all slots of the last 128 features are written
+  const int features = a.sumsq_out ? (a.N + 127) / 128 * 128 : a.N;
+  const dim3 grid((features + GEMV_F - 1) / GEMV_F);
+  if (a.K > 2048) hb_launch(gemv_bf16_kernel<TT, 2>, grid, dim3(512), 0, stream, a);
+  else hb_launch(gemv_bf16_kernel<TT, 1>, grid, dim3(256), 0, stream, a);
+  return hb_check_launch();
+}
+
+}  // namespace
+
+// As hb_gemm_bf16_fused without a gated unit, for 1 to 4 tokens; rows of x and w in whole 16-byte pieces.
+HB_EXPORT int hb_gemv_bf16(void* out, const void* x, const void* w, const float* bias, int T, int N, int K, int ldx,
+                           int ldw, int ldo, int out_f32, float* residual,
+                           const float* norm_weight, float* sumsq_out, const float* sumsq_in, int slots_in, float eps,
+                           cudaStream_t stream) {
+  if (T <= 0 || N <= 0) return HB_OK;
+  if (T > 4 || K <= 0 || K % 8 || ldx % 8 || ldw % 8 ||
+      (residual && out_f32) || (norm_weight && (!residual || !sumsq_out || !out)) || (!residual && !out) ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15))
+    return HB_BAD_ARGUMENT;
+  GemvArgs a;
+  a.out = out; a.x = (const __nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.bias = bias;
+  a.residual = residual; a.norm_weight = norm_weight; a.sumsq_out = norm_weight ? sumsq_out : nullptr;
+  a.sumsq_in = sumsq_in; a.T = T; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldo = ldo;
+  a.out_f32 = out_f32; a.slots_in = slots_in; a.slots_out = 8 * ((N + 127) / 128); a.eps = eps;
+  return T == 1 ? launch_gemv<1>(a, stream) : T == 2 ? launch_gemv<2>(a, stream) : launch_gemv<4>(a, stream);
+}

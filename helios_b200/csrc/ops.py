@@ -681,6 +681,14 @@ def tc_gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
 GLU_EPILOGUES = {False: 0, True: 1, "silu": 1, "gelu_tanh": 2}
 
 
+#: Plain products of so many tokens with a weight matrix of at most so many bytes run on the FMA pipes
+#: (``gemv_bf16.cuh``).  Tensor cores / FMA pipes, microseconds, chains over cold weights.  One token:
+#: 2 MB 4.95 / 2.30, 9 MB 6.06 / 5.08, 33 MB 9.98 / 8.62 and 9.22 / 8.86, 117 MB 22.5 / 24.9.  Two: 2 MB
+#: 4.99 / 2.64, 9 MB 6.15 / 6.27, 13 MB 6.40 / 5.97, 27 MB 9.41 / 10.6.  Four: 2 MB 4.74 / 3.54, 3 MB
+#: 4.01 / 3.93, 6 MB 4.86 / 6.01.
+GEMV_WEIGHT_BYTES = {1: 36 << 20, 2: 13 << 20, 3: 3 << 20, 4: 3 << 20}
+
+
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
                 glu=False, out_dtype: torch.dtype = torch.bfloat16,
                 plan=None, cluster: Optional[bool] = None, two_sm: Optional[bool] = None,
@@ -757,6 +765,17 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         out = torch.empty((T, N), dtype=out_dtype, device=x.device)
     if T == 0:
         return out if residual is None else ((out, sumsq_out) if norm_weight is not None else None)
+    if plan is None and not glu and rows * K * 2 <= GEMV_WEIGHT_BYTES.get(T, 0) \
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0:
+        f = _fn("gemm_bf16", "hb_gemv_bf16",
+                [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                 c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
+        _run(f(_p(out), _p(x), _p(weight), _p(bias), T, N, K, K, K, N, 1 if out_dtype == torch.float32 else 0,
+               _p(residual), _p(norm_weight), _p(sumsq_out), _p(sumsq), 0 if sumsq is None else sumsq.shape[1],
+               float(eps), _stream()), "gemv_bf16")
+        if residual is not None:
+            return (out, sumsq_out) if norm_weight is not None else None
+        return out
     bn, splits = plan if plan is not None else gemm_plan(T, N, K, bool(glu))
     if few and (bn == 0 or T > bn):
         raise KernelError("the residual and 1 / rms epilogues need the swapped orientation and one token tile")

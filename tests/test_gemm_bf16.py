@@ -221,3 +221,39 @@ def test_float32_output_of_the_two_sm_kernel_at_odd_widths(T, N):
     x, w, _b = _case(T, N, 136, T * N)
     got = ops().linear_bf16(x.to(DEV), w.to(DEV), plan=(0, 1), two_sm=True, out_dtype=torch.float32)
     torch.testing.assert_close(got.double().cpu(), x.double() @ w.double().T, atol=2e-3, rtol=1e-3)
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(16, 8), (100, 248), (129, 256), (896, 264), (1152, 896), (17, 2048), (250, 2056), (896, 4864)])
+def test_products_of_few_tokens_with_a_small_weight(T, N, K, monkeypatch):
+    """Every epilogue of the kernel on the FMA pipes against float64: one and two warps a row, rows that
+    end inside a step of 256, features that end inside a block and inside a slot of the squares."""
+    o = ops()
+    monkeypatch.setattr(o, "GEMV_WEIGHT_BYTES", {1: 1 << 30, 2: 1 << 30, 3: 1 << 30, 4: 1 << 30})
+    x, w, b = _case(T, N, K, T + N + K)
+    xd, wd, bd = x.to(DEV), w.to(DEV), b.to(DEV)
+    want = x.double() @ w.double().T
+    _close(o.linear_bf16(xd, wd), want)
+    _close(o.linear_bf16(xd, wd, bd), want + b.double())
+    # float32 out: K products, each sum of 8 * K / 256 + 6 roundings
+    bound = (K / 32 + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1e-6
+    assert ((o.linear_bf16(xd, wd, out_dtype=torch.float32).double().cpu() - want).abs() <= bound).all()
+    g = torch.Generator().manual_seed(K)
+    slots = torch.rand(T, 8 * -(-K // 128), generator=g)
+    inv = torch.rsqrt(slots.double().sum(-1, keepdim=True) / K + 1e-5)
+    _close(o.linear_bf16(xd, wd, bd, sumsq=slots.to(DEV), eps=1e-5), want * inv + b.double(), scale=float(inv.max()) + 1)
+    res, nw = torch.randn(T, N, generator=g), torch.rand(N, generator=g) + 0.5
+    r1 = res.to(DEV)
+    assert o.linear_bf16(xd, wd, residual=r1) is None
+    assert ((r1.double().cpu() - res.double() - want).abs() <= bound + 1e-6).all()
+    r2 = res.to(DEV)
+    scaled, squares = o.linear_bf16(xd, wd, bd, residual=r2, norm_weight=nw.to(DEV))
+    assert ((r2.double().cpu() - res.double() - want - b.double()).abs() <= bound + 1e-6).all()
+    assert torch.equal(scaled.cpu(), (r2.cpu() * nw).to(torch.bfloat16))
+    torch.testing.assert_close(squares.double().cpu().sum(-1), (r2.double().cpu() ** 2).sum(-1), rtol=1e-5, atol=1e-6)
+    # the same through the tensor-core kernel, and a row alone is the row in the batch
+    first = o.linear_bf16(xd, wd, out_dtype=torch.float32)
+    assert torch.equal(o.linear_bf16(xd[T - 1:].contiguous(), wd, out_dtype=torch.float32), first[T - 1:])
+    monkeypatch.setattr(o, "GEMV_WEIGHT_BYTES", {})
+    torch.testing.assert_close(o.linear_bf16(xd, wd, out_dtype=torch.float32), first, atol=2e-4, rtol=1e-4)
+
