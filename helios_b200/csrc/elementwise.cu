@@ -493,40 +493,12 @@ HB_EXPORT int hb_rope_kv_write(void* qkv, const float* cos_tab, const float* sin
   return hb_check_launch();
 }
 
-// ---------------------------------------------------------------- SwiGLU gate
-// out[t, i] = silu(gu[t, i]) * gu[t, I + i]        python/helios/exec/model.py:336-337
-template <typename T>
-__global__ void silu_mul_kernel(T* __restrict__ out, const T* __restrict__ gu, size_t total, int I) {
-  pdl_launch_dependents();
-  pdl_wait();
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const size_t t = idx / I;
-    const int i = (int)(idx - t * I);
-    const float g = to_float(gu[t * 2 * I + i]);
-    const float u = to_float(gu[t * 2 * I + I + i]);
-    out[idx] = from_float<T>(g / (1.f + expf(-g)) * u);
-  }
-}
-
-HB_EXPORT int hb_silu_mul(void* out, const void* gate_up, int T, int I, int act_dt,
-                          cudaStream_t stream) {
-  if (T <= 0) return HB_OK;
-  const size_t total = (size_t)T * I;
-  const int threads = 256;
-  size_t blocks = (total + threads - 1) / threads;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  HB_DISPATCH_DTYPE(act_dt, TA,
-    hb_launch(silu_mul_kernel<TA>, dim3((unsigned)blocks), dim3(threads), 0, stream, (TA*)out, (const TA*)gate_up, total, I));
-  return hb_check_launch();
-}
-
-
 // ---------------------------------------------------------------- gated activations
 // out[t, i] = act(gu[t, i]) * gu[t, I + i] for a feed-forward whose gate and up rows come
 // out of one product.  kind 0: silu(g) * u.  kind 1: the tanh form of gelu,
 // 0.5 g (1 + tanh(sqrt(2/pi) (g + 0.044715 g^3))) * u.  kind 2: the clamped form
 // g' = min(g, limit), u' = clamp(u, -limit, limit), g' sigmoid(1.702 g') (u' + 1).
+// (silu: python/helios/exec/model.py:336-337)
 enum { HB_GLU_SILU = 0, HB_GLU_GELU_TANH = 1, HB_GLU_CLAMPED_SWISH = 2 };
 
 __device__ __forceinline__ float glu_value(float g, float u, int kind, float limit) {
@@ -598,6 +570,12 @@ HB_EXPORT int hb_glu_act(void* out, const void* gate_up, int T, int I, int kind,
     hb_launch(glu_act_kernel<TA>, dim3((unsigned)blocks), dim3(threads), 0, stream, (TA*)out,
               (const TA*)gate_up, total, I, kind, limit));
   return hb_check_launch();
+}
+
+// silu(gate) * up.  (Value by value, with a 64-bit division each, this took 5.0 µs for 224 rows of
+// 4,864 bfloat16 values where eight at a time take 3.1.)
+HB_EXPORT int hb_silu_mul(void* out, const void* gate_up, int T, int I, int act_dt, cudaStream_t stream) {
+  return hb_glu_act(out, gate_up, T, I, HB_GLU_SILU, 0.f, act_dt, stream);
 }
 
 // ---------------------------------------------------------------- norm on a sublayer's output
