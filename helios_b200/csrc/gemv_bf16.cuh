@@ -3,14 +3,15 @@
 //
 // A step of a small model is a chain of such products, each over in less time than the tensor-core
 // kernel takes around its sums (barriers, tensor memory, copies through shared memory, a cluster's
-// two barriers).  Here a warp takes two rows of w, a lane 16 bytes of a row at a time, straight into
-// registers, and asks for its first rows before the kernel before is done, as the tensor-core
+// two barriers).  Here a warp takes two rows of w (four for a gated unit, two features' gate and up
+// rows), a lane 16 bytes of a row at a time, straight into registers, and asks for its first rows before the kernel before is done, as the tensor-core
 // kernel does; then x, the sums, one barrier, and 16 features x tokens finish, a thread each.  A block
 // has 16 features: they share a slot of the sums of squares (eight slots to 128 features, as the
 // tensor-core kernel leaves them).  Long rows are split over two warps.  Chains over cold weights,
 // tensor cores / this, µs at one token: 1,152 x 896 4.95 / 2.30, 896 x 896 4.05 / 2.18, 896 x 4,864
-// 6.06 / 5.08, 2,048 x 8,192 9.98 / 8.62.  (Gated units, four rows a warp, were not ahead: 4,864 x 896
-// 6.36 / 7.30; they stay there.)
+// 6.06 / 5.08, 2,048 x 8,192 9.98 / 8.62.  Gated units of one token and 17 MB of weights are level alone
+// (2 x 4,096 x 1,024 5.9 / 5.7, 2 x 4,864 x 896 6.4 / 7.3) and ahead in a step, between kernels of this
+// kind (24 layers of Qwen2.5-0.5B sizes 608 / 593); larger ones are behind.
 #pragma once
 #include "common.cuh"
 
@@ -25,7 +26,7 @@ struct GemvArgs {
   const float* norm_weight;
   float* sumsq_out;            // [T, slots_out]
   const float* sumsq_in;       // [T, slots_in]
-  int T, N, K, ldx, ldw, ldo, out_f32, slots_in, slots_out;
+  int T, N, K, ldx, ldw, ldo, up_row, out_f32, slots_in, slots_out;
   float eps;
 };
 
@@ -41,12 +42,14 @@ __device__ __forceinline__ float gemv_dot8(const uint4& a, const uint4& b, float
   return acc;
 }
 
-// TT: tokens (T <= TT); KS: warps that share a row
-template <int TT, int KS>
+// TT: tokens (T <= TT); KS: warps that share a row; EPI: EPI_STORE, EPI_GLU or EPI_GELU
+template <int TT, int KS, int EPI>
 __global__ void __launch_bounds__(256 * KS)
 gemv_bf16_kernel(GemvArgs a) {
-  constexpr int ROWS = 2, PRE = 4;               // rows a warp; 256-element steps a register buffer holds
-  __shared__ float part[KS][TT][GEMV_F];
+  constexpr bool GATED = EPI != EPI_STORE;
+  constexpr int ROWS = GATED ? 4 : 2;            // rows a warp: features f, f + 1, then their up rows
+  constexpr int PRE = GATED ? 2 : 4;             // 256-element steps a register buffer holds
+  __shared__ float part[KS][ROWS / 2][TT][GEMV_F];
   __shared__ float scale[TT];
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -59,8 +62,9 @@ gemv_bf16_kernel(GemvArgs a) {
       const int k = ((s0 + i) * KS + ks) * 256 + 8 * lane;
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {
-        const int n = n0 + f0 + r;
-        buf[i][r] = (k < a.K && n < a.N) ? __ldg(reinterpret_cast<const uint4*>(a.w + (size_t)n * a.ldw + k))
+        const int n = n0 + f0 + (r & 1);
+        const size_t row = (size_t)(n + (r >= 2 ? a.up_row : 0));
+        buf[i][r] = (k < a.K && n < a.N) ? __ldg(reinterpret_cast<const uint4*>(a.w + row * a.ldw + k))
                                          : make_uint4(0, 0, 0, 0);
       }
     }
@@ -122,14 +126,21 @@ gemv_bf16_kernel(GemvArgs a) {
 #pragma unroll
     for (int t = 0; t < TT; ++t) {
       const float v = warp_sum(acc[r][t]);
-      if (lane == 0) part[ks][t][f0 + r] = v;
+      if (lane == 0) part[ks][r >> 1][t][f0 + (r & 1)] = v;
     }
   __syncthreads();
   if (tid >= TT * GEMV_F) return;                          // whole warps but for TT = 1: half a warp stays
-  float val = 0.f;
+  float val = 0.f, up = 0.f;
 #pragma unroll
-  for (int i = 0; i < KS; ++i) val += part[i][et][ef];
-  if (a.sumsq_in && et < a.T) val *= scale[et];
+  for (int i = 0; i < KS; ++i) {
+    val += part[i][0][et][ef];
+    if (GATED) up += part[i][ROWS / 2 - 1][et][ef];
+  }
+  if (a.sumsq_in && et < a.T) {
+    val *= scale[et];
+    up *= scale[et];
+  }
+  if (GATED) val = finishes ? glu_value<EPI>(val, up) : 0.f;
   val += bias_n;
   if (a.residual) {
     val += old;
@@ -148,32 +159,34 @@ gemv_bf16_kernel(GemvArgs a) {
   }
 }
 
-template <int TT>
+template <int TT, int EPI>
 int launch_gemv(const GemvArgs& a, cudaStream_t stream) {
   // with sums of squares all slots of the last 128 features are written
   const int features = a.sumsq_out ? (a.N + 127) / 128 * 128 : a.N;
   const dim3 grid((features + GEMV_F - 1) / GEMV_F);
-  if (a.K > 2048) hb_launch(gemv_bf16_kernel<TT, 2>, grid, dim3(512), 0, stream, a);
-  else hb_launch(gemv_bf16_kernel<TT, 1>, grid, dim3(256), 0, stream, a);
+  if (a.K > 2048) hb_launch(gemv_bf16_kernel<TT, 2, EPI>, grid, dim3(512), 0, stream, a);
+  else hb_launch(gemv_bf16_kernel<TT, 1, EPI>, grid, dim3(256), 0, stream, a);
   return hb_check_launch();
 }
 
 }  // namespace
 
-// As hb_gemm_bf16_fused without a gated unit, for 1 to 4 tokens; rows of x and w in whole 16-byte pieces.
+// As hb_gemm_bf16_fused, for 1 to 4 tokens (one with a gated unit); rows of x and w in whole 16-byte pieces.
 HB_EXPORT int hb_gemv_bf16(void* out, const void* x, const void* w, const float* bias, int T, int N, int K, int ldx,
-                           int ldw, int ldo, int out_f32, float* residual,
+                           int ldw, int ldo, int glu, int up_row, int out_f32, float* residual,
                            const float* norm_weight, float* sumsq_out, const float* sumsq_in, int slots_in, float eps,
                            cudaStream_t stream) {
   if (T <= 0 || N <= 0) return HB_OK;
-  if (T > 4 || K <= 0 || K % 8 || ldx % 8 || ldw % 8 ||
-      (residual && out_f32) || (norm_weight && (!residual || !sumsq_out || !out)) || (!residual && !out) ||
+  if (T > 4 || K <= 0 || K % 8 || ldx % 8 || ldw % 8 || glu < 0 || glu > 2 ||
+      (glu && (T > 1 || bias || residual || out_f32)) || (residual && out_f32) || (norm_weight && (!residual || !sumsq_out || !out)) || (!residual && !out) ||
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15))
     return HB_BAD_ARGUMENT;
   GemvArgs a;
   a.out = out; a.x = (const __nv_bfloat16*)x; a.w = (const __nv_bfloat16*)w; a.bias = bias;
   a.residual = residual; a.norm_weight = norm_weight; a.sumsq_out = norm_weight ? sumsq_out : nullptr;
-  a.sumsq_in = sumsq_in; a.T = T; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldo = ldo;
+  a.sumsq_in = sumsq_in; a.T = T; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldo = ldo; a.up_row = up_row;
   a.out_f32 = out_f32; a.slots_in = slots_in; a.slots_out = 8 * ((N + 127) / 128); a.eps = eps;
-  return T == 1 ? launch_gemv<1>(a, stream) : T == 2 ? launch_gemv<2>(a, stream) : launch_gemv<4>(a, stream);
+  if (glu) return glu == 1 ? launch_gemv<1, EPI_GLU>(a, stream) : launch_gemv<1, EPI_GELU>(a, stream);
+  return T == 1 ? launch_gemv<1, EPI_STORE>(a, stream)
+       : T == 2 ? launch_gemv<2, EPI_STORE>(a, stream) : launch_gemv<4, EPI_STORE>(a, stream);
 }

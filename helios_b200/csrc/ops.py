@@ -687,6 +687,8 @@ GLU_EPILOGUES = {False: 0, True: 1, "silu": 1, "gelu_tanh": 2}
 #: 4.99 / 2.64, 9 MB 6.15 / 6.27, 13 MB 6.40 / 5.97, 27 MB 9.41 / 10.6.  Four: 2 MB 4.74 / 3.54, 3 MB
 #: 4.01 / 3.93, 6 MB 4.86 / 6.01.
 GEMV_WEIGHT_BYTES = {1: 36 << 20, 2: 13 << 20, 3: 3 << 20, 4: 3 << 20}
+#: ... and gated units of one token with a weight of at most so many bytes
+GEMV_GATED_WEIGHT_BYTES = 18 << 20
 
 
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -765,12 +767,14 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         out = torch.empty((T, N), dtype=out_dtype, device=x.device)
     if T == 0:
         return out if residual is None else ((out, sumsq_out) if norm_weight is not None else None)
-    if plan is None and not glu and rows * K * 2 <= GEMV_WEIGHT_BYTES.get(T, 0) \
+    gemv_bytes = (GEMV_GATED_WEIGHT_BYTES if T == 1 and out_dtype == torch.bfloat16 else 0) if glu \
+        else GEMV_WEIGHT_BYTES.get(T, 0)
+    if plan is None and rows * K * 2 <= gemv_bytes \
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0:
         f = _fn("gemm_bf16", "hb_gemv_bf16",
-                [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                 c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
-        _run(f(_p(out), _p(x), _p(weight), _p(bias), T, N, K, K, K, N, 1 if out_dtype == torch.float32 else 0,
+                [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                 c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
+        _run(f(_p(out), _p(x), _p(weight), _p(bias), T, N, K, K, K, N, glu_code, N if glu else 0, 1 if out_dtype == torch.float32 else 0,
                _p(residual), _p(norm_weight), _p(sumsq_out), _p(sumsq), 0 if sumsq is None else sumsq.shape[1],
                float(eps), _stream()), "gemv_bf16")
         if residual is not None:

@@ -257,3 +257,18 @@ def test_products_of_few_tokens_with_a_small_weight(T, N, K, monkeypatch):
     monkeypatch.setattr(o, "GEMV_WEIGHT_BYTES", {})
     torch.testing.assert_close(o.linear_bf16(xd, wd, out_dtype=torch.float32), first, atol=2e-4, rtol=1e-4)
 
+
+@pytest.mark.parametrize("kind", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("N,K", [(16, 8), (100, 248), (129, 256), (4864, 896), (17, 2048), (250, 2056), (64, 4864)])
+def test_gated_units_of_one_token_with_a_small_weight(N, K, kind):
+    """As above, with and without the token's 1 / rms; gate and up rows of a feature end together."""
+    o = ops()
+    assert 2 * N * K * 2 <= o.GEMV_GATED_WEIGHT_BYTES
+    x, w, _b = _case(1, N, K, N + K, glu=True)
+    both = x.double() @ w.double().T
+    _close(o.linear_bf16(x.to(DEV), w.to(DEV), glu=kind), _gated(both[:, :N], both[:, N:], kind))
+    slots = torch.rand(1, 8 * -(-K // 128), generator=torch.Generator().manual_seed(K))
+    both = both * torch.rsqrt(slots.double().sum(-1, keepdim=True) / K + 1e-5)
+    got = o.linear_bf16(x.to(DEV), w.to(DEV), glu=kind, sumsq=slots.to(DEV), eps=1e-5).double().cpu()
+    # one rounding to eight bits, after sums of 32 bits
+    torch.testing.assert_close(got, _gated(both[:, :N], both[:, N:], kind), rtol=2.0 ** -8, atol=1e-4)
