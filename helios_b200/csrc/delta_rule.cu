@@ -74,6 +74,11 @@ causal_conv_silu_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloa
        idx += (size_t)gridDim.x * blockDim.x) {
     const int tg = (int)(idx / pieces), c = (int)(idx - (size_t)tg * pieces) * 8;
     const int t0 = tg * CONV_TOKENS;
+    // where the tokens stand in their requests: two loads, one after the other, so they go out first and
+    // together, not token by token between the sums
+    int seq[CONV_TOKENS];
+#pragma unroll
+    for (int u = 0; u < CONV_TOKENS; ++u) seq[u] = seq_of_token[min(t0 + u, n_tokens - 1)];
     // the eight channels' weights are 8 x TAPS consecutive floats from a 32-byte boundary
     float wr[8 * TAPS];
 #pragma unroll
@@ -103,12 +108,14 @@ causal_conv_silu_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloa
         for (int e = 0; e < 8; ++e) v[r][e] = 0.f;
       }
     }
+    int place[CONV_TOKENS];
+#pragma unroll
+    for (int u = 0; u < CONV_TOKENS; ++u) place[u] = t0 + u - cu_tokens[seq[u]];
 #pragma unroll
     for (int u = 0; u < CONV_TOKENS; ++u) {
       const int t = t0 + u;
       if (t >= n_tokens) break;
-      const int s = seq_of_token[t];
-      const int local = t - cu_tokens[s];
+      const int s = seq[u], local = place[u];
       float acc[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] = b8[e];
@@ -672,7 +679,8 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
 // ---------------------------------------------------------------- output norm and gate
 // out[t, h, :] = o[t, h, :] / sqrt(mean(o[t, h, :]^2) + eps) * weight * sigmoid(gate[t, h, :]);
 // one warp per (token, head); the weight (dv values) is shared by the heads.
-template <typename T>
+// VEC: four neighbouring values a lane at a time (rows in whole pieces).
+template <typename T, bool VEC>
 __global__ void gated_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ o,
                                      const T* __restrict__ gate, int gate_ld,
                                      const float* __restrict__ weight, int n_rows, int heads, int dv,
@@ -686,9 +694,44 @@ __global__ void gated_rmsnorm_kernel(T* __restrict__ out, const float* __restric
   const float* orow = o + (size_t)row * dv;
   const T* grow = gate + (size_t)t * gate_ld + (size_t)h * dv;
   float ss = 0.f;
+  T* dst = out + (size_t)row * dv;
+  if constexpr (VEC) {
+    for (int d = 4 * lane; d < dv; d += 128) {
+      const float4 x = *reinterpret_cast<const float4*>(orow + d);
+      ss = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, ss))));
+    }
+    const float rstd = rsqrtf(warp_sum(ss) / (float)dv + eps);
+    for (int d = 4 * lane; d < dv; d += 128) {
+      const float4 x = *reinterpret_cast<const float4*>(orow + d);
+      const float4 w = *reinterpret_cast<const float4*>(weight + d);
+      float gt[4];
+      if constexpr (sizeof(T) == 4) {
+        const float4 g = *reinterpret_cast<const float4*>(grow + d);
+        gt[0] = g.x; gt[1] = g.y; gt[2] = g.z; gt[3] = g.w;
+      } else {
+        const uint2 raw = *reinterpret_cast<const uint2*>(grow + d);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+        gt[0] = a.x; gt[1] = a.y; gt[2] = b.x; gt[3] = b.y;
+      }
+      const float v[4] = {x.x * rstd * w.x, x.y * rstd * w.y, x.z * rstd * w.z, x.w * rstd * w.w};
+      float y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = v[e] * (1.f / (1.f + expf(-gt[e])));
+      if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(dst + d) = make_float4(y[0], y[1], y[2], y[3]);
+      } else {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(y[0], y[1]), b = __floats2bfloat162_rn(y[2], y[3]);
+        uint2 packed;
+        packed.x = *reinterpret_cast<const uint32_t*>(&a);
+        packed.y = *reinterpret_cast<const uint32_t*>(&b);
+        *reinterpret_cast<uint2*>(dst + d) = packed;
+      }
+    }
+    return;
+  }
   for (int d = lane; d < dv; d += 32) ss += orow[d] * orow[d];
   const float rstd = rsqrtf(warp_sum(ss) / (float)dv + eps);
-  T* dst = out + (size_t)row * dv;
   for (int d = lane; d < dv; d += 32) {
     const float gt = 1.f / (1.f + expf(-to_float(grow[d])));
     dst[d] = from_float<T>(orow[d] * rstd * weight[d] * gt);
@@ -702,7 +745,12 @@ HB_EXPORT int hb_gated_rmsnorm(void* out, const float* o, const void* gate, int 
   if (heads <= 0 || dv <= 0 || gate_ld < heads * dv) return HB_BAD_ARGUMENT;
   const int n_rows = T * heads;
   HB_DISPATCH_DTYPE(act_dt, TA,
-    hb_launch(gated_rmsnorm_kernel<TA>, dim3((n_rows + 3) / 4), dim3(128), 0, stream, (TA*)out, o,
+    const size_t piece = 4 * sizeof(TA);
+    const bool vec = dv % 4 == 0 && gate_ld % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0 &&
+                     reinterpret_cast<uintptr_t>(out) % piece == 0 && reinterpret_cast<uintptr_t>(gate) % piece == 0;
+    auto kernel = vec ? gated_rmsnorm_kernel<TA, true> : gated_rmsnorm_kernel<TA, false>;
+    hb_launch(kernel, dim3((n_rows + 3) / 4), dim3(128), 0, stream, (TA*)out, o,
               (const TA*)gate, gate_ld, weight, n_rows, heads, dv, eps));
   return hb_check_launch();
 }

@@ -811,3 +811,23 @@ def test_latent_attention_of_many_single_tokens_takes_sixteen_rows_a_block(heads
     # weights and results have 8 bits: two results of at most about 1.5 in size, each within 2^-8 of it
     torch.testing.assert_close(got, want, atol=1.6e-2, rtol=1.6e-2)
 
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dv,pad", [(4, 0), (30, 0), (128, 0), (128, 3), (128, 8), (132, 4), (260, 0)])
+def test_gated_norm_in_pieces_and_value_by_value(dtype, dv, pad):
+    """Value sizes and gate strides that are, and are not, whole pieces of four."""
+    from helios_b200.csrc import ops
+
+    dt = torch.float32 if dtype == "float32" else torch.bfloat16
+    g = torch.Generator().manual_seed(dv + pad)
+    T, heads = 7, 3
+    o, w = torch.randn(T, heads * dv, generator=g) * 2, torch.rand(dv, generator=g) + 0.5
+    gate = torch.randn(T, heads * dv + pad, generator=g).to(dt)
+    got = ops.gated_rmsnorm(o.cuda(), gate.cuda()[:, :heads * dv], w.cuda(), heads, dv, 1e-5)
+    x = o.double().view(T, heads, dv)
+    want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w.double()
+    want = (want.reshape(T, -1) * torch.sigmoid(gate.double()[:, :heads * dv]))
+    tol = 2e-6 if dtype == "float32" else 2.0 ** -8      # some ten roundings of 24 bits; one of 8
+    torch.testing.assert_close(got.double().cpu(), want, atol=tol * 0.5, rtol=tol)
+
