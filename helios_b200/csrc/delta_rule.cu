@@ -150,6 +150,67 @@ causal_conv_silu_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloa
   }
 }
 
+// Steps of single tokens: the sum and the shift of the slot's inputs in one launch, four neighbouring
+// channels a thread, whose inputs, weights and outputs are whole pieces (`causal_conv_silu` and
+// `causal_conv_state` read the same inputs one after the other, value by value: 64 requests of 6,144
+// channels 13.4 µs, so 5.1).  A request's sum per channel has the same order.
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(128)
+causal_conv_step_kernel(T* __restrict__ out, const T* __restrict__ x, int ld, const float* __restrict__ w,
+                        const float* __restrict__ bias, float* __restrict__ state, long state_stride,
+                        const int* __restrict__ cu_tokens, const int* __restrict__ slots, int channels) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int s = blockIdx.y, c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (c >= channels) return;
+  const int t0 = cu_tokens[s], t1 = cu_tokens[s + 1];
+  if (t0 >= t1) return;
+  float* st = state + (size_t)slots[s] * state_stride + (size_t)c * (TAPS - 1);
+  __align__(16) float in[4 * (TAPS - 1)];
+  __align__(16) float wr[4 * TAPS];
+#pragma unroll
+  for (int i = 0; i < TAPS; ++i) *reinterpret_cast<float4*>(wr + 4 * i) = *reinterpret_cast<const float4*>(w + (size_t)c * TAPS + 4 * i);
+#pragma unroll
+  for (int i = 0; i < TAPS - 1; ++i) *reinterpret_cast<float4*>(in + 4 * i) = *reinterpret_cast<const float4*>(st + 4 * i);
+  for (int t = t0; t < t1; ++t) {
+    float v[4], y[4];
+    const T* xr = x + (size_t)t * ld + c;
+    if constexpr (sizeof(T) == 4) {
+      const float4 a = *reinterpret_cast<const float4*>(xr);
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    } else {
+      const uint2 raw = *reinterpret_cast<const uint2*>(xr);
+      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+      const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float* own = in + e * (TAPS - 1);
+      float acc = bias ? bias[c + e] : 0.f;
+#pragma unroll
+      for (int j = 0; j < TAPS - 1; ++j) acc = fmaf(wr[e * TAPS + j], own[j], acc);
+      acc = fmaf(wr[e * TAPS + TAPS - 1], v[e], acc);
+      y[e] = acc / (1.f + expf(-acc));
+#pragma unroll
+      for (int j = 0; j + 1 < TAPS - 1; ++j) own[j] = own[j + 1];
+      own[TAPS - 2] = v[e];
+    }
+    T* dst = out + (size_t)t * channels + c;
+    if constexpr (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(dst) = make_float4(y[0], y[1], y[2], y[3]);
+    } else {
+      const __nv_bfloat162 a = __floats2bfloat162_rn(y[0], y[1]), b = __floats2bfloat162_rn(y[2], y[3]);
+      uint2 packed;
+      packed.x = *reinterpret_cast<const uint32_t*>(&a);
+      packed.y = *reinterpret_cast<const uint32_t*>(&b);
+      *reinterpret_cast<uint2*>(dst) = packed;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < TAPS - 1; ++i) *reinterpret_cast<float4*>(st + 4 * i) = *reinterpret_cast<const float4*>(in + 4 * i);
+}
+
 HB_EXPORT int hb_causal_conv_silu(void* out, const void* x, int ld, const float* w, const float* bias,
                                   float* state,
                                   long state_stride, const int* seq_of_token, const int* cu_tokens,
@@ -157,6 +218,21 @@ HB_EXPORT int hb_causal_conv_silu(void* out, const void* x, int ld, const float*
                                   int act_dt, cudaStream_t stream) {
   if (n_tokens <= 0 || channels <= 0) return HB_OK;
   if (taps < 1 || ld < channels) return HB_BAD_ARGUMENT;
+  const size_t piece = act_dt == HB_BF16 ? 8 : 16;
+  if (n_tokens == n_seqs && n_seqs <= 65535 && taps >= 2 && taps <= 4 && channels % 4 == 0 && ld % 4 == 0 &&
+      state_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(state)) & 15) == 0 &&
+      (reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(x)) % piece == 0) {
+    const dim3 grid1((channels / 4 + 127) / 128, n_seqs);
+#define HB_CONV_STEP(TP)                                                                                        \
+    HB_DISPATCH_DTYPE(act_dt, TA,                                                                               \
+      hb_launch(causal_conv_step_kernel<TA, TP>, grid1, dim3(128), 0, stream, (TA*)out, (const TA*)x, ld, w,     \
+                bias, state, state_stride, cu_tokens, slots, channels))
+    if (taps == 2) HB_CONV_STEP(2);
+    else if (taps == 3) HB_CONV_STEP(3);
+    else HB_CONV_STEP(4);
+#undef HB_CONV_STEP
+    return hb_check_launch();
+  }
   const size_t total = (size_t)n_tokens * channels;
   // steps of few tokens keep a thread a (token, channel): more threads, shorter chains of loads
   if (act_dt == HB_BF16 && n_tokens >= 64 && channels % 8 == 0 && ld % 8 == 0 && taps >= 2 && taps <= 4 &&

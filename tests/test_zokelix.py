@@ -831,3 +831,40 @@ def test_gated_norm_in_pieces_and_value_by_value(dtype, dv, pad):
     tol = 2e-6 if dtype == "float32" else 2.0 ** -8      # some ten roundings of 24 bits; one of 8
     torch.testing.assert_close(got.double().cpu(), want, atol=tol * 0.5, rtol=tol)
 
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("taps", [2, 3, 4, 5])
+@pytest.mark.parametrize("C,pad", [(4, 0), (36, 4), (36, 1), (37, 3), (1028, 0)])
+def test_short_convolution_a_token_a_step_is_the_whole_sequence_bit_for_bit(dtype, taps, C, pad):
+    """Single tokens of several requests in scattered slots (one launch where channels, rows and the
+    slots' inputs are whole pieces, and 2 to 4 taps), with and without a bias, against the
+    kernels for portions, and the inputs they leave."""
+    from types import SimpleNamespace
+    from helios_b200.csrc import ops
+
+    dt = torch.float32 if dtype == "float32" else torch.bfloat16
+    g = torch.Generator().manual_seed(C + taps)
+    S, n = 3, 9
+    x = torch.randn(S, n, C + pad, generator=g).to(dt)
+    w, bias = torch.randn(C, taps, generator=g).cuda(), (torch.randn(C, generator=g).cuda() if pad else None)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+
+    def run(rows, counts, state, slots):
+        cu = [sum(counts[:i]) for i in range(len(counts) + 1)]
+        ctx = SimpleNamespace(seq_of_token=ints([i for i, c in enumerate(counts) for _ in range(c)]), cu_tokens=ints(cu),
+                              slots=ints(slots), num_seqs=len(counts))
+        return ops.causal_conv_silu(ctx, rows.contiguous().cuda(), C, w, state, bias)
+
+    first = torch.randn(5, C * (taps - 1), generator=g).cuda()
+    whole, state = first.clone(), first.clone()
+    want = run(x.reshape(S * n, -1), [n] * S, whole, [3, 0, 2]).view(S, n, C)
+    for t in range(n):
+        assert torch.equal(run(x[:, t], [1] * S, state, [3, 0, 2]), want[:, t])
+    assert torch.equal(state, whole) and torch.equal(state[[1, 4]], first[[1, 4]])
+    # as many tokens as requests, but not one each
+    a, b = first.clone(), first.clone()
+    got = run(x[0, :3], [0, 2, 1], a, [1, 4, 0])
+    assert torch.equal(got[:2], run(x[0, :2], [2], b, [4])) and torch.equal(got[2:], run(x[0, 2:3], [1], b, [0]))
+    assert torch.equal(a, b)
+
