@@ -453,7 +453,9 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
       bool raised = false;
 #pragma unroll
       for (int j = 6; j >= 0; --j) {                        // from the highest cut down
-        const uint32_t cut = float_key(fmaf(step, (float)(j + 1), v0));
+        // (the values were counted by their size, the list goes by key: a cut at zero lies below -0.0)
+        const float at = fmaf(step, (float)(j + 1), v0);
+        const uint32_t cut = float_key(at == 0.f ? -0.f : at);
         if (raised || cut <= old_lo || cut >= old_up) continue;
         raised = satisfies(base_mass + acc[j], base_count + acc[7 + j]);
         if (raised) { lo = cut; lo_count = base_count + acc[7 + j]; }

@@ -621,6 +621,25 @@ def test_tcgen05_attention_refuses_sizes_it_does_not_take():
                                    case.start_pos, 6, 2, 96, 16, None, 0.125)
 
 
+@pytest.mark.parametrize("k,p", [(60, 1.0), (0, 0.08)])
+def test_a_threshold_at_zero_keeps_the_negative_zeros(k, p):
+    """The interval around the threshold is cut at exactly zero, and the values that end it are -0.0:
+    21 values above them, too many below for the list at first."""
+    V, R = 40003, 64
+    g = torch.Generator().manual_seed(k)
+    row = torch.full((V,), -30.0)
+    at = torch.randperm(V, generator=g)
+    row[at[:1]] = 3.0
+    row[at[1:21]] = torch.linspace(0.05, 0.8, 20)
+    row[at[21:121]] = -0.0
+    row[at[121:2121]] = -0.1 - 0.8 * torch.rand(2000, generator=g)
+    args = (row.expand(R, V).contiguous(), [1.0] * R, [k] * R, [p] * R, list(range(R)), [3] * R)
+    got = _sample(*args)
+    kept = set(at[:121].tolist())
+    assert set(got) <= kept and set(got) & set(at[21:121].tolist())
+    assert got == _sample(*args, kind="one_block")
+
+
 # ---------------------------------------------------------------------- float32 products of few rows
 @pytest.mark.parametrize("K", [4, 16, 20, 124, 128, 132, 512, 900, 4096, 4868, 19000])
 @pytest.mark.parametrize("M,N", [(1, 1), (1, 1201), (2, 130), (3, 37), (4, 600), (5, 64), (8, 9), (9, 33), (16, 5), (17, 40)])
