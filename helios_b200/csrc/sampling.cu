@@ -178,12 +178,16 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, int V, in
 // sixteen for a row with top-k and top-p, though the tokens that matter are a few hundred.  So
 // one pass counts (and weighs) the values above SC_LEVELS levels below the maximum, in steps of
 // the temperature; the threshold lies between the highest level that holds k values, or more than
-// p of the mass, and the next.  Up to three more passes narrow that interval to an eighth each,
+// p of the mass, and the next.  Up to four more passes narrow that interval to an eighth each,
 // until it holds at most SC_LIST values; these go to the first block's shared memory, which sorts
-// them and reads the threshold off the sorted list.  Rows that stay wider (masses of equal
-// values, thresholds below the lowest level) keep the search.  128,256 values a row, µs a launch,
+// them and reads the threshold off the sorted list.  Rows that stay wider are searched, within the
+// interval: masses of equal values (a pass that does not halve the interval is the last) and
+// thresholds below the lowest level.  With top-k and top-p the list begins at the maximum, so that
+// rows with k above SC_LIST are searched from the start.  128,256 values a row, µs a launch,
 // search / list: 64 rows N(0, 4) of mixed options 166 / 50, all top-k 50 and top-p 0.9 265 / 68,
-// one row 81 / 25; top-p 0.95 of 64 rows N(0, 1), 60,000 tokens kept, 452 / 146.
+// one row 81 / 25; top-p 0.95 of 64 rows N(0, 1), 60,000 tokens kept, 452 / 149.  Eight rows, search of
+// whole keys alone / list tried in vain, then that search / this: top-k 2,000 and top-p 0.9 of N(0, 4)
+// 111 / 141 / 101; top-k 2,000 of whole numbers 48 / 80 / 50; top-k 50 of equal values 39 / 71 / 50.
 constexpr int SC_THREADS = 512;
 constexpr int SC_CLUSTER = 8;
 constexpr int SC_MOST = 40;          // elements a thread keeps: rows of up to 8 * 512 * 40 values
@@ -321,6 +325,7 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
   __shared__ int s_idx[SC_WARPS];
   __shared__ float x_f[5];                 // what a block shows its peers: key, index, total, pick, threshold
   __shared__ uint32_t list[SC_LIST];       // of the first block: the row's largest values
+  __shared__ uint32_t range[2];            // where a search looks for the threshold, both included
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t rank = sc_rank();
   const int row = blockIdx.x / SC_CLUSTER;
@@ -386,7 +391,9 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
   const int k_row = top_k[row], k_on = (k_row > 0 && k_row < V) ? k_row : 0;
   const float p_on = top_p[row];
   uint32_t sorted_thr = 0;
-  if ((k_on > 0 || p_on < 1.f) && !(p_on < 0.f) && fabsf(key_float(bk)) < INFINITY && inv_t < INFINITY) {
+  if (tid == 0) { range[0] = 0u; range[1] = bk; }
+  if ((k_on > 0 || p_on < 1.f) && !(p_on < 1.f && k_on > SC_LIST) && !(p_on < 0.f) &&
+      fabsf(key_float(bk)) < INFINITY && inv_t < INFINITY) {
     constexpr float depth[SC_LEVELS] = {1.f, 2.f, 4.f, 7.f, 12.f, 24.f};
     uint32_t level[SC_LEVELS];
 #pragma unroll
@@ -429,8 +436,10 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
     bool fits = false;
     for (int round = 0; settled; ++round) {
       fits = lo_count - (whole ? 0.f : up_count) <= (float)SC_LIST;
-      if (fits || round == 4) break;
+      // (the pass before left its count beside its sums, which alternate)
+      if (fits || round == 4 || (round > 0 && 2.f * (lo_count - up_count) > block_part[slot][15])) break;
       slot ^= 1;
+      if (tid == 0) block_part[slot][15] = lo_count - up_count;
       const float v0 = key_float(lo), step = (key_float(up == 0xffffffffu ? bk : up) - v0) * 0.125f;
 #pragma unroll
       for (int j = 0; j < 15; ++j) acc[j] = 0.f;
@@ -462,7 +471,9 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
         else { up = cut; up_mass = base_mass + acc[j]; up_count = base_count + acc[7 + j]; }
       }
     }
-    if (fits) {                                              // the same in every thread of the cluster
+    if (!fits) {                                             // the same in every thread of the cluster
+      if (settled && tid == 0) { range[0] = lo; range[1] = min(bk, up - 1u); }
+    } else {
       const uint32_t list_up = whole ? 0xffffffffu : up;
       const float above_count = whole ? 0.f : up_count, above_mass = whole ? 0.f : up_mass;
       int kept = 0;
@@ -505,12 +516,20 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
   }
   const bool search = sorted_thr == 0;
 
+  // The bits of a search's first pass: those of the distance between the ends, or of whole keys where
+  // that has as many (or its sums with `from` would not fit 32 bits); -4 where the ends meet.
+  auto first_shift = [](uint32_t& from, uint32_t to) {
+    if (to - from >= (1u << 28) || from >= 0xf0000000u) from = 0u;
+    return from == 0u ? 28 : (31 - __clz(to - from)) & ~3;
+  };
+
   // ---- top-k: the largest key c with #(key >= c) >= k, four bits a pass
   uint32_t thr = 1;                        // keeps every value, and none of the padding
   const int k = k_on;
+  if (search) __syncthreads();             // `range` is there
   if (k > 0 && search) {
-    uint32_t cand = 0;
-    for (int shift = 28; shift >= 0; shift -= 4) {
+    uint32_t cand = range[0];
+    for (int shift = first_shift(cand, range[1]); shift >= 0; shift -= 4) {
 #pragma unroll
       for (int j = 0; j < 15; ++j) acc[j] = 0.f;
 #pragma unroll
@@ -519,7 +538,7 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
         // after a pass or two that is nearly everything, and whole warps skip it)
         if (key[i] > cand) {
 #pragma unroll
-          for (int j = 0; j < 15; ++j) acc[j] += (key[i] >= (cand | ((uint32_t)(j + 1) << shift))) ? 1.f : 0.f;
+          for (int j = 0; j < 15; ++j) acc[j] += (key[i] >= cand + ((uint32_t)(j + 1) << shift)) ? 1.f : 0.f;
         }
       }
       sc_sum15(acc, warp_part, block_part, total, slot);
@@ -528,7 +547,7 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
 #pragma unroll
       for (int j = 0; j < 15; ++j)
         if (acc[j] >= (float)k) digit = j + 1;
-      cand |= digit << shift;
+      cand += digit << shift;
     }
     if (cand > thr) thr = cand;
   }
@@ -543,8 +562,9 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
     sc_sum15(acc, warp_part, block_part, total, slot);
     slot ^= 1;
     const float want = pp * acc[0];
-    uint32_t cand = 0;
-    for (int shift = 28; shift >= 0; shift -= 4) {
+    // (any mass is more than a negative share: nothing is kept)
+    uint32_t cand = pp < 0.f ? 0u : k > 0 ? thr : range[0];
+    for (int shift = first_shift(cand, k > 0 ? bk : range[1]); shift >= 0; shift -= 4) {
 #pragma unroll
       for (int j = 0; j < 15; ++j) acc[j] = 0.f;
 #pragma unroll
@@ -552,7 +572,7 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
         if (key[i] >= thr && key[i] > cand) {
           const float e = expf(key_float(key[i]) * inv_t - mx_t);
 #pragma unroll
-          for (int j = 0; j < 15; ++j) acc[j] += (key[i] >= (cand | ((uint32_t)(j + 1) << shift))) ? e : 0.f;
+          for (int j = 0; j < 15; ++j) acc[j] += (key[i] >= cand + ((uint32_t)(j + 1) << shift)) ? e : 0.f;
         }
       }
       sc_sum15(acc, warp_part, block_part, total, slot);
@@ -561,7 +581,7 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
 #pragma unroll
       for (int j = 0; j < 15; ++j)
         if (acc[j] > want) digit = j + 1;
-      cand |= digit << shift;
+      cand += digit << shift;
     }
     if (cand > thr) thr = cand;
   }

@@ -532,6 +532,30 @@ def test_sampling_from_the_sorted_list_follows_the_reference_rules(kind, V):
             assert kept[got[i]] > 0 and min(near, share) < 1e-6, f"row {i}: got {got[i]}, reference {want}, u={u}"
 
 
+@pytest.mark.parametrize("V", [4099, 128256])
+@pytest.mark.parametrize("kind", ["whole numbers", "zeros", "equal", "negative", "far maximum"])
+def test_rows_wider_than_the_sorted_list_are_searched(kind, V):
+    """Masses of equal values, thresholds below the lowest level, and lists that could not hold k values:
+    the search within the interval found so far keeps what the one-block kernel keeps."""
+    g = torch.Generator().manual_seed(V)
+    row = torch.randn(V, generator=g)
+    if kind == "whole numbers":
+        row = (2 * row).round()
+    elif kind in ("zeros", "equal"):
+        row = torch.full((V,), 0.0 if kind == "zeros" else -7.25)
+    elif kind == "negative":
+        row = row - 1000
+    else:
+        row[V // 3] = 60.0
+    options = [(1.0, k, p) for k in (1024, 1025, 1500, 2000, V - 2) for p in (0.3, 0.9, 1.0)]
+    options += [(1.0, 50, 0.9), (0.05, 2000, 1.0), (0.05, 0, 0.9), (3.0, 0, 0.9), (1.0, 0, 1.0 - 2.0 ** -22), (1.0, 0, 0.0)]
+    args = tuple(map(list, zip(*options)))
+    for seed in range(4):
+        seeds, offsets = [100 * seed + i for i in range(len(options))], [7] * len(options)
+        got = _sample(row.expand(len(options), V).contiguous(), *args, seeds, offsets)
+        assert got == _sample(row.expand(len(options), V).contiguous(), *args, seeds, offsets, kind="one_block")
+
+
 @pytest.mark.parametrize("bad", [float("inf"), float("nan"), -float("inf")])
 def test_rows_without_a_finite_maximum_end(bad):
     """Rows of infinities and NaN have no distribution; the kernel returns some id of the vocabulary."""
