@@ -556,6 +556,17 @@ def test_rows_wider_than_the_sorted_list_are_searched(kind, V):
         assert got == _sample(row.expand(len(options), V).contiguous(), *args, seeds, offsets, kind="one_block")
 
 
+@pytest.mark.parametrize("V", [4096, 9001, 70000, 128256, 163840])
+@pytest.mark.parametrize("kind", ["greedy", "draw"])
+def test_what_the_caller_knows_of_the_options_changes_no_result(kind, V):
+    """The kernel without the sorted list, one per number of values a thread keeps."""
+    g = torch.Generator().manual_seed(V)
+    options = [(0.0, 0, 1.0), (1.0, 0, 1.0), (0.7, 0, 1.0), (1.0, 40, 1.0), (1.0, 0, 0.9), (0.8, 300, 0.7)]
+    logits = 2 * torch.randn(len(options), V, generator=g)
+    args = (logits, *map(list, zip(*options)), [3, 1, 4, 1, 5, 9], [2, 6, 5, 3, 5, 8])
+    assert _sample(*args, kind=kind) == _sample(*args, kind="narrow") == _sample(*args, kind="one_block")
+
+
 @pytest.mark.parametrize("bad", [float("inf"), float("nan"), -float("inf")])
 def test_rows_without_a_finite_maximum_end(bad):
     """Rows of infinities and NaN have no distribution; the kernel returns some id of the vocabulary."""
