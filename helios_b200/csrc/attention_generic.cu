@@ -21,7 +21,7 @@
 // request was cut into steps, nor on the rest of the batch.
 //
 // Bound by the latency of its loads: a decode step has a few dozen rows of some hundred keys.
-// So a row has a block of eight warps, and a run's loads are independent: eight lanes share a
+// So a row has a block of eight warps where its keys make as many runs (below: SHARE), and a run's loads are independent: eight lanes share a
 // key (four elements a lane and load, the key's dot product finished by three shuffles), a
 // warp's four groups of eight lanes walk eight keys of the run each, and values the same way.
 // In chains, 14 heads of 64 on 2 KV heads, float32, one warp a row with a key a lane / this:
@@ -67,12 +67,19 @@ __device__ __forceinline__ float4 load_four(const T* row, int d, int n) {
 }
 
 // NJ: 32 * NJ >= hd, vd.  VEC: rows of keys and values are whole 4-element pieces.
-template <typename T, int NJ, bool VEC>
+// SHARE: a token whose keys make one, two or three to four runs has 8, 4 or 2 of its heads in one block,
+// with 1, 2 or 4 warps each, and the blocks of the other heads end at once (the position is on the
+// device).  The sums are the same ones in the same order.  A row of at most 32 keys alone keeps one warp of
+// eight, and two blocks fit an SM.  14 heads of 64 on 2 KV heads, float32, a block a row / shared, µs: 67 prompts
+// of 30 tokens 347 / 67, 2,048 tokens with a window of 16 356 / 69 and of 128 383 / 236, 600 decode rows of 30
+// keys 116 / 25; but 600 of 250 keys 223 / 246 (half a microsecond a block until the position is there
+// and the warps are dealt), and one row of 30 5.6 / 6.1.  So it is for launches of many rows that may be short.
+template <typename T, int NJ, bool VEC, bool SHARE>
 __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
     T* __restrict__ out, const T* __restrict__ q, int q_stride,
     const T* __restrict__ k_pages, const T* __restrict__ v_pages,
     const int* __restrict__ block_table, int bt_stride, const int* __restrict__ seq_of_token,
-    const int* __restrict__ positions, int nh, int nkv, int hd, int vd, int page_size,
+    const int* __restrict__ positions, int head_blocks, int head_step, int nh, int nkv, int hd, int vd, int page_size,
     int window, float scale, const float* __restrict__ slopes, int sink,
     const T* __restrict__ gate, int gate_stride, const float* __restrict__ bias_table, int bias_rows,
     const float* __restrict__ sink_values, int keep_first, int gate_wide, PooledPages<T> pooled,
@@ -84,20 +91,39 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
   constexpr int KEYS = NJ <= 4 ? 8 / NJ : 1;         // keys a group has in flight: eight loads a lane
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = lane >> 3, gl = lane & 7;
-  const int t = blockIdx.x / nh, h = blockIdx.x - t * nh;
-  const int kvh = h / (nh / nkv);
+  const int t = blockIdx.x / head_blocks;
+  int h = (blockIdx.x - t * head_blocks) * head_step, kvh = h / (nh / nkv);
   const int pos = positions[t];
   const int* token_table = block_table + (size_t)seq_of_token[t] * bt_stride;
   const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
 
   // this lane's pieces of a row: elements 4 (8 j + gl) .. + 3
   float4 qr[NJ], acc[NJ];
-  const T* qrow = q + (size_t)t * q_stride + (size_t)h * hd;
+  auto load_query = [&] {
+    const T* qrow = q + (size_t)t * q_stride + (size_t)h * hd;
 #pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    qr[j] = load_four<T, false>(qrow, 4 * (8 * j + gl), hd);
-    acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < NJ; ++j) qr[j] = load_four<T, false>(qrow, 4 * (8 * j + gl), hd);
+  };
+  int wpr = ATTN_WARPS;                                // warps of a row
+  if constexpr (SHARE) {
+    if constexpr (NJ == 8) load_query();               // (while the position is on its way; smaller heads are slower so)
+    const int total = (pos - lo) / 32 + 1 + (min(keep_first, lo) + 31) / 32 +
+                      (pooled.pool > 0 ? (lo / pooled.pool + 31) / 32 : 0);
+    wpr = total <= 1 ? 1 : total <= 2 ? 2 : total <= 4 ? 4 : ATTN_WARPS;
+    if (h & (ATTN_WARPS / wpr - 1)) return;            // another block has this head
+    if (wpr < ATTN_WARPS) {
+      h += warp / wpr;
+      if (h >= nh) return;
+      kvh = h / (nh / nkv);
+      if constexpr (NJ == 8) load_query();
+    }
+    if constexpr (NJ < 8) load_query();
+  } else {
+    load_query();
   }
+  const int part = warp & (wpr - 1), row_warp = warp - part;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
   float m = -INFINITY, l = 0.f;
   const float slope = slopes ? slopes[h] : 0.f;
 
@@ -112,7 +138,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
     const T* kp = stretch < 0 ? pooled.k : k_pages;
     const T* vp = stretch < 0 ? pooled.v : v_pages;
     const int runs = last >= first ? (last - first) / 32 + 1 : 0;
-    for (int r = (warp - run % ATTN_WARPS + ATTN_WARPS) % ATTN_WARPS; r < runs; r += ATTN_WARPS) {
+    for (int r = (part - run % ATTN_WARPS + ATTN_WARPS) % ATTN_WARPS; r < runs; r += ATTN_WARPS) {
       const int base = first + 32 * r;
       const int key = base + lane;
       const bool valid = key <= last;
@@ -202,32 +228,33 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
   }
   if (lane == 0) { part_m[warp] = m; part_l[warp] = l; }
   __syncthreads();
-  const int d = threadIdx.x;
-  if (d >= vd) return;
   m = -INFINITY;
 #pragma unroll
-  for (int w = 0; w < ATTN_WARPS; ++w) m = fmaxf(m, part_m[w]);
-  l = 0.f;
-  float y = 0.f;
+  for (int w = 0; w < ATTN_WARPS; ++w)
+    if (w < wpr) m = fmaxf(m, part_m[row_warp + w]);
+  for (int d = threadIdx.x - 32 * row_warp; d < vd; d += 32 * wpr) {
+    l = 0.f;
+    float y = 0.f;
 #pragma unroll
-  for (int w = 0; w < ATTN_WARPS; ++w) {
-    if (w >= run) break;                               // the warps behind the last run have seen no key
-    const float f = part_m[w] == -INFINITY ? 0.f : expf(part_m[w] - m);
-    l = fmaf(part_l[w], f, l);
-    y = fmaf(part_acc[w][d], f, y);
+    for (int w = 0; w < ATTN_WARPS; ++w) {
+      if (w >= run) break;                             // the warps behind the last run have seen no key
+      const float pm = part_m[row_warp + w], f = pm == -INFINITY ? 0.f : expf(pm - m);
+      l = fmaf(part_l[row_warp + w], f, l);
+      y = fmaf(part_acc[row_warp + w][d], f, y);
+    }
+    if (sink) {                     // a key without a value: it adds exp(s - m) to the sum only (s = 0 unless given)
+      const float sv = sink_values ? sink_values[h] : 0.f;
+      const float m_new = fmaxf(m, sv);
+      const float corr = expf(m - m_new);
+      l = l * corr + expf(sv - m_new);
+      y *= corr;
+    }
+    float inv = factor / l;
+    if (gate && !gate_wide) inv /= 1.f + expf(-to_float(gate[(size_t)t * gate_stride + h]));
+    y *= inv;
+    if (gate && gate_wide) y /= 1.f + expf(-to_float(gate[(size_t)t * gate_stride + (size_t)h * vd + d]));
+    out[(size_t)t * out_stride + (size_t)h * vd + d] = from_float<T>(y);
   }
-  if (sink) {                       // a key without a value: it adds exp(s - m) to the sum only (s = 0 unless given)
-    const float sv = sink_values ? sink_values[h] : 0.f;
-    const float m_new = fmaxf(m, sv);
-    const float corr = expf(m - m_new);
-    l = l * corr + expf(sv - m_new);
-    y *= corr;
-  }
-  float inv = factor / l;
-  if (gate && !gate_wide) inv /= 1.f + expf(-to_float(gate[(size_t)t * gate_stride + h]));
-  y *= inv;
-  if (gate && gate_wide) y /= 1.f + expf(-to_float(gate[(size_t)t * gate_stride + (size_t)h * vd + d]));
-  out[(size_t)t * out_stride + (size_t)h * vd + d] = from_float<T>(y);
 }
 
 HB_EXPORT int hb_attention_generic(void* out, const void* q, int q_stride, const void* k_pages,
@@ -239,7 +266,7 @@ HB_EXPORT int hb_attention_generic(void* out, const void* q, int q_stride, const
                                    const float* sink_values, int keep_first, int gate_wide,
                                    const void* pooled_k, const void* pooled_v, const int* pooled_table,
                                    int pooled_table_stride, int pool, int out_stride, float factor, int act_dt,
-                                   cudaStream_t stream) {
+                                   int sms, cudaStream_t stream) {
   if (T <= 0) return HB_OK;
   if (hd <= 0 || hd > ATTN_MAX_HD || vd <= 0 || vd > ATTN_MAX_HD || nkv <= 0 || nh % nkv != 0 ||
       page_size <= 0 || keep_first < 0 || pool < 0 || out_stride < nh * vd ||
@@ -247,14 +274,32 @@ HB_EXPORT int hb_attention_generic(void* out, const void* q, int q_stride, const
     return HB_BAD_ARGUMENT;
   if ((long)T * nh > 0x7fffffffL) return HB_BAD_ARGUMENT;
   const int most = hd > vd ? hd : vd;
-#define HB_GENERIC_LAUNCH(NJ, VEC)                                                                             \
-    hb_launch(attention_generic_kernel<TA, NJ, VEC>, dim3((unsigned)(T * nh)), dim3(ATTN_WARPS * 32), 0, stream,  \
+  // The runs of keys a row can have, as far as the arguments say: by the window, or the table's width
+  // (in a captured step that is what a request may grow to, so that many rows may be short all the same).
+  // Up to four, the heads that share a block are known here, and the others get no blocks.
+  const long keys_of_table = (long)bt_stride * page_size;
+  long keys = keys_of_table;
+  if (window > 0 && window < keys) keys = window;
+  long runs = (keys + 31) / 32 + (window > 0 ? (keep_first + 31) / 32 : 0);
+  if (pool > 0) runs += ((long)pooled_table_stride * page_size + 31) / 32;
+  const long rows = (long)T * nh;
+  const bool share = runs <= 4 ? rows > 2L * sms : rows > 8L * sms && (window <= 0 || window >= keys_of_table);
+  const int head_step = !share ? 1 : runs <= 1 ? 8 : runs <= 2 ? 4 : runs <= 4 ? 2 : 1;
+  const int head_blocks = (nh + head_step - 1) / head_step;
+#define HB_GENERIC_SHARE(NJ, VEC, SHARE)                                                                       \
+    hb_launch(attention_generic_kernel<TA, NJ, VEC, SHARE>, dim3((unsigned)(T * head_blocks)),                 \
+        dim3(ATTN_WARPS * 32), 0, stream,                                                                      \
         (TA*)out, (const TA*)q, q_stride, (const TA*)k_pages, (const TA*)v_pages, block_table,                 \
-        bt_stride, seq_of_token, positions, nh, nkv, hd, vd, page_size, window, scale,                         \
+        bt_stride, seq_of_token, positions, head_blocks, head_step, nh, nkv, hd, vd, page_size, window, scale, \
         slopes, sink, (const TA*)gate, gate_stride, bias_table, bias_rows, sink_values, keep_first,            \
         gate_wide,                                                                                             \
         PooledPages<TA>{(const TA*)pooled_k, (const TA*)pooled_v, pooled_table, pooled_table_stride, pool},    \
         out_stride, factor)
+#define HB_GENERIC_LAUNCH(NJ, VEC)                                                                             \
+    do {                                                                                                       \
+      if (share) HB_GENERIC_SHARE(NJ, VEC, true);                                                              \
+      else HB_GENERIC_SHARE(NJ, VEC, false);                                                                   \
+    } while (0)
   HB_DISPATCH_DTYPE(act_dt, TA,
     const uintptr_t addresses = reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages) |
                                 (pool > 0 ? reinterpret_cast<uintptr_t>(pooled_k) | reinterpret_cast<uintptr_t>(pooled_v) : 0);
@@ -265,5 +310,6 @@ HB_EXPORT int hb_attention_generic(void* out, const void* q, int q_stride, const
     else if (most <= 128) HB_GENERIC_LAUNCH(4, true);
     else HB_GENERIC_LAUNCH(8, true));
 #undef HB_GENERIC_LAUNCH
+#undef HB_GENERIC_SHARE
   return hb_check_launch();
 }

@@ -480,15 +480,15 @@ def attention_generic(qkv: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.T
             [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
              c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p,
              c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-             c_float, c_int, c_void_p])
+             c_float, c_int, c_int, c_void_p])
     _run(f(_p(out), _p(qkv), qkv.shape[1], _p(k_pages), _p(v_pages), _p(block_table),
            block_table.shape[1], _p(seq_of_token), _p(positions), T, num_heads, num_kv_heads,
            head_dim, vd, page_size, int(window or 0), float(scale), _p(opt.slopes), int(opt.sink),
            _p(opt.gate), opt.gate_stride, _p(opt.bias_table),
            0 if opt.bias_table is None else opt.bias_table.shape[0], _p(opt.sink_values),
            opt.keep_first if window else 0, 1 if opt.gate_wide else 0, _p(pk), _p(pv), _p(pt),
-           0 if pt is None else pt.shape[1], pool, out.stride(0), float(factor), _dt(qkv.dtype), _stream()),
-         "attention_generic")
+           0 if pt is None else pt.shape[1], pool, out.stride(0), float(factor), _dt(qkv.dtype),
+           sm_count(qkv.device), _stream()), "attention_generic")
     return out
 
 

@@ -707,3 +707,35 @@ def test_generic_attention_at_the_edges_of_runs_and_head_sizes(nh, nkv, hd, dtyp
         got = ops().attention_generic(case.qkv, case.k_pages, case.v_pages, case.table, case.seq_of_token,
                                       case.positions, nh, nkv, hd, 8, window, scale)
         torch.testing.assert_close(got.cpu().double(), dense_attention(case, scale, window), **tol(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd", [(14, 2, 64), (5, 5, 20), (6, 2, 33), (7, 1, 100), (3, 1, 200)])
+def test_generic_attention_of_many_short_rows_is_each_row_alone_bit_for_bit(nh, nkv, hd, dtype):
+    """Many rows share blocks where their keys make one to four runs, few rows have a block each: contexts
+    at the edges of one, two, four and eight runs, windows that bound them, and every option."""
+    o = ops()
+    lens = (1, 2, 31, 32, 33, 63, 64, 65, 127, 128, 129, 256, 257, 300)
+    seqs = [(lens[i % len(lens)] - 1, 1) for i in range(420)] + [(0, 40)]
+    page, scale = 8, 1.0 / math.sqrt(hd)
+    case = make_paged_case(seqs, nh, nkv, hd, page, dtype, DEV, seed=hd)
+    T = case.qkv.shape[0]
+    g = torch.Generator().manual_seed(hd)
+    gate = torch.randn(T, nh * hd, generator=g).to(DEV, dtype)
+    sinks, bias = torch.randn(nh, generator=g).to(DEV), torch.randn(50, nh, generator=g).to(DEV)
+    # (any pages do as the means of blocks of seven tokens)
+    pooled = (case.k_pages.nan_to_num(), case.v_pages.nan_to_num(), torch.zeros((len(seqs), 6), dtype=torch.int32, device=DEV), 7)
+    plain = lambda a, b: None
+    everything = lambda keep: lambda a, b: o.AttentionOptions(gate=gate[a:b], gate_wide=True, sink_values=sinks, bias_table=bias,
+                                                              keep_first=keep)
+    few = max(1, 296 // nh)
+    for window, options, means in ((None, plain, None), (None, everything(0), None), (1, plain, None), (32, everything(0), None),
+                                   (33, plain, None), (40, everything(3), None), (64, plain, None), (128, plain, None),
+                                   (60, plain, pooled), (300, plain, None)):
+        call = lambda a, b: o.attention_generic(
+            case.qkv[a:b], case.k_pages, case.v_pages, case.table, case.seq_of_token[a:b], case.positions[a:b], nh, nkv, hd, page,
+            window, scale, options(a, b), means)
+        got = call(0, T)
+        assert torch.equal(got, torch.cat([call(a, min(T, a + few)) for a in range(0, T, few)]))
+        if options is plain and means is None:
+            torch.testing.assert_close(got.cpu().double(), dense_attention(case, scale, window), **tol(dtype))
