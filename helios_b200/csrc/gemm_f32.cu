@@ -26,6 +26,22 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
+// Lets a kernel take up to BYTES of dynamic shared memory.  Once per device, and the same for every
+// call: the limit belongs to the function, and a call that set its own size could lower it between
+// another thread's setting and launch.
+template <auto KERNEL, int BYTES>
+static bool allow_shared_memory() {
+  constexpr int MOST_DEVICES = 64;
+  static bool done[MOST_DEVICES] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MOST_DEVICES) return false;
+  if (!done[dev]) {
+    if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES) != cudaSuccess) return false;
+    done[dev] = true;
+  }
+  return true;
+}
+
 // ---------------------------------------------------------------- few rows
 // Bound by reading W once.  A warp takes four rows of W and 32 runs of k, a run a lane: the 64
 // bytes of a lane's run come straight into registers (16 loads of 16 bytes a lane, 8 KB a warp
@@ -39,6 +55,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 constexpr int ROWS_W = 4;                        // rows of W a warp
 constexpr int ROWS_RUN = RUN + 4;
 constexpr int ROWS_MOST_THREADS = 256;
+constexpr int ROWS_MOST_SMEM = 200 * 1024;       // what a block may take of shared memory
 
 template <int MT>
 __global__ void __launch_bounds__(ROWS_MOST_THREADS, 2)
@@ -297,9 +314,8 @@ gemm_f32_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
 template <bool VEC>
 static int launch_tiles(float* C, const float* A, const float* W, const float* bias, int M, int N, int K, int lda,
                         int ldw, int ldc, int sms, cudaStream_t stream) {
-  const size_t smem = (size_t)STAGES * STAGE_FLOATS * sizeof(float);
-  if (cudaFuncSetAttribute(gemm_f32_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return HB_LAUNCH_FAILED;
+  constexpr int smem = STAGES * STAGE_FLOATS * (int)sizeof(float);
+  if (!allow_shared_memory<gemm_f32_kernel<VEC>, smem>()) return HB_LAUNCH_FAILED;
   const long tiles = (long)((N + BN - 1) / BN) * ((M + BM - 1) / BM);
   // three blocks fit an SM: the quarters go to blocks of their own until all SMs are full a few
   // times over, if each then still has some tiles to walk
@@ -335,10 +351,9 @@ static int launch_rows(float* C, const float* A, const float* W, const float* bi
   int groups = 1;
   while (2 * groups * wpg <= 8 && (long)N >= (long)sms * 2 * groups * ROWS_W) groups *= 2;
   const long smem = ((long)MT * runs * ROWS_RUN + 2L * groups * ROWS_W * MT * (runs + 1)) * (long)sizeof(float);
-  *fits = smem <= 200 * 1024;
+  *fits = smem <= ROWS_MOST_SMEM;
   if (!*fits) return HB_OK;
-  if (cudaFuncSetAttribute(gemm_f32_rows_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return HB_LAUNCH_FAILED;
+  if (!allow_shared_memory<gemm_f32_rows_kernel<MT>, ROWS_MOST_SMEM>()) return HB_LAUNCH_FAILED;
   const int tiles = (N + groups * ROWS_W - 1) / (groups * ROWS_W);
   // a block takes up to four tiles (A is staged once for them), fewer where that leaves SMs idle
   int per_block = tiles / (2 * sms);

@@ -694,6 +694,39 @@ def test_gemm_f32_of_few_rows_is_the_tiled_product_bit_for_bit(M, N, K, monkeypa
     assert torch.equal(ops().linear_f32(x.to(DEV), w.to(DEV), b.to(DEV)), got)
 
 
+def test_gemm_f32_of_short_and_long_rows_from_two_threads():
+    """Both threads launch the kernel for four rows, one with ten times the shared memory of the other; a
+    limit that one call sets is not another's.  (The exported function, called as fast as two threads can.)"""
+    import threading
+
+    o, g = ops(), torch.Generator().manual_seed(9)
+    started, seen = threading.Barrier(2), []
+
+    def work(args, stream):
+        started.wait()
+        seen.append(sum(f(*args, stream.cuda_stream) != 0 for _ in range(30000)))
+
+    threads, checks = [], []
+    for K in (256, 4864):
+        x, w = torch.randn(4, K, generator=g), torch.randn(8, K, generator=g)
+        xd, wd = x.to(DEV), w.to(DEV)
+        out = o.linear_f32(xd, wd)
+        f = o.load_library("gemm_f32").hb_gemm_f32
+        stream = torch.cuda.Stream()
+        checks.append((out, x.double() @ w.double().T, xd, wd, stream))
+        threads.append(threading.Thread(target=work, args=((out.data_ptr(), xd.data_ptr(), wd.data_ptr(), None, 4, 8, K, K, K, 8,
+                                                            o.GEMM_F32_FEW_ROWS, o.sm_count()), stream)))
+    torch.cuda.synchronize()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert seen == [0, 0], f"{seen} launches refused"
+    for out, want, xd, _wd, _stream in checks:
+        torch.testing.assert_close(out.double().cpu(), want, atol=xd.shape[1] * 1e-6, rtol=1e-5)
+
+
 # ---------------------------------------------------------------------- generic attention, runs dealt to warps
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("nh,nkv,hd", [(2, 1, 4), (3, 3, 20), (4, 2, 33), (7, 1, 64), (2, 2, 100), (4, 1, 130), (2, 1, 255), (1, 1, 256)])
