@@ -42,6 +42,7 @@ struct GemmArgs {
   int* error;           // set non-zero when a wait ran out
   int T, N, K;          // tokens, output features (for GLU: of the result, = half the weight rows), reduction
   int ldo;
+  int out_pieces = 0;   // out's rows are whole 16-byte pieces from a 16-byte address on: 16-byte stores
   int glu_offset;       // GLU: row of the weight where the second half ("up") begins
   int out_f32;
   int k_splits;
@@ -371,7 +372,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             for (int j = 0; j < 16; ++j) store(tile_b * BN + c + j, tile_a * BM + r, val[j]);
           } else {
             const int t = tile_a * BM + r, n0 = tile_b * HALF + c;
-            if (!args.out_f32 && t < args.T && n0 + 16 <= args.N && (args.ldo & 7) == 0) {
+            if (!args.out_f32 && t < args.T && n0 + 16 <= args.N && args.out_pieces) {
               uint32_t packed[8];
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
@@ -428,7 +429,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
               store(tile_b * BN + c + j, tile_a * BM + r, scaled ? v[j] * col_scale[c + j] : v[j]);
           } else {
             const int t = tile_a * BM + r, n0 = tile_b * BN + c;
-            if (!args.out_f32 && t < args.T && n0 + 16 <= args.N && (args.ldo & 7) == 0) {
+            if (!args.out_f32 && t < args.T && n0 + 16 <= args.N && args.out_pieces) {
               // 16 bfloat16 of one row: two 16-byte stores
               uint32_t packed[8];
 #pragma unroll
@@ -737,7 +738,7 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll
             for (int i = 0; i < 16; ++i) if (n0 + i < args.N) val[i] += args.bias[n0 + i];
           }
-          if (!args.out_f32 && n0 + 16 <= args.N && (args.ldo & 7) == 0) {
+          if (!args.out_f32 && n0 + 16 <= args.N && args.out_pieces) {
             uint32_t packed[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -747,7 +748,7 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(args.out) + (size_t)t * args.ldo + n0);
             dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
             dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-          } else if (args.out_f32 && n0 + 16 <= args.N && (args.ldo & 3) == 0) {
+          } else if (args.out_f32 && n0 + 16 <= args.N && args.out_pieces) {
             // (one value a store instead: every store of a warp begins 32 sectors of which it fills an
             // eighth; the head of 151,936 x 896 at 200 tokens took 278 µs so, against 95)
             float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(args.out) + (size_t)t * args.ldo + n0);
@@ -978,6 +979,7 @@ static int gemm_bf16_call(void* out, const void* x, const void* w, const float* 
   GemmArgs a;
   a.out = out; a.bias = bias; a.scratch = scratch; a.tickets = tickets; a.error = error;
   a.T = T; a.N = N; a.K = K; a.ldo = ldo; a.glu_offset = glu_offset; a.out_f32 = out_f32;
+  a.out_pieces = ((uintptr_t)out & 15) == 0 && ldo % (out_f32 ? 4 : 8) == 0 ? 1 : 0;
   a.k_splits = k_splits;
   a.cluster_reduce = clustered ? 1 : 0;
   a.residual = residual; a.norm_weight = norm_weight; a.sumsq_out = sumsq_out;

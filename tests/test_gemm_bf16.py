@@ -272,3 +272,33 @@ def test_gated_units_of_one_token_with_a_small_weight(N, K, kind):
     got = o.linear_bf16(x.to(DEV), w.to(DEV), glu=kind, sumsq=slots.to(DEV), eps=1e-5).double().cpu()
     # one rounding to eight bits, after sums of 32 bits
     torch.testing.assert_close(got, _gated(both[:, :N], both[:, N:], kind), rtol=2.0 ** -8, atol=1e-4)
+
+
+@pytest.mark.parametrize("cluster", [0, 2])
+@pytest.mark.parametrize("out_dtype,offset", [(torch.float32, 0), (torch.float32, 1), (torch.float32, 2), (torch.bfloat16, 0),
+                                              (torch.bfloat16, 1), (torch.bfloat16, 4)])
+def test_results_at_addresses_that_are_no_whole_pieces(out_dtype, offset, cluster):
+    """The exported function takes any address for its results (the Python call allocates them): the kernels
+    for many tokens, one and two SMs a tile, store value by value where 16-byte stores would be misaligned."""
+    import ctypes
+
+    o = ops()
+    T, N, K = 257, 272, 136
+    x, w, _b = _case(T, N, K, offset)
+    xd, wd = x.to(DEV), w.to(DEV)
+    o.linear_bf16(xd, wd)                                     # (sets the function's argument types)
+    _scratch, _tickets, err = o._gemm_workspace(xd.device)
+    room = torch.full((T * N + 8 + offset,), 7.0, dtype=out_dtype, device=DEV)
+    out = room[offset:offset + T * N]
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    f = o.load_library("gemm_bf16").hb_gemm_bf16
+    rc = f(p(out), p(xd), p(wd), None, None, None, p(err), T, N, K, K, K, N, N, 0, 0, int(out_dtype == torch.float32), 0, 1,
+           cluster, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    want = x.double() @ w.double().T
+    if out_dtype == torch.float32:
+        torch.testing.assert_close(out.view(T, N).double().cpu(), want, atol=2e-3, rtol=1e-3)
+    else:
+        _close(out.view(T, N), want)
+    assert bool((room[offset + T * N:] == 7).all()) and bool((room[:offset] == 7).all())
