@@ -697,7 +697,9 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
                 sumsq: Optional[torch.Tensor] = None, eps: float = 0.0,
                 residual: Optional[torch.Tensor] = None, norm_weight: Optional[torch.Tensor] = None,
                 norm_out: Optional[tuple] = None):
-    """y = x W^T (+ bias) on tcgen05 tensor cores; bfloat16 operands, float32 accumulate.
+    """y = x W^T (+ bias); bfloat16 operands, float32 accumulate.  On tcgen05 tensor cores, or, for
+    one to four tokens and a small weight, on the FMA pipes (``gemv_bf16.cuh``); ``plan``, ``cluster``
+    and ``two_sm`` are settings of the tensor-core kernels and choose those.
 
     With ``glu`` (True or "silu", or "gelu_tanh") the weight is [gate rows; up rows] ([2 I, K]) and
     the result is act(x gate^T) * (x up^T), [T, I].  ``out_dtype`` bfloat16 or float32.  K must be a
@@ -769,7 +771,7 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         return out if residual is None else ((out, sumsq_out) if norm_weight is not None else None)
     gemv_bytes = (GEMV_GATED_WEIGHT_BYTES if T == 1 and out_dtype == torch.bfloat16 else 0) if glu \
         else GEMV_WEIGHT_BYTES.get(T, 0)
-    if plan is None and rows * K * 2 <= gemv_bytes \
+    if plan is None and cluster is None and two_sm is None and rows * K * 2 <= gemv_bytes \
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0:
         f = _fn("gemm_bf16", "hb_gemv_bf16",
                 [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -927,8 +929,8 @@ def _library_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = x W^T + b.  float32: this package's FMA kernel.  bfloat16: the tcgen05 kernels,
-    or the library for plain products in the token ranges of GEMM_LIBRARY_TOKEN_RANGE and
+    """y = x W^T + b.  float32: this package's FMA kernels.  bfloat16: ``linear_bf16`` (tcgen05, or the
+    FMA pipes for few tokens and a small weight), or the library for plain products in the token ranges of GEMM_LIBRARY_TOKEN_RANGE and
     GEMM_LIBRARY_SMALL_TOKENS (small weight matrices); a K that is no multiple of 8 goes to
     the library too, as TMA needs 16-byte rows."""
     if x.dtype == torch.float32:

@@ -302,3 +302,17 @@ def test_results_at_addresses_that_are_no_whole_pieces(out_dtype, offset, cluste
     else:
         _close(out.view(T, N), want)
     assert bool((room[offset + T * N:] == 7).all()) and bool((room[:offset] == 7).all())
+
+
+@pytest.mark.parametrize("settings", [dict(cluster=True), dict(cluster=False), dict(two_sm=False), dict(plan=(16, 1)), {}])
+@pytest.mark.parametrize("glu", [False, True])
+def test_settings_of_the_tensor_core_kernels_choose_them(settings, glu, monkeypatch):
+    """One token and a small weight, which go to the FMA pipes unless the caller sets something of the others."""
+    o, seen = ops(), []
+    plain = o._fn
+    monkeypatch.setattr(o, "_fn", lambda lib, name, types: seen.append(name) or plain(lib, name, types))
+    x, w, _b = _case(1, 256, 512, 5, glu=glu)
+    got = o.linear_bf16(x.to(DEV), w.to(DEV), glu=glu, **settings)
+    want = x.double() @ w.double().T
+    _close(got, _gated(want[:, :256], want[:, 256:], True) if glu else want)
+    assert seen == ["hb_gemm_bf16" if settings else "hb_gemv_bf16"]
