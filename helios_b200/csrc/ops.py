@@ -681,14 +681,49 @@ def tc_gemm_supported(x: torch.Tensor, weight: torch.Tensor) -> bool:
 GLU_EPILOGUES = {False: 0, True: 1, "silu": 1, "gelu_tanh": 2}
 
 
-#: Plain products of so many tokens with a weight matrix of at most so many bytes run on the FMA pipes
-#: (``gemv_bf16.cuh``).  Tensor cores / FMA pipes, microseconds, chains over cold weights.  One token:
-#: 2 MB 4.95 / 2.30, 9 MB 6.06 / 5.08, 33 MB 9.98 / 8.62 and 9.22 / 8.86, 117 MB 22.5 / 24.9.  Two: 2 MB
-#: 4.99 / 2.64, 9 MB 6.15 / 6.27, 13 MB 6.40 / 5.97, 27 MB 9.41 / 10.6.  Four: 2 MB 4.74 / 3.54, 3 MB
-#: 4.01 / 3.93, 6 MB 4.86 / 6.01.
-GEMV_WEIGHT_BYTES = {1: 36 << 20, 2: 13 << 20, 3: 3 << 20, 4: 3 << 20}
-#: ... and gated units of one token with a weight of at most so many bytes
-GEMV_GATED_WEIGHT_BYTES = 18 << 20
+def gemv_features(tokens: int, K: int, gated: bool) -> int:
+    """The most features (result columns) of a product that the FMA pipes take (``gemv_bf16.cuh``): one to
+    four tokens, rows of K values.  Blocks have 16 features, two blocks an SM up to K = 2,048 (a warp
+    a row) and one above (two warps a row).  Where the last block has no place beside the others it runs
+    alone, and the tensor-core kernel, whose K slices fill the SMs whatever the features, is ahead; more tokens
+    cost the FMA pipes as many sums more and the tensor cores nothing, so that the rows get shorter.
+    Tensor cores / FMA pipes, chains over cold weights, as a ratio:
+    one token, up to one round of blocks 1.03 to 2.05 (K 128 to 65,536), over it 0.70 to 1.08 (up to K =
+    2,048; 4,752 features 0.99 to 1.21, 6,144 0.82 to 1.05) and 0.74 to 0.97 above;
+    two, one round, K to 1,024 1.07 to 1.81; K 1,280 to 2,048 0.94 to 1.45; 2,304 to 4,096 with 1,024 features
+    1.03 to 1.24, with 2,048 0.95 to 1.07; longer 0.87 to 1.02;
+    three and four, K to 1,024, 1,024 features 0.97 to 1.40, 2,048 0.92 to 1.06; longer 0.61 to 0.99.
+    A gated unit is chosen in a step, between the products before and behind it (a layer's four products,
+    us): one round 1.00 to 1.24 up to K = 4,864 (2 x 4,096 x 1,024 16.1 / 14.3, 2 x 2,048 x 2,048 20.5 / 18.7,
+    2 x 2,048 x 4,864 40.8 / 41.0) and 0.95 to 0.97 above; up to seven quarters of a round 0.99 to 1.08 at K up
+    to 1,024 (2 x 4,864 x 896 17.2 / 16.9, 2 x 8,192 x 1,024 22.3 / 21.3) and 0.90 to 0.97 above that; twice a
+    round 0.84 to 1.01.  In chains of its own it is level or behind at K of 1,280 to 2,048 (0.90 to 1.10) and
+    beyond one round (0.91 to 1.08)."""
+    one_round = 16 * sm_count() * (2 if K <= 2048 else 1)
+    if gated:
+        return (7 * one_round // 4 if K <= 1024 else one_round if K <= 4864 else 0) if tokens == 1 else 0
+    if tokens == 1 or (tokens == 2 and K <= 1024):
+        return one_round
+    if tokens == 2 and 2048 < K <= 4096:
+        return 1024
+    if tokens in (3, 4) and K <= 1024:
+        return 1280
+    return 0
+
+
+#: tokens -> bytes of a weight matrix up to which plain products run on the FMA pipes; None: what
+#: ``gemv_features`` says
+GEMV_WEIGHT_BYTES = {1: None, 2: None, 3: None, 4: None}
+#: ... and the most bytes of a gated unit's weight (measured so far)
+GEMV_GATED_WEIGHT_BYTES = 38 << 20
+
+
+def _on_fma_pipes(tokens: int, features: int, K: int, gated: bool) -> bool:
+    """Whether a product of one to four tokens runs on the FMA pipes."""
+    if gated:
+        return 4 * features * K <= GEMV_GATED_WEIGHT_BYTES and features <= gemv_features(tokens, K, True)
+    most = GEMV_WEIGHT_BYTES.get(tokens, 0)
+    return features <= gemv_features(tokens, K, False) if most is None else 2 * features * K <= most
 
 
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -769,9 +804,8 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         out = torch.empty((T, N), dtype=out_dtype, device=x.device)
     if T == 0:
         return out if residual is None else ((out, sumsq_out) if norm_weight is not None else None)
-    gemv_bytes = (GEMV_GATED_WEIGHT_BYTES if T == 1 and out_dtype == torch.bfloat16 else 0) if glu \
-        else GEMV_WEIGHT_BYTES.get(T, 0)
-    if plan is None and cluster is None and two_sm is None and rows * K * 2 <= gemv_bytes \
+    if plan is None and cluster is None and two_sm is None and T <= 4 \
+            and (not glu or out_dtype == torch.bfloat16) and _on_fma_pipes(T, N, K, bool(glu)) \
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0:
         f = _fn("gemm_bf16", "hb_gemv_bf16",
                 [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,

@@ -316,3 +316,18 @@ def test_settings_of_the_tensor_core_kernels_choose_them(settings, glu, monkeypa
     want = x.double() @ w.double().T
     _close(got, _gated(want[:, :256], want[:, 256:], True) if glu else want)
     assert seen == ["hb_gemm_bf16" if settings else "hb_gemv_bf16"]
+
+
+@pytest.mark.parametrize("T,N,K,gated,takes", [
+    (1, 16 * 296, 2048, False, True), (1, 16 * 296 + 1, 2048, False, False), (1, 16 * 148, 2056, False, True),
+    (1, 16 * 148 + 1, 2056, False, False), (1, 32000, 512, False, False), (1, 16, 65536, False, True),
+    (2, 16 * 296, 1024, False, True), (2, 16 * 296 + 1, 1024, False, False), (2, 128, 1032, False, False),
+    (2, 1024, 2056, False, True), (2, 1025, 2056, False, False), (2, 1024, 4096, False, True), (2, 16, 4104, False, False),
+    (3, 1280, 1024, False, True), (4, 1281, 1024, False, False), (4, 16, 1032, False, False), (5, 16, 64, False, False),
+    (1, 8288, 1024, True, True), (1, 8289, 1024, True, False), (1, 16 * 296, 1032, True, True), (1, 16 * 296 + 1, 1032, True, False),
+    (1, 1024, 4864, True, True), (1, 1024, 4872, True, False), (1, 16 * 296, 2048, True, True), (2, 16, 64, True, False)])
+def test_which_products_the_fma_pipes_take(T, N, K, gated, takes, monkeypatch):
+    """By rounds of blocks of 16 features on 148 SMs and by the length of a row, at the edges."""
+    o = ops()
+    monkeypatch.setattr(o, "sm_count", lambda device=None: 148)
+    assert o._on_fma_pipes(T, N, K, gated) == takes
