@@ -2004,6 +2004,26 @@ def linear_rows(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     return head_gemm(x.unsqueeze(1), weight.unsqueeze(0)).view(x.shape[0], weight.shape[0])
 
 
+def latent_block_rows(tokens: int, single: bool, heads: int, width: int, most_keys: int) -> int:
+    """Query rows a block of the tensor-core kernel of latent attention takes.  32, or 16 (four warps
+    instead of eight, half of which would have no rows) for steps of ``single`` tokens with at most 16
+    heads, where two such blocks then fit an SM (rows of ``width`` values) and there are ranges of 256 of
+    the ``most_keys`` keys, at most 32 a request, for more than the SMs.  In a captured step ``most_keys``
+    is the capacity, not a length, and requests that are shorter leave ranges empty; up to eight requests,
+    cut into many ranges, need a quarter more of them than SMs.
+    32 rows / 16 of 576 values, 16 heads, us, at capacities and lengths (keys): 4 requests, 20,480 and 250
+    to 3,000: 26.1 to 31.0 / 27.8 to 35.0; 8, 5,120 and 250 to 3,000: 22 to 33 / 23 to 31, 12,288 and the same:
+    30.5 to 41.6 / 29.7 to 37.8; 10, 4,096: 1.13 to 1.17 times as fast from 500 keys on, 0.96 times at 100;
+    16, 20,480: 29.6 to 56.8 / 24.3 to 42.8; 64, 1,000 keys 59 / 52, 3,000 138 / 96.  Below the line, 16
+    requests of 1,000 keys 24.7 / 28.6, 48 of 1,000 34.6 / 42.8.  Rows of 288, which fit twice as they are,
+    64 of 1,000 28 / 33."""
+    row_bytes = 2 * (width + 8)
+    fits = 96 * row_bytes > 108 * 1024 and 80 * row_bytes <= 108 * 1024
+    ranges = tokens * min(32, max(1, most_keys // 256))
+    least = sm_count() * 5 // 4 if tokens <= 8 else sm_count()
+    return 16 if single and heads <= 16 and fits and ranges > least else 32
+
+
 def latent_attention(ctx, q_lat: torch.Tensor, q_rot: torch.Tensor, pages: torch.Tensor,
                      block_table: torch.Tensor, rank: int, rot: int, page_size: int,
                      scale: float, window: Optional[int] = None,
@@ -2033,16 +2053,9 @@ def latent_attention(ctx, q_lat: torch.Tensor, q_rot: torch.Tensor, pages: torch
             raise KernelError(f"{sink_values.numel()} sink values for {H} heads")
     out = torch.empty((T, H, rank), dtype=q_lat.dtype, device=q_lat.device)
     if LATENT_ATTENTION_TENSOR_CORES and q_lat.dtype == torch.bfloat16 and rank % 32 == 0 and rot % 16 == 0:
-        # 32 query rows a block: (token, head) pairs of one request, which share every key.  Steps of
-        # single tokens with at most 16 heads take 16 rows (four warps instead of eight, half of which
-        # would have no rows) where two such blocks then fit an SM and there are ranges of keys for more
-        # than the SMs.  32 rows / 16, microseconds: 64 requests of 1,000 rows of 576 53 / 40, 16 of 3,000
-        # 51 / 45, 24 of 1,000 32 / 32, 8 of 1,024 24 / 27; rows of 288, which fit twice as they are,
-        # 64 of 1,000 28 / 33.
+        # query rows a block: (token, head) pairs of one request, which share every key
         max_keys = min(ctx.max_context_len, window) if window else ctx.max_context_len
-        row_bytes = 2 * (rank + rot + 8)
-        rows = 16 if T == len(ctx.seqs) and H <= 16 and 96 * row_bytes > 108 * 1024 \
-            and 80 * row_bytes <= 108 * 1024 and T * max(1, max_keys // 256) > sm_count() else 32
+        rows = latent_block_rows(T, T == len(ctx.seqs), H, rank + rot, max_keys)
         hpb = min(H, rows)
         tpt = 1 if rows == 16 else rows // hpb
         tiles = _step_tiles(ctx, tpt, False, q_lat.device)

@@ -868,3 +868,26 @@ def test_short_convolution_a_token_a_step_is_the_whole_sequence_bit_for_bit(dtyp
     assert torch.equal(got[:2], run(x[0, :2], [2], b, [4])) and torch.equal(got[2:], run(x[0, 2:3], [1], b, [0]))
     assert torch.equal(a, b)
 
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,rank,rot,count", [(16, 512, 64, 200), (1, 512, 96, 170), (16, 480, 112, 333)])
+@pytest.mark.parametrize("window", [None, 40, 700])
+def test_latent_attention_with_sixteen_rows_a_block_at_every_window(heads, rank, rot, count, window):
+    """As above, where the rule chooses the kernel for each window and with the sink."""
+    from helios_b200.csrc import ops
+
+    assert ops.latent_block_rows(count, True, heads, rank + rot, min(1000, window or 1000)) == 16
+    test_latent_attention_of_many_single_tokens_takes_sixteen_rows_a_block(heads, rank, rot, count, window)
+
+
+@pytest.mark.parametrize("tokens,single,heads,width,keys,rows", [
+    (1, True, 16, 576, 131072, 32), (4, True, 16, 576, 20480, 32), (8, True, 16, 576, 5120, 32), (8, True, 16, 576, 6144, 16),
+    (8, True, 16, 576, 32768, 16), (10, True, 16, 576, 4096, 16), (9, True, 16, 576, 4096, 32), (16, True, 16, 576, 2560, 16),
+    (16, True, 16, 576, 2303, 32), (64, True, 16, 576, 1000, 16), (64, False, 16, 576, 1000, 32), (64, True, 17, 576, 1000, 32),
+    (64, True, 16, 288, 1000, 32), (64, True, 16, 704, 1000, 32), (149, True, 1, 576, 1, 16), (148, True, 1, 576, 511, 32)])
+def test_query_rows_a_block_of_latent_attention(tokens, single, heads, width, keys, rows, monkeypatch):
+    """On 148 SMs: the edges of the ranges, of a quarter more for up to eight requests, and of what fits an SM."""
+    from helios_b200.csrc import ops
+
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    assert ops.latent_block_rows(tokens, single, heads, width, keys) == rows
