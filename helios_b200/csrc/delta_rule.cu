@@ -578,15 +578,18 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
 }
 
 // Steps of single tokens (decode), bound by reading and writing the states once: a block owns
-// the whole S of a (request, head), 128 columns of it, warp `part` the rows a thread of that
-// part owns above, four neighbouring columns a lane, so that a row is one 512-byte access and
-// all of a block's rows are in flight at once.  The preparation is done here as well (every
-// warp computes the norms; nothing goes through memory), and every sum has the order of the two
-// kernels above: dot products by element of a group of four, then the parts pairwise.
+// the whole S of a (request, head), 4 LANES columns of it, the LANES threads of a `part` the rows a
+// thread of that part owns above, four neighbouring columns a thread, so that a row is one access of
+// up to 512 bytes and all of a block's rows are in flight at once.  The preparation is done here as
+// well (every warp computes the norms; nothing goes through memory), and every sum has the order of the
+// two kernels above: dot products by element of a group of four, then the parts pairwise.  LANES is 32, or
+// 16 or 8 where the values of a head are 64 or 32 columns, so that no lane is idle (160 requests, two
+// kernels / 32 lanes / this, µs: 16 heads of 24 x 24 14.3 / 25.2 / 9.2,
+// 8 of 64 x 64 15.8 / 17.4 / 12.0).
 // 16 heads of 128 x 128, preparation and recurrence: 42 -> 34 µs at 64 requests, 100 -> 81 at 160,
 // 9.7 -> 7.5 at 8, 7.8 -> 5.5 at one.
-template <typename T, int G>
-__global__ void __launch_bounds__(32 * DR_PARTS, G <= 4 ? 2 : 1)
+template <typename T, int G, int LANES>
+__global__ void __launch_bounds__(LANES * DR_PARTS, G <= 4 ? 2 : 1)
 delta_step_kernel(float* __restrict__ o, const T* __restrict__ qkv, int qkv_ld, int q_off, int k_off, int v_off,
                   const T* __restrict__ beta_raw, int beta_ld, const T* __restrict__ a_raw, int a_ld,
                   const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ state,
@@ -596,9 +599,9 @@ delta_step_kernel(float* __restrict__ o, const T* __restrict__ qkv, int qkv_ld, 
   pdl_wait();
   constexpr int STEP = 4 * DR_PARTS, DK = STEP * G;
   __shared__ __align__(16) float kqg[3][DK];
-  __shared__ __align__(16) float sums[2][DR_PARTS][128];
-  const int s = blockIdx.x, h = blockIdx.y, part = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = blockIdx.z * 128 + 4 * lane;
+  __shared__ __align__(16) float sums[2][DR_PARTS][4 * LANES];
+  const int s = blockIdx.x, h = blockIdx.y, part = threadIdx.x / LANES, piece = threadIdx.x % LANES;
+  const int col = (blockIdx.z * LANES + piece) * 4;
   const bool live = col < dv;                         // dv is a multiple of four here
   const int t0 = cu_tokens[s], n = cu_tokens[s + 1] - t0;
   if (n <= 0) return;
@@ -621,8 +624,8 @@ delta_step_kernel(float* __restrict__ o, const T* __restrict__ qkv, int qkv_ld, 
       return live ? make_float4(to_float(p[0]), to_float(p[1]), to_float(p[2]), to_float(p[3]))
                   : make_float4(0.f, 0.f, 0.f, 0.f);
     }();
-    const DeltaNorms nm = delta_norms(kr, qr, dk, lane);
-    for (int i = threadIdx.x; i < DK; i += 32 * DR_PARTS) {
+    const DeltaNorms nm = delta_norms(kr, qr, dk, threadIdx.x & 31);
+    for (int i = threadIdx.x; i < DK; i += LANES * DR_PARTS) {
       kqg[0][i] = i < dk ? to_float(kr[i]) * nm.kn : 0.f;
       kqg[1][i] = i < dk ? to_float(qr[i]) * nm.qn : 0.f;
       kqg[2][i] = i < dk ? delta_decay(to_float(a_raw[(size_t)t * a_ld + (size_t)h * dk + i]) + dt_bias[(size_t)h * dk + i], rate) : 0.f;
@@ -649,13 +652,13 @@ delta_step_kernel(float* __restrict__ o, const T* __restrict__ qkv, int qkv_ld, 
       }
     }
     auto add = [](float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); };
-    *reinterpret_cast<float4*>(&sums[0][part][4 * lane]) = add(add(d[0], d[1]), add(d[2], d[3]));
-    *reinterpret_cast<float4*>(&sums[1][part][4 * lane]) = add(add(r[0], r[1]), add(r[2], r[3]));
+    *reinterpret_cast<float4*>(&sums[0][part][4 * piece]) = add(add(d[0], d[1]), add(d[2], d[3]));
+    *reinterpret_cast<float4*>(&sums[1][part][4 * piece]) = add(add(r[0], r[1]), add(r[2], r[3]));
     __syncthreads();
     auto parts_sum = [&](int which) {
       float4 p[DR_PARTS];
 #pragma unroll
-      for (int i = 0; i < DR_PARTS; ++i) p[i] = *reinterpret_cast<const float4*>(&sums[which][i][4 * lane]);
+      for (int i = 0; i < DR_PARTS; ++i) p[i] = *reinterpret_cast<const float4*>(&sums[which][i][4 * piece]);
 #pragma unroll
       for (int x = 1; x < DR_PARTS; x *= 2)
 #pragma unroll
@@ -705,18 +708,25 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
   // one token a request: the state's rows in whole 16-byte pieces, everything in one launch
   if (n_tokens == n_seqs && dv % 4 == 0 && state_stride % 4 == 0 &&
       ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(o)) & 15) == 0) {
-    const dim3 grid1(n_seqs, heads, (dv + 127) / 128);
-#define HB_DR_STEP(G)                                                                                        \
+    const int lanes = dv <= 32 ? 8 : dv <= 64 ? 16 : 32;
+    const dim3 grid1(n_seqs, heads, (dv + 4 * lanes - 1) / (4 * lanes));
+#define HB_DR_STEP_LANES(G, LANES)                                                                           \
     HB_DISPATCH_DTYPE(act_dt, TA,                                                                            \
-      hb_launch(delta_step_kernel<TA, G>, grid1, dim3(32 * DR_PARTS), 0, stream, o, (const TA*)qkv, qkv_ld,  \
-                q_off, k_off, v_off, (const TA*)beta_raw, beta_ld, (const TA*)a_raw, a_ld, a_log, dt_bias,   \
-                state, state_stride, cu_tokens, slots, heads, kv_heads, dk, dv))
+      hb_launch(delta_step_kernel<TA, G, LANES>, grid1, dim3(LANES * DR_PARTS), 0, stream, o,                \
+                (const TA*)qkv, qkv_ld, q_off, k_off, v_off, (const TA*)beta_raw, beta_ld,                   \
+                (const TA*)a_raw, a_ld, a_log, dt_bias, state, state_stride, cu_tokens, slots, heads,        \
+                kv_heads, dk, dv))
+#define HB_DR_STEP(G)                                                                                        \
+    if (lanes == 8) HB_DR_STEP_LANES(G, 8);                                                                  \
+    else if (lanes == 16) HB_DR_STEP_LANES(G, 16);                                                           \
+    else HB_DR_STEP_LANES(G, 32)
     if (grid1.z > 65535) return HB_BAD_ARGUMENT;
-    if (dk <= 32) HB_DR_STEP(1);
-    else if (dk <= 64) HB_DR_STEP(2);
-    else if (dk <= 128) HB_DR_STEP(4);
-    else HB_DR_STEP(8);
+    if (dk <= 32) { HB_DR_STEP(1); }
+    else if (dk <= 64) { HB_DR_STEP(2); }
+    else if (dk <= 128) { HB_DR_STEP(4); }
+    else { HB_DR_STEP(8); }
 #undef HB_DR_STEP
+#undef HB_DR_STEP_LANES
     return hb_check_launch();
   }
   const int dkp = (dk + 3) / 4 * 4;

@@ -891,3 +891,36 @@ def test_query_rows_a_block_of_latent_attention(tokens, single, heads, width, ke
 
     monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
     assert ops.latent_block_rows(tokens, single, heads, width, keys) == rows
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dk,dv", [(96, 32), (40, 36), (24, 64), (128, 68), (200, 64)])
+def test_delta_rule_a_token_a_step_at_the_widths_of_its_blocks(dk, dv):
+    """As above: values of exactly 32 and 64 columns a head, and of four more."""
+    test_delta_rule_a_token_a_step_is_the_walk_over_all_tokens_bit_for_bit(dk, dv)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dk,dv", [(24, 24), (64, 64), (128, 128), (200, 36)])
+def test_delta_rule_of_as_many_tokens_as_requests_but_not_one_each(dk, dv):
+    """The kernel for single tokens walks what a request has, and leaves a request without tokens alone."""
+    from types import SimpleNamespace
+    from helios_b200.csrc import ops
+
+    dev, heads = "cuda", 2
+    g = torch.Generator().manual_seed(dk)
+    new = lambda *shape: torch.randn(*shape, generator=g).to(dev)
+    qkv, beta, a = new(4, heads * (2 * dk + dv)), new(4, heads) + 2, new(4, heads * dk) - 2
+    a_log, dt_bias, first = new(heads) * 0.3, new(heads * dk) * 0.3, new(5, heads * dk * dv)
+
+    def run(t0, lens, state, slots):
+        cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).int().to(dev)
+        ctx = SimpleNamespace(cu_tokens=cu, slots=torch.tensor(slots, dtype=torch.int32, device=dev), num_seqs=len(lens))
+        part = slice(t0, t0 + sum(lens))
+        return ops.delta_rule(ctx, qkv[part], (0, heads * dk, 2 * heads * dk), beta[part], a[part], a_log, dt_bias, state, heads,
+                              heads, dk, dv)
+
+    state, alone = first.clone(), first.clone()
+    got = run(0, [0, 3, 0, 1], state, [1, 4, 2, 0])
+    assert torch.equal(got[:3], run(0, [3], alone, [4])) and torch.equal(got[3:], run(3, [1], alone, [0]))
+    assert torch.equal(state, alone)
