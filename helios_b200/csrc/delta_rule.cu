@@ -288,10 +288,10 @@ constexpr int DR_PARTS = 8;         // threads a column of S is spread over
 // shared-memory path does (a 16-byte load takes four cycles whatever it broadcasts; 212 of 345 cycles
 // a token), and a row's piece is read once for two columns; 32 columns a block where that leaves two
 // blocks an SM.  One column a thread / two, µs: one request of 2,048 tokens 447 / 498; 3 of 700 328 /
-// 284; 24 of 40 150 / 110; 64 of 8 130 / 103.
+// 284; 24 of 40 150 / 110; 64 of 8 130 / 103.  Keys of more than 128 values take one column a thread (two
+// do not fit its registers) and are padded to 160, 192 or 256 (8 heads of 160 x 160, padded to 256 / 160,
+// µs: one request of 2,048 tokens 770 / 491, 24 of 40 187 / 114, 64 of 8 175 / 92).
 constexpr int DR_COLS = 16, DR_COLS_WIDE = 32;
-constexpr int DR_SMS = 148;
-constexpr int DR_WIDE_BLOCKS = 296;
 
 __device__ __forceinline__ void dr_cp_async16(void* smem, const void* gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
@@ -700,10 +700,10 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
                             const float* a_log, const float* dt_bias, float* state,
                             long state_stride, const int* cu_tokens, const int* slots, int n_tokens,
                             int n_seqs, int heads, int kv_heads, int dk, int dv, int act_dt,
-                            cudaStream_t stream) {
+                            int sms, cudaStream_t stream) {
   if (n_seqs <= 0 || n_tokens <= 0) return HB_OK;
   if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || dk <= 0 || dk > 256 || dv <= 0 ||
-      heads > 65535 || scratch == nullptr)
+      heads > 65535 || scratch == nullptr || sms <= 0)
     return HB_BAD_ARGUMENT;
   // one token a request: the state's rows in whole 16-byte pieces, everything in one launch
   if (n_tokens == n_seqs && dv % 4 == 0 && state_stride % 4 == 0 &&
@@ -737,8 +737,8 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
     hb_launch(delta_prepare_kernel<TA>, dim3((n_rows + 3) / 4), dim3(128), 0, stream, kqg, beta,
               (const TA*)qkv, qkv_ld, q_off, k_off, (const TA*)beta_raw, beta_ld, (const TA*)a_raw, a_ld,
               a_log, dt_bias, n_rows, heads, kv_heads, dk, dkp));
-  const bool alone = (long)n_seqs * heads * ((dv + DR_COLS - 1) / DR_COLS) <= DR_SMS;
-  const int cols = dk <= 128 && (long)n_seqs * heads * ((dv + DR_COLS_WIDE - 1) / DR_COLS_WIDE) >= DR_WIDE_BLOCKS ? DR_COLS_WIDE : DR_COLS;
+  const bool alone = (long)n_seqs * heads * ((dv + DR_COLS - 1) / DR_COLS) <= sms;
+  const int cols = dk <= 128 && (long)n_seqs * heads * ((dv + DR_COLS_WIDE - 1) / DR_COLS_WIDE) >= 2L * sms ? DR_COLS_WIDE : DR_COLS;
   dim3 grid(n_seqs, heads, (dv + cols - 1) / cols);
 #define HB_DR_LAUNCH_COLS(DKMAX, COLS, W)                                                            \
   HB_DISPATCH_DTYPE(act_dt, TA,                                                                   \
@@ -756,6 +756,8 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
   if (dk <= 32) { HB_DR_LAUNCH(32); }
   else if (dk <= 64) { HB_DR_LAUNCH(64); }
   else if (dk <= 128) { HB_DR_LAUNCH(128); }
+  else if (dk <= 160) HB_DR_LAUNCH_COLS(160, DR_COLS, 1);
+  else if (dk <= 192) HB_DR_LAUNCH_COLS(192, DR_COLS, 1);
   else HB_DR_LAUNCH_COLS(256, DR_COLS, 1);
 #undef HB_DR_LAUNCH_COLS
 #undef HB_DR_LAUNCH

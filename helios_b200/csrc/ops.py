@@ -2254,11 +2254,12 @@ def delta_rule(ctx, qkv: torch.Tensor, offsets, beta_raw: torch.Tensor, a_raw: t
     scratch = torch.empty((T * heads * (3 * (-(-dk // 4) * 4) + 2),), dtype=torch.float32, device=qkv.device)
     f = _fn("delta_rule", "hb_delta_rule",
             [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
-             c_void_p, c_void_p, _LONG, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+             c_void_p, c_void_p, _LONG, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+             c_void_p])
     _run(f(_p(o), _p(scratch), _p(qkv), qkv.shape[1], offsets[0], offsets[1], offsets[2], _p(beta_raw),
            beta_raw.stride(0), _p(a_raw), a_raw.stride(0), _p(a_log), _p(dt_bias), _p(state),
            state.stride(0), _p(ctx.cu_tokens), _p(ctx.slots), T, ctx.num_seqs, heads, kv_heads, dk, dv,
-           _dt(qkv.dtype), _stream()), "delta_rule")
+           _dt(qkv.dtype), sm_count(qkv.device), _stream()), "delta_rule")
     return o
 
 

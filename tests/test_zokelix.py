@@ -924,3 +924,10 @@ def test_delta_rule_of_as_many_tokens_as_requests_but_not_one_each(dk, dv):
     got = run(0, [0, 3, 0, 1], state, [1, 4, 2, 0])
     assert torch.equal(got[:3], run(0, [3], alone, [4])) and torch.equal(got[3:], run(3, [1], alone, [0]))
     assert torch.equal(state, alone)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dk,dv", [(160, 36), (161, 4), (192, 30), (193, 16)])
+def test_delta_rule_at_the_sizes_its_keys_are_padded_to(dk, dv):
+    """As above, for keys of more than 128 values."""
+    test_delta_rule_a_token_a_step_is_the_walk_over_all_tokens_bit_for_bit(dk, dv)
