@@ -386,12 +386,19 @@ __device__ __forceinline__ float dr_hi(uint64_t v) { return __uint_as_float((uin
 // threads: thread `part` keeps the rows 4 (DR_PARTS m + part) .. + 3, and the two sums over dk
 // are finished with shuffles.  A thread has W (1 or 2) columns.  COLS and W change which block and
 // thread own a column, never a sum's order.
-template <typename T, int DK, int COLS, int W>
+// MANY: for launches of more blocks than SMs.  A request's blocks follow one another, so that those of a
+// long request lie on SMs of their own; and the state's columns go in whole 16-byte pieces (`in_pieces`) by
+// way of the second staging buffer.  A warp's threads hold four (or eight) neighbouring columns of eight rows,
+// so that their own loads fetch half a sector each, which is most of the time of a few tokens a request.
+// Value by value / so, 16 heads of 128 x 128, µs: 64 requests of 4 tokens 70 / 56, of 2 62 / 47, of 8 95 / 77; 7 of one
+// token beside one of 500 223 / 139.  4 heads of 256 x 256: 64 of 8 123 / 109.  Keys of at most 64 values gain less
+// than the longer code costs their walk (3 requests of 700 tokens, 8 heads of 64 x 64, 112 / 122).
+template <typename T, int DK, int COLS, int W, bool MANY>
 __global__ void __launch_bounds__(COLS * DR_PARTS / W)
 delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const float* __restrict__ beta,
                   const T* __restrict__ qkv, int qkv_ld, int v_off, float* __restrict__ state,
                   long state_stride, const int* __restrict__ cu_tokens, const int* __restrict__ slots,
-                  int heads, int dk, int dkp, int dv) {
+                  int heads, int dk, int dkp, int dv, int in_pieces) {
   // Neither launched early nor releasing the next kernel early: a long prompt of one request
   // is a few blocks that run for a long time.  Launched while the kernel before still holds
   // the SMs they land two to an SM wherever room is, and share its issue slots for all that
@@ -406,9 +413,15 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
   float* stage_buf = dr_sm;                         // [2][CHUNK][ROW]
   float* bs = dr_sm + 2 * DR_CHUNK * ROW;           // [2][CHUNK][2]: beta, k . q
   float* vs = bs + 4 * DR_CHUNK;                    // [2][CHUNK][COLS]
-  const int s = blockIdx.x, h = blockIdx.y;
+  int s = blockIdx.x, h = blockIdx.y, col_block = blockIdx.z;
+  if constexpr (MANY) {
+    const int col_blocks = (dv + COLS - 1) / COLS;
+    s = blockIdx.x / col_blocks / heads;
+    h = blockIdx.x / col_blocks - s * heads;
+    col_block = blockIdx.x % col_blocks;
+  }
   const int part = threadIdx.x % DR_PARTS, lcol = threadIdx.x / DR_PARTS;
-  const int col = blockIdx.z * COLS + W * lcol;
+  const int col = col_block * COLS + W * lcol;
   bool live[W];
 #pragma unroll
   for (int w = 0; w < W; ++w) live[w] = col + w < dv;
@@ -417,6 +430,7 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
   const T* v_head = qkv + v_off + (size_t)h * dv;
 
   uint64_t S[W][G][2];
+  if constexpr (!MANY) {
 #pragma unroll
   for (int m = 0; m < G; ++m)
 #pragma unroll
@@ -427,9 +441,13 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
         S[w][m][e] = dr_pack((live[w] && i < dk) ? S_g[(size_t)i * dv + col + w] : 0.f,
                              (live[w] && i + 1 < dk) ? S_g[(size_t)(i + 1) * dv + col + w] : 0.f);
       }
+  }
   // the staged rows behind dkp hold nothing: k = q = g = 0 there, once for all tokens
+  auto clear_padding = [&] {
   for (int idx = threadIdx.x; idx < 2 * DR_CHUNK * 3 * (DK - dkp); idx += THREADS)
     stage_buf[idx / (DK - dkp) * DK + dkp + idx % (DK - dkp)] = 0.f;
+  };
+  if constexpr (!MANY) clear_padding();
 
   // (nothing here waits for a load: a warp issues in order, and a conversion or a store of what was
   // just asked for would hold up the tokens of the chunk that is there)
@@ -464,11 +482,48 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
     }
   };
 
-  if (n > 0) {
+  const bool pieces = MANY && in_pieces;
+  constexpr int TLINE = COLS + 4;
+  static_assert(!MANY || DK * TLINE <= DR_CHUNK * ROW, "");
+  if constexpr (MANY) {
+    if (n <= 0) return;
+    float* tile = stage_buf + DR_CHUNK * ROW;
+    if (pieces) {
+      for (int idx = threadIdx.x; idx < dk * (COLS / 4); idx += THREADS) {
+        const int i = idx / (COLS / 4), c = 4 * (idx % (COLS / 4));
+        if (col_block * COLS + c < dv)
+          dr_cp_async16(tile + i * TLINE + c, S_g + (size_t)i * dv + col_block * COLS + c);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
     stage(0, 0);
     fetch_v(0);
+    asm volatile("cp.async.commit_group;\n" ::);
+    if (pieces) {
+      asm volatile("cp.async.wait_group 1;\n" ::);
+      __syncthreads();
+    }
+    const float* from = pieces ? tile + W * lcol : S_g + col;
+    const int line = pieces ? TLINE : dv;
+#pragma unroll
+    for (int m = 0; m < G; ++m)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const int i = STEP * m + 4 * part + 2 * e;
+          S[w][m][e] = dr_pack((live[w] && i < dk) ? from[(size_t)i * line + w] : 0.f,
+                               (live[w] && i + 1 < dk) ? from[(size_t)(i + 1) * line + w] : 0.f);
+        }
+    if (pieces && dkp < DK) __syncthreads();           // the zeros go where the tile lies
+    clear_padding();
+  } else {
+    if (n > 0) {
+      stage(0, 0);
+      fetch_v(0);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
   }
-  asm volatile("cp.async.commit_group;\n" ::);
   int b = 0;
   float* o_next = o + (size_t)t0 * heads * dv + (size_t)h * dv + col;
   const size_t o_step = (size_t)heads * dv;
@@ -563,6 +618,30 @@ delta_rule_kernel(float* __restrict__ o, const float* __restrict__ kqg, const fl
     b ^= 1;
   }
   asm volatile("cp.async.wait_group 0;\n" ::);
+  if (pieces) {
+    __syncthreads();                                   // nobody reads staged rows any more
+    float* to = stage_buf + W * lcol;
+#pragma unroll
+    for (int w = 0; w < W; ++w)
+      if (live[w]) {
+#pragma unroll
+        for (int m = 0; m < G; ++m)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int i = STEP * m + 4 * part + 2 * e;
+            if (i < dk) to[i * TLINE + w] = dr_lo(S[w][m][e]);
+            if (i + 1 < dk) to[(i + 1) * TLINE + w] = dr_hi(S[w][m][e]);
+          }
+      }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < dk * (COLS / 4); idx += THREADS) {
+      const int i = idx / (COLS / 4), c = 4 * (idx % (COLS / 4));
+      if (col_block * COLS + c < dv)
+        *reinterpret_cast<float4*>(S_g + (size_t)i * dv + col_block * COLS + c) =
+            *reinterpret_cast<const float4*>(stage_buf + i * TLINE + c);
+    }
+    return;
+  }
 #pragma unroll
   for (int w = 0; w < W; ++w)
     if (live[w]) {
@@ -706,8 +785,8 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
       heads > 65535 || scratch == nullptr || sms <= 0)
     return HB_BAD_ARGUMENT;
   // one token a request: the state's rows in whole 16-byte pieces, everything in one launch
-  if (n_tokens == n_seqs && dv % 4 == 0 && state_stride % 4 == 0 &&
-      ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(o)) & 15) == 0) {
+  const int pieces = dv % 4 == 0 && state_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0 ? 1 : 0;
+  if (n_tokens == n_seqs && pieces && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
     const int lanes = dv <= 32 ? 8 : dv <= 64 ? 16 : 32;
     const dim3 grid1(n_seqs, heads, (dv + 4 * lanes - 1) / (4 * lanes));
 #define HB_DR_STEP_LANES(G, LANES)                                                                           \
@@ -739,26 +818,32 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
               a_log, dt_bias, n_rows, heads, kv_heads, dk, dkp));
   const bool alone = (long)n_seqs * heads * ((dv + DR_COLS - 1) / DR_COLS) <= sms;
   const int cols = dk <= 128 && (long)n_seqs * heads * ((dv + DR_COLS_WIDE - 1) / DR_COLS_WIDE) >= 2L * sms ? DR_COLS_WIDE : DR_COLS;
-  dim3 grid(n_seqs, heads, (dv + cols - 1) / cols);
-#define HB_DR_LAUNCH_COLS(DKMAX, COLS, W)                                                            \
+  const long blocks = (long)n_seqs * heads * ((dv + cols - 1) / cols);
+  if (blocks > 0x7fffffffL) return HB_BAD_ARGUMENT;
+#define HB_DR_LAUNCH_COLS(DKMAX, COLS, W, MANY)                                                      \
   HB_DISPATCH_DTYPE(act_dt, TA,                                                                   \
     const size_t smem = (2 * DR_CHUNK * 3 * DKMAX + 4 * DR_CHUNK + 2 * DR_CHUNK * COLS) * sizeof(float); \
     if (smem > 48 * 1024)                                                                         \
-      cudaFuncSetAttribute(delta_rule_kernel<TA, DKMAX, COLS, W>,                                 \
+      cudaFuncSetAttribute(delta_rule_kernel<TA, DKMAX, COLS, W, MANY>,                           \
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-    delta_rule_kernel<TA, DKMAX, COLS, W><<<grid, dim3(COLS * DR_PARTS / W), smem, stream>>>(              \
+    const dim3 grid = MANY ? dim3((unsigned)blocks) : dim3(n_seqs, heads, (dv + cols - 1) / cols); \
+    delta_rule_kernel<TA, DKMAX, COLS, W, MANY><<<grid, dim3(COLS * DR_PARTS / W), smem, stream>>>(   \
         o, (const float*)kqg, (const float*)beta, (const TA*)qkv, qkv_ld, v_off, state,           \
-        state_stride, cu_tokens, slots, heads, dk, dkp, dv))
+        state_stride, cu_tokens, slots, heads, dk, dkp, dv, pieces))
 #define HB_DR_LAUNCH(DKMAX)                                                                       \
-  if (alone) HB_DR_LAUNCH_COLS(DKMAX, DR_COLS, 1);                                                \
-  else if (cols == DR_COLS) HB_DR_LAUNCH_COLS(DKMAX, DR_COLS, 2);                                 \
-  else HB_DR_LAUNCH_COLS(DKMAX, DR_COLS_WIDE, 2)
+  if (alone) HB_DR_LAUNCH_COLS(DKMAX, DR_COLS, 1, false);                                         \
+  else if (cols == DR_COLS) HB_DR_LAUNCH_COLS(DKMAX, DR_COLS, 2, (DKMAX >= 128));                 \
+  else HB_DR_LAUNCH_COLS(DKMAX, DR_COLS_WIDE, 2, (DKMAX >= 128))
+#define HB_DR_LAUNCH_LONG(DKMAX)                                                                  \
+  if (alone) HB_DR_LAUNCH_COLS(DKMAX, DR_COLS, 1, false);                                         \
+  else HB_DR_LAUNCH_COLS(DKMAX, DR_COLS, 1, true)
   if (dk <= 32) { HB_DR_LAUNCH(32); }
   else if (dk <= 64) { HB_DR_LAUNCH(64); }
   else if (dk <= 128) { HB_DR_LAUNCH(128); }
-  else if (dk <= 160) HB_DR_LAUNCH_COLS(160, DR_COLS, 1);
-  else if (dk <= 192) HB_DR_LAUNCH_COLS(192, DR_COLS, 1);
-  else HB_DR_LAUNCH_COLS(256, DR_COLS, 1);
+  else if (dk <= 160) { HB_DR_LAUNCH_LONG(160); }
+  else if (dk <= 192) { HB_DR_LAUNCH_LONG(192); }
+  else { HB_DR_LAUNCH_LONG(256); }
+#undef HB_DR_LAUNCH_LONG
 #undef HB_DR_LAUNCH_COLS
 #undef HB_DR_LAUNCH
   return hb_check_launch();
