@@ -679,14 +679,15 @@ def test_a_threshold_at_zero_keeps_the_negative_zeros(k, p):
 @pytest.mark.parametrize("K", [4, 16, 20, 124, 128, 132, 512, 900, 4096, 4868, 19000])
 @pytest.mark.parametrize("M,N", [(1, 1), (1, 1201), (2, 130), (3, 37), (4, 600), (5, 64), (8, 9), (9, 33), (16, 5), (17, 40)])
 def test_gemm_f32_of_few_rows_is_the_tiled_product_bit_for_bit(M, N, K, monkeypatch):
-    """Edges of runs (16), of blocks of runs (128), of a warp's piece (512) and of a row's place in
-    shared memory; both kernels add in the same order, and a row alone is the row in the batch."""
+    """Edges of runs (16), of quarters (whole tiles of 32, so 128 for the four), of a warp's piece (512) and of a
+    row's place in shared memory; both kernels add in the same order, and a row alone is the row in the batch."""
     g = torch.Generator().manual_seed(M * N + K)
     x, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
     got = ops().linear_f32(x.to(DEV), w.to(DEV), b.to(DEV))
     want = x.double() @ w.double().T + b.double()
-    # |error| <= (additions an element goes through) * eps * sum |x||w|; sums of 16, of 8, of K / 128
-    bound = (26 + K / 128) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs()) + 1e-30
+    # |error| <= (roundings an element goes through) * eps * sum |x||w|: 16 in its run, one a run of its
+    # quarter (2 for each 128 of K), two for the quarters, one for the bias
+    bound = (19 + 2 * -(-K // 128)) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs()) + 1e-30
     assert ((got.cpu().double() - want).abs() <= bound).all()
     alone = ops().linear_f32(x[M - 1:].contiguous().to(DEV), w.to(DEV), b.to(DEV))
     assert torch.equal(got[M - 1:], alone)
