@@ -6,15 +6,15 @@
 //   S <- S + k u^T
 //   o  = S^T q              (the read-out sees this token's write)
 //
-// The columns of S never mix: a thread owns one column (dk values in registers) and walks
-// the request's tokens in order, so a request's numbers do not depend on how its tokens
-// were cut into steps or on the rest of the batch.  State, decays, gates, unit norms and
+// The columns of S never mix: eight threads own a column (or two), an eighth of its dk values in
+// registers each, and walk the request's tokens in order, so a request's numbers do not depend on
+// how its tokens were cut into steps or on the rest of the batch.  State, decays, gates, unit norms and
 // the recurrence are float32.
 //
 // Kernels: `causal_conv_silu` (short causal convolution over time per channel + silu, the
 // taps - 1 inputs before a step's first token taken from the request's slot),
-// `causal_conv_state` (leaves the last taps - 1 inputs in the slot), `delta_prepare` and
-// `delta_rule` (the recurrence) and `gated_rmsnorm` (o / rms(o) * weight * sigmoid(gate) per head).
+// `causal_conv_state` (leaves the last taps - 1 inputs in the slot; steps of single tokens do both in
+// `causal_conv_step`), `delta_prepare` and `delta_rule` (the recurrence; `delta_step` both for single tokens) and `gated_rmsnorm` (o / rms(o) * weight * sigmoid(gate) per head).
 #include "common.cuh"
 #include "causal_conv.cuh"
 
@@ -267,8 +267,8 @@ HB_EXPORT int hb_causal_conv_silu(void* out, const void* x, int ld, const float*
 }
 
 // ---------------------------------------------------------------- the recurrence
-// Two kernels, and one that does both for steps of single tokens.  `delta_prepare` is parallel over (token, head): unit-norm k and q (q also
-// times dk^-1/2), the decays g = exp(-exp(A_log) softplus(a + dt_bias)) and the write strength
+// Two kernels, and one that does both for steps of single tokens.  `delta_prepare` is parallel over
+// (token, head): unit-norm k and q (q also times dk^-1/2), the decays g = exp(-exp(A_log) softplus(a + dt_bias)) and the write strength
 // beta = sigmoid(b), all float32, left as kqg [T, heads, 3, dkp] (dkp = dk rounded up to 4;
 // the padding holds k = q = 0, g = 1) and (beta, k . q) [T, heads, 2].  `delta_rule` then walks each
 // request's tokens in order: a block owns 16 (or 32) columns of one head's S, eight threads one

@@ -4,14 +4,14 @@
 // A step of a small model is a chain of such products, each over in less time than the tensor-core
 // kernel takes around its sums (barriers, tensor memory, copies through shared memory, a cluster's
 // two barriers).  Here a warp takes two rows of w (four for a gated unit, two features' gate and up
-// rows), a lane 16 bytes of a row at a time, straight into registers, and asks for its first rows before the kernel before is done, as the tensor-core
-// kernel does; then x, the sums, one barrier, and 16 features x tokens finish, a thread each.  A block
+// rows), a lane 16 bytes of a row at a time, straight into registers, and asks for its first rows before
+// the kernel before is done, as the tensor-core kernel does; then x, the sums, one barrier, and 16 features x tokens finish, a thread each.  A block
 // has 16 features: they share a slot of the sums of squares (eight slots to 128 features, as the
 // tensor-core kernel leaves them).  Long rows are split over two warps.  Chains over cold weights,
 // tensor cores / this, µs at one token: 1,152 x 896 4.95 / 2.30, 896 x 896 4.05 / 2.18, 896 x 4,864
-// 6.06 / 5.08, 2,048 x 8,192 9.98 / 8.62.  Gated units of one token and 17 MB of weights are level alone
-// (2 x 4,096 x 1,024 5.9 / 5.7, 2 x 4,864 x 896 6.4 / 7.3) and ahead in a step, between kernels of this
-// kind (24 layers of Qwen2.5-0.5B sizes 608 / 593); larger ones are behind.
+// 6.06 / 5.08, 2,048 x 8,192 9.98 / 8.62.  119 registers at 256 threads: two blocks an SM, one of the long
+// rows.  Beyond one round of them the last blocks run alone, and the tensor-core kernel is ahead; which
+// products come here, and both sides' figures, stand at `gemv_features` (ops.py).
 #pragma once
 #include "common.cuh"
 

@@ -355,15 +355,15 @@ latent_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__
   pdl_wait();
   extern __shared__ __align__(16) unsigned char lm_smem[];
   const int D = rank + rot, RS = D + 8;
-  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lm_smem);      // [32][RS]
-  __nv_bfloat16* k_s = q_s + ROWS * RS;                             // [2][32][RS]
-  float* s_s = reinterpret_cast<float*>(k_s + 2 * LM_KEYS * RS);       // [32][LM_SPAD]
-  int* row_pos = reinterpret_cast<int*>(s_s + ROWS * LM_SPAD);      // [32]
-  int* row_out = row_pos + ROWS;                                    // [32]: token * heads + head, -1 for none
-  float* corr_s = reinterpret_cast<float*>(row_out + ROWS);         // [32]
-  float* m_s = corr_s + ROWS;                                       // [32]
-  float* l_s = m_s + ROWS;                                          // [32]
-  __nv_bfloat16* p_s = reinterpret_cast<__nv_bfloat16*>(l_s + ROWS);  // [32][LM_PPAD]
+  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lm_smem);      // [ROWS][RS]
+  __nv_bfloat16* k_s = q_s + ROWS * RS;                                // [2][LM_KEYS][RS]
+  float* s_s = reinterpret_cast<float*>(k_s + 2 * LM_KEYS * RS);       // [ROWS][LM_SPAD]
+  int* row_pos = reinterpret_cast<int*>(s_s + ROWS * LM_SPAD);         // [ROWS]
+  int* row_out = row_pos + ROWS;                                       // [ROWS]: token * heads + head, -1 for none
+  float* corr_s = reinterpret_cast<float*>(row_out + ROWS);            // [ROWS]
+  float* m_s = corr_s + ROWS;                                          // [ROWS]
+  float* l_s = m_s + ROWS;                                             // [ROWS]
+  __nv_bfloat16* p_s = reinterpret_cast<__nv_bfloat16*>(l_s + ROWS);   // [ROWS][LM_PPAD]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rg = warp >> 2, cq = warp & 3, g = lane >> 2, t4 = lane & 3;
@@ -392,7 +392,7 @@ latent_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__
   // rows are handed out from 0 on: a group whose first row is none has none (steps of single
   // tokens with 16 heads or fewer fill one group only)
   const bool group_live = row_out[rg * 16] >= 0;
-  // a warp copies 4 query rows (index arithmetic once a row, not once a value)
+  // each of the ROWS / 4 warps copies four query rows (index arithmetic once a row, not once a value)
   for (int r = warp; r < ROWS; r += ROWS / 4) {
     __nv_bfloat16* dst = q_s + r * RS;
     if (row_out[r] >= 0) {

@@ -1468,7 +1468,7 @@ def _attention_with_options(ctx, qkv, k_pages, v_pages, block_table, num_heads, 
     for portions, the ``mma.sync`` kernel for the sizes that one does not take.  Other sizes
     that are multiples of 8, with a sink or a gate as the only options, run on the same two
     kernels compiled for sizes of their own (``sized_attention_supported``).  Everything
-    else, and float32, runs one warp a (token, head)."""
+    else, and float32, runs on the generic kernel (a block of eight warps a row, shared by rows of few keys)."""
     value_dim = options.value_dim or head_dim
     tiled = (ATTENTION_OPTIONS_TILED and qkv.dtype == torch.bfloat16 and head_dim in TILED_HEAD_DIMS
              and options.tiled)
