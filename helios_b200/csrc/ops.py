@@ -688,11 +688,13 @@ def gemv_features(tokens: int, K: int, gated: bool) -> int:
     alone, and the tensor-core kernel, whose K slices fill the SMs whatever the features, is ahead; more tokens
     cost the FMA pipes as many sums more and the tensor cores nothing, so that the rows get shorter.
     Tensor cores / FMA pipes, chains over cold weights, as a ratio:
-    one token, up to one round of blocks 1.03 to 2.05 (K 128 to 65,536), over it 0.70 to 1.08 (up to K =
-    2,048; 4,752 features 0.99 to 1.21, 6,144 0.82 to 1.05) and 0.74 to 0.97 above;
-    two, one round, K to 1,024 1.07 to 1.81; K 1,280 to 2,048 0.94 to 1.45; 2,304 to 4,096 with 1,024 features
-    1.03 to 1.24, with 2,048 0.95 to 1.07; longer 0.87 to 1.02;
-    three and four, K to 1,024, 1,024 features 0.97 to 1.40, 2,048 0.92 to 1.06; longer 0.61 to 0.99.
+    one token, up to one round of blocks 1.03 to 2.05 (K 128 to 65,536), to nine eighths of one 0.96 to 1.21 at K
+    of 256 to 1,024, 0.85 to 1.00 at 128 and 0.94 to 1.09 at 1,536 and 2,048; 6,144 features 0.81 to 1.07; K above
+    2,048, over one round 0.74 to 0.97;
+    two, one round, K to 1,024 1.07 to 1.81, over it 0.80 to 1.05; K 1,032 to 2,048 with 768 features 0.98 to 1.55,
+    with 1,024 to 4,736 0.94 to 1.04; 2,304 to 4,096 with 1,024 features 1.03 to 1.42, with 2,048 0.95 to 1.07;
+    longer 0.87 to 1.02 (16 features 1.19);
+    three and four, K to 1,024, 1,536 features 0.96 to 1.40, 2,048 0.92 to 1.06; longer 0.61 to 1.01.
     A gated unit is chosen in a step, between the products before and behind it (a layer's four products,
     us): one round 1.00 to 1.24 up to K = 4,864 (2 x 4,096 x 1,024 16.1 / 14.3, 2 x 2,048 x 2,048 20.5 / 18.7,
     2 x 2,048 x 4,864 40.8 / 41.0) and 0.95 to 0.97 above; up to seven quarters of a round 0.99 to 1.08 at K up
@@ -702,13 +704,11 @@ def gemv_features(tokens: int, K: int, gated: bool) -> int:
     one_round = 16 * sm_count() * (2 if K <= 2048 else 1)
     if gated:
         return (7 * one_round // 4 if K <= 1024 else one_round if K <= 4864 else 0) if tokens == 1 else 0
-    if tokens == 1 or (tokens == 2 and K <= 1024):
-        return one_round
-    if tokens == 2 and 2048 < K <= 4096:
-        return 1024
-    if tokens in (3, 4) and K <= 1024:
-        return 1280
-    return 0
+    if tokens == 1:
+        return 9 * one_round // 8 if 256 <= K <= 1024 else one_round
+    if tokens == 2:
+        return one_round if K <= 1024 else 768 if K <= 2048 else 1024 if K <= 4096 else 0
+    return 1536 if tokens in (3, 4) and K <= 1024 else 0
 
 
 #: tokens -> bytes of a weight matrix up to which plain products run on the FMA pipes; None: what

@@ -319,11 +319,12 @@ def test_settings_of_the_tensor_core_kernels_choose_them(settings, glu, monkeypa
 
 
 @pytest.mark.parametrize("T,N,K,gated,takes", [
-    (1, 16 * 296, 2048, False, True), (1, 16 * 296 + 1, 2048, False, False), (1, 16 * 148, 2056, False, True),
+    (1, 16 * 296, 2048, False, True), (1, 16 * 296 + 1, 2048, False, False), (1, 16 * 333, 1024, False, True),
+    (1, 16 * 333 + 1, 1024, False, False), (1, 16 * 296 + 1, 248, False, False), (1, 16 * 333, 256, False, True), (1, 16 * 148, 2056, False, True),
     (1, 16 * 148 + 1, 2056, False, False), (1, 32000, 512, False, False), (1, 16, 65536, False, True),
-    (2, 16 * 296, 1024, False, True), (2, 16 * 296 + 1, 1024, False, False), (2, 128, 1032, False, False),
+    (2, 16 * 296, 1024, False, True), (2, 16 * 296 + 1, 1024, False, False), (2, 768, 1032, False, True), (2, 769, 2048, False, False),
     (2, 1024, 2056, False, True), (2, 1025, 2056, False, False), (2, 1024, 4096, False, True), (2, 16, 4104, False, False),
-    (3, 1280, 1024, False, True), (4, 1281, 1024, False, False), (4, 16, 1032, False, False), (5, 16, 64, False, False),
+    (3, 1536, 1024, False, True), (4, 1537, 1024, False, False), (4, 16, 1032, False, False), (5, 16, 64, False, False),
     (1, 8288, 1024, True, True), (1, 8289, 1024, True, False), (1, 16 * 296, 1032, True, True), (1, 16 * 296 + 1, 1032, True, False),
     (1, 1024, 4864, True, True), (1, 1024, 4872, True, False), (1, 16 * 296, 2048, True, True), (2, 16, 64, True, False)])
 def test_which_products_the_fma_pipes_take(T, N, K, gated, takes, monkeypatch):
