@@ -62,7 +62,7 @@ _INCLUDES: Dict[str, List[str]] = {"gemm_bf16": ["gemv_bf16.cuh"],
                                    "latent_attention": ["attention_mma.cuh"],
                                    "linear_attention": ["linear_attention.cuh"],
                                    "gated_linear_attention": ["linear_attention.cuh"],
-                                   "delta_rule": ["causal_conv.cuh"],
+                                   "delta_rule": ["causal_conv.cuh", "delta_chunk.cuh"],
                                    "pooled_window": ["causal_conv.cuh"]}
 
 NVCC_FLAGS = [

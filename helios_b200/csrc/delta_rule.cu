@@ -14,7 +14,8 @@
 // Kernels: `causal_conv_silu` (short causal convolution over time per channel + silu, the
 // taps - 1 inputs before a step's first token taken from the request's slot),
 // `causal_conv_state` (leaves the last taps - 1 inputs in the slot; steps of single tokens do both in
-// `causal_conv_step`), `delta_prepare` and `delta_rule` (the recurrence; `delta_step` both for single tokens) and `gated_rmsnorm` (o / rms(o) * weight * sigmoid(gate) per head).
+// `causal_conv_step`), `delta_prepare` and `delta_rule` (the recurrence; `delta_step` both for single tokens;
+// `delta_chunk.cuh` for 16-bit activations and portions of many tokens) and `gated_rmsnorm` (o / rms(o) * weight * sigmoid(gate) per head).
 #include "common.cuh"
 #include "causal_conv.cuh"
 
@@ -846,6 +847,53 @@ HB_EXPORT int hb_delta_rule(float* o, float* scratch, const void* qkv, int qkv_l
 #undef HB_DR_LAUNCH_LONG
 #undef HB_DR_LAUNCH_COLS
 #undef HB_DR_LAUNCH
+  return hb_check_launch();
+}
+
+#include "delta_chunk.cuh"
+
+// The 32-bit words a (chunk, head) takes of `hb_delta_chunk`'s scratch; 0: this key size goes by `hb_delta_rule`
+HB_EXPORT int hb_delta_chunk_words(int dk) {
+  return dk <= 0 || dk > 128 ? 0 : dk <= 64 ? DeltaChunk<64>::WORDS : DeltaChunk<128>::WORDS;
+}
+
+// scratch: dc_chunks(n_tokens, n_seqs) * heads * hb_delta_chunk_words(dk) words, 16-byte aligned
+HB_EXPORT int hb_delta_chunk(float* o, uint32_t* scratch, const void* qkv, int qkv_ld, int q_off, int k_off,
+                             int v_off, const void* beta_raw, int beta_ld, const void* a_raw, int a_ld,
+                             const float* a_log, const float* dt_bias, float* state,
+                             long state_stride, const int* cu_tokens, const int* slots, int n_tokens,
+                             int n_seqs, int heads, int kv_heads, int dk, int dv, int sms, cudaStream_t stream) {
+  if (n_seqs <= 0 || n_tokens <= 0) return HB_OK;
+  if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || hb_delta_chunk_words(dk) == 0 || dv <= 0 ||
+      heads > 65535 || scratch == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15) || sms <= 0)
+    return HB_BAD_ARGUMENT;
+  const long ids = dc_chunks(n_tokens, n_seqs);
+  // one group of 16 columns a block where every block has an SM; else two, which share the staged chunks
+  const long alone = (long)n_seqs * heads * ((dv + DC_COLS - 1) / DC_COLS);
+  const int cols = alone <= sms ? DC_COLS : 2 * DC_COLS;
+  const long blocks = (long)n_seqs * heads * ((dv + cols - 1) / cols);
+  if (blocks > 0x7fffffffL || ids > 0x7fffffffL) return HB_BAD_ARGUMENT;
+  using TA = __nv_bfloat16;
+#define HB_DC_LAUNCH(DK, GROUPS, STAGES)                                                                      \
+  do {                                                                                                        \
+    hb_launch(delta_chunk_prepare_kernel<TA, DK>, dim3((unsigned)ids, heads), dim3(128), 0, stream, scratch,  \
+              (const TA*)qkv, qkv_ld, q_off, k_off, (const TA*)beta_raw, beta_ld, (const TA*)a_raw, a_ld,     \
+              a_log, dt_bias, cu_tokens, n_seqs, heads, kv_heads, dk);                                        \
+    auto kernel = delta_chunk_kernel<TA, DK, GROUPS, STAGES>;                                                 \
+    constexpr size_t smem = DeltaChunkSmem<DK, GROUPS, STAGES>::BYTES;                                        \
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                     \
+    kernel<<<(unsigned)blocks, GROUPS * DC_GROUP_THREADS, smem, stream>>>(                                    \
+        o, (const uint32_t*)scratch, (const TA*)qkv, qkv_ld, v_off, state, state_stride, cu_tokens, slots,    \
+        heads, dk, dv);                                                                                       \
+  } while (0)
+  if (dk <= 64) {
+    if (cols == DC_COLS) HB_DC_LAUNCH(64, 1, 4);
+    else HB_DC_LAUNCH(64, 2, 3);
+  } else {
+    if (cols == DC_COLS) HB_DC_LAUNCH(128, 1, 4);
+    else HB_DC_LAUNCH(128, 2, 3);
+  }
+#undef HB_DC_LAUNCH
   return hb_check_launch();
 }
 

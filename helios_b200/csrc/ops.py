@@ -2227,6 +2227,24 @@ def causal_conv_silu(ctx, x: torch.Tensor, channels: int, weight: torch.Tensor,
     return out
 
 
+#: Steps whose longest portion may have this many tokens, and that have DELTA_CHUNK_MEAN a request, walk the
+#: delta rule in chunks of 16 tokens (16-bit activations, keys of at most 128 values): keys of more than 64
+#: values | fewer, blocks of 16 columns that all have an SM of their own | fewer, more blocks.
+#: By tokens / by chunks, µs, 16 heads of 128 x 128: one request of 2,048 tokens 448 / 184, of 333 77 / 37, of 64
+#: 20 / 16; 64 tokens of 32 requests 189 / 171, 32 of 16 53 / 52, 16 of 64 114 / 131; 1,000 beside 24 of one 272 /
+#: 143, 300 90 / 66.  8 heads of 64 x 64: 2,048 297 / 119, 700 of three 110 / 54, 64 13.9 / 12.2, 64 of 32 41 / 44,
+#: 1,000 beside 24 of one 190 / 95.  16 of 24 x 24: 200 29 / 20, 64 of 24 30 / 40.
+DELTA_CHUNK_TOKENS = (64, 128, 512)
+DELTA_CHUNK_MEAN = 24
+
+
+def delta_rule_by_chunks(ctx, dtype: torch.dtype, tokens: int, heads: int, dk: int, dv: int) -> bool:
+    longest = min(getattr(ctx, "max_tokens_per_seq", 0) or tokens, tokens)
+    alone = ctx.num_seqs * heads * -(-dv // 16) <= sm_count()
+    return dtype == torch.bfloat16 and dk <= 128 and tokens >= DELTA_CHUNK_MEAN * ctx.num_seqs \
+        and longest >= DELTA_CHUNK_TOKENS[0 if dk > 64 else 1 if alone else 2]
+
+
 def delta_rule(ctx, qkv: torch.Tensor, offsets, beta_raw: torch.Tensor, a_raw: torch.Tensor,
                a_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor, heads: int,
                kv_heads: int, dk: int, dv: int) -> torch.Tensor:
@@ -2250,6 +2268,19 @@ def delta_rule(ctx, qkv: torch.Tensor, offsets, beta_raw: torch.Tensor, a_raw: t
         raise KernelError("delta_rule: sizes do not fit (key size at most 256)")
     T = qkv.shape[0]
     o = torch.empty((T, heads * dv), dtype=torch.float32, device=qkv.device)
+    if delta_rule_by_chunks(ctx, qkv.dtype, T, heads, dk, dv):
+        lib = load_library("delta_rule")
+        scratch = torch.empty((((T - 1) // 16 + ctx.num_seqs) * heads * lib.hb_delta_chunk_words(dk),),
+                              dtype=torch.float32, device=qkv.device)
+        f = _fn("delta_rule", "hb_delta_chunk",
+                [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
+                 c_void_p, c_void_p, _LONG, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                 c_void_p])
+        _run(f(_p(o), _p(scratch), _p(qkv), qkv.shape[1], offsets[0], offsets[1], offsets[2], _p(beta_raw),
+               beta_raw.stride(0), _p(a_raw), a_raw.stride(0), _p(a_log), _p(dt_bias), _p(state),
+               state.stride(0), _p(ctx.cu_tokens), _p(ctx.slots), T, ctx.num_seqs, heads, kv_heads, dk, dv,
+               sm_count(qkv.device), _stream()), "delta_chunk")
+        return o
     # unit-norm k and q, decays and write strengths of every (token, head), float32
     scratch = torch.empty((T * heads * (3 * (-(-dk // 4) * 4) + 2),), dtype=torch.float32, device=qkv.device)
     f = _fn("delta_rule", "hb_delta_rule",

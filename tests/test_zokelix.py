@@ -756,6 +756,67 @@ def test_delta_rule_a_token_a_step_is_the_walk_over_all_tokens_bit_for_bit(dk, d
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[1], [16], [17], [15, 40, 1, 33], [20] * 60], ids=lambda x: f"{len(x)}x{x[0]}")
+@pytest.mark.parametrize("dk,dv", [(4, 4), (64, 16), (65, 17), (100, 36), (128, 128)])
+def test_delta_rule_by_chunks_of_tokens_is_the_plain_scan(dk, dv, lens, monkeypatch):
+    """bfloat16: whole, short and ragged last chunks, blocks of one and of two column groups, slots in any
+    order, a slot that nobody owns; a token that holds NaN reaches neither the tokens before it nor
+    other requests."""
+    from types import SimpleNamespace
+    from helios_b200.csrc import ops
+
+    monkeypatch.setattr(ops, "DELTA_CHUNK_TOKENS", (0, 0, 0))
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MEAN", 0)
+    dev, heads, kv_heads, S, T = "cuda", 4, 2, len(lens), sum(lens)
+    g = torch.Generator().manual_seed(dk + dv + T)
+    qkv = torch.randn(T, 2 * kv_heads * dk + heads * dv, generator=g).bfloat16()
+    beta = (torch.randn(T, heads, generator=g) + 1).bfloat16()
+    a = (torch.randn(T, heads * dk, generator=g) - 2).bfloat16()
+    a_log, dt_bias = torch.randn(heads, generator=g) * 0.3, torch.randn(heads * dk, generator=g) * 0.3
+    before = torch.randn(S + 1, heads * dk * dv, generator=g) * 0.3
+    slots = list(range(S, 0, -1))
+    ctx = SimpleNamespace(cu_tokens=torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).int().to(dev),
+                          slots=torch.tensor(slots, dtype=torch.int32, device=dev), num_seqs=S)
+
+    def run(rows):
+        state = before.to(dev)
+        o = ops.delta_rule(ctx, rows.to(dev), (0, kv_heads * dk, 2 * kv_heads * dk), beta.to(dev), a.to(dev),
+                           a_log.to(dev), dt_bias.to(dev), state, heads, kv_heads, dk, dv)
+        return o.cpu(), state.cpu()
+
+    got, state = run(qkv)
+    assert torch.equal(state[0], before[0])
+    x, at = qkv.double(), 0
+    for s in range(S if S <= 4 else 2):
+        r = slice(at, at + lens[s])
+        for h in range(heads):
+            kh = h // (heads // kv_heads)
+            q, k = x[r, kh * dk:(kh + 1) * dk], x[r, (kv_heads + kh) * dk:(kv_heads + kh + 1) * dk]
+            q = q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * dk ** -0.5
+            k = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+            v = x[r, 2 * kv_heads * dk + h * dv:2 * kv_heads * dk + (h + 1) * dv]
+            gd = torch.exp(-torch.exp(a_log[h].double()) * torch.nn.functional.softplus(
+                a[r, h * dk:(h + 1) * dk].double() + dt_bias[h * dk:(h + 1) * dk].double()))
+            b = torch.sigmoid(beta[r, h].double())
+            want = before[slots[s]].double().view(heads, dk, dv)[h].clone()
+            for t in range(lens[s]):
+                want = gd[t][:, None] * want
+                want = want + k[t][:, None] * (b[t] * (v[t] - want.T @ k[t]))[None, :]
+                o = want.T @ q[t]
+                # 32-bit sums of dk values of about one: some dk / 2 roundings of 6e-8, most averaged out
+                assert (got[at + t, h * dv:(h + 1) * dv].double() - o).abs().max() < 1e-5
+            assert (state[slots[s]].double().view(heads, dk, dv)[h] - want).abs().max() < 1e-5
+        at += lens[s]
+    if lens[0] < 2:
+        return
+    bad = qkv.clone()
+    bad[lens[0] - 1] = float("nan")
+    o2, state2 = run(bad)
+    assert torch.equal(o2[:lens[0] - 1], got[:lens[0] - 1]) and torch.equal(o2[lens[0]:], got[lens[0]:])
+    assert o2[lens[0] - 1].isnan().all() and torch.equal(state2[:S], state[:S])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("y_dtype", DTYPES)
 @pytest.mark.parametrize("H", [4, 37, 1020, 1024, 1028, 2052, 4100, 8192, 8196])
 def test_norm_on_an_output_at_the_widths_its_rows_are_kept_at(H, y_dtype):
