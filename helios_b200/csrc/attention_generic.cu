@@ -74,7 +74,11 @@ __device__ __forceinline__ float4 load_four(const T* row, int d, int n) {
 // of 30 tokens 347 / 67, 2,048 tokens with a window of 16 356 / 69 and of 128 383 / 236, 600 decode rows of 30
 // keys 116 / 25; but 600 of 250 keys 223 / 246 (half a microsecond a block until the position is there
 // and the warps are dealt), and one row of 30 5.6 / 6.1.  So it is for launches of many rows that may be short.
-template <typename T, int NJ, bool VEC, bool SHARE>
+// AHEAD: for launches of at most a block an SM.  All keys and values of a run are asked for at once, before its
+// scores: one trip to memory a run instead of four, for registers that leave an SM one block.  14 heads of 64 on 2 KV
+// heads, float32, µs: 3 rows of 20 keys 4.6 / 3.7, of 313 7.8 / 6.2, of 4,096 49 / 36; 10 of 1,000 14.9 / 11.0.  Heads
+// of at most 32 values have all of it under way as it is (5.56 / 5.60), and of 128 it does not fit the registers.
+template <typename T, int NJ, bool VEC, bool SHARE, bool AHEAD>
 __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
     T* __restrict__ out, const T* __restrict__ q, int q_stride,
     const T* __restrict__ k_pages, const T* __restrict__ v_pages,
@@ -88,7 +92,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
   pdl_wait();
   __shared__ float part_acc[ATTN_WARPS][32 * NJ];
   __shared__ float part_m[ATTN_WARPS], part_l[ATTN_WARPS];
-  constexpr int KEYS = NJ <= 4 ? 8 / NJ : 1;         // keys a group has in flight: eight loads a lane
+  constexpr int KEYS = AHEAD ? 8 : NJ <= 4 ? 8 / NJ : 1;     // keys a group has in flight: eight loads a lane
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = lane >> 3, gl = lane & 7;
   const int t = blockIdx.x / head_blocks;
@@ -146,6 +150,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
       size_t place = 0;
       if (valid) place = ((size_t)table[key / page_size] * nkv + kvh) * page_size + key % page_size;
       float score = -INFINITY;
+      float4 values[AHEAD ? 8 : 1][NJ];
 #pragma unroll 1
       for (int i0 = 0; i0 < 8; i0 += KEYS) {           // the group's keys 8 group + i
         float4 kv[KEYS][NJ];
@@ -155,6 +160,15 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
           const int n = base + 8 * group + i0 + u <= last ? hd : 0;
 #pragma unroll
           for (int j = 0; j < NJ; ++j) kv[u][j] = load_four<T, VEC>(kp + at * hd, 4 * (8 * j + gl), n);
+        }
+        if constexpr (AHEAD) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const size_t at = __shfl_sync(0xffffffffu, (unsigned long long)place, 8 * group + u);
+            const int n = base + 8 * group + u <= last ? vd : 0;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) values[u][j] = load_four<T, VEC>(vp + at * vd, 4 * (8 * j + gl), n);
+          }
         }
 #pragma unroll
         for (int u = 0; u < KEYS; ++u) {
@@ -196,11 +210,16 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_generic_kernel(
         float pj[KEYS];
 #pragma unroll
         for (int u = 0; u < KEYS; ++u) {
-          const size_t at = __shfl_sync(0xffffffffu, (unsigned long long)place, 8 * group + i0 + u);
           pj[u] = __shfl_sync(0xffffffffu, p, 8 * group + i0 + u);
-          const int n = base + 8 * group + i0 + u <= last ? vd : 0;
+          if constexpr (AHEAD) {
 #pragma unroll
-          for (int j = 0; j < NJ; ++j) kv[u][j] = load_four<T, VEC>(vp + at * vd, 4 * (8 * j + gl), n);
+            for (int j = 0; j < NJ; ++j) kv[u][j] = values[u][j];
+          } else {
+            const size_t at = __shfl_sync(0xffffffffu, (unsigned long long)place, 8 * group + i0 + u);
+            const int n = base + 8 * group + i0 + u <= last ? vd : 0;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) kv[u][j] = load_four<T, VEC>(vp + at * vd, 4 * (8 * j + gl), n);
+          }
         }
 #pragma unroll
         for (int u = 0; u < KEYS; ++u)
@@ -286,8 +305,8 @@ HB_EXPORT int hb_attention_generic(void* out, const void* q, int q_stride, const
   const bool share = runs <= 4 ? rows > 2L * sms : rows > 8L * sms && (window <= 0 || window >= keys_of_table);
   const int head_step = !share ? 1 : runs <= 1 ? 8 : runs <= 2 ? 4 : runs <= 4 ? 2 : 1;
   const int head_blocks = (nh + head_step - 1) / head_step;
-#define HB_GENERIC_SHARE(NJ, VEC, SHARE)                                                                       \
-    hb_launch(attention_generic_kernel<TA, NJ, VEC, SHARE>, dim3((unsigned)(T * head_blocks)),                 \
+#define HB_GENERIC_SHARE(NJ, VEC, SHARE, AHEAD)                                                                       \
+    hb_launch(attention_generic_kernel<TA, NJ, VEC, SHARE, AHEAD>, dim3((unsigned)(T * head_blocks)),                 \
         dim3(ATTN_WARPS * 32), 0, stream,                                                                      \
         (TA*)out, (const TA*)q, q_stride, (const TA*)k_pages, (const TA*)v_pages, block_table,                 \
         bt_stride, seq_of_token, positions, head_blocks, head_step, nh, nkv, hd, vd, page_size, window, scale, \
@@ -297,8 +316,10 @@ HB_EXPORT int hb_attention_generic(void* out, const void* q, int q_stride, const
         out_stride, factor)
 #define HB_GENERIC_LAUNCH(NJ, VEC)                                                                             \
     do {                                                                                                       \
-      if (share) HB_GENERIC_SHARE(NJ, VEC, true);                                                              \
-      else HB_GENERIC_SHARE(NJ, VEC, false);                                                                   \
+      constexpr bool MAY = VEC && NJ == 2;                                                                     \
+      if (share) HB_GENERIC_SHARE(NJ, VEC, true, false);                                                       \
+      else if (MAY && rows <= sms) HB_GENERIC_SHARE(NJ, VEC, false, MAY);                                      \
+      else HB_GENERIC_SHARE(NJ, VEC, false, false);                                                            \
     } while (0)
   HB_DISPATCH_DTYPE(act_dt, TA,
     const uintptr_t addresses = reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages) |

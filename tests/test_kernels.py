@@ -773,3 +773,26 @@ def test_generic_attention_of_many_short_rows_is_each_row_alone_bit_for_bit(nh, 
         assert torch.equal(got, torch.cat([call(a, min(T, a + few)) for a in range(0, T, few)]))
         if options is plain and means is None:
             torch.testing.assert_close(got.cpu().double(), dense_attention(case, scale, window), **tol(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd", [(14, 2, 64), (5, 5, 36), (2, 1, 48)])
+def test_generic_attention_of_few_rows_with_all_loads_ahead_is_the_same_bit_for_bit(nh, nkv, hd, dtype):
+    """At most a block an SM: keys and values of a run are asked for together.  Against the same rows in
+    larger launches, at the edges of runs, with windows, kept first tokens, means and a gate."""
+    o = ops()
+    lens = (1, 2, 31, 32, 33, 64, 65, 255, 256, 257, 300, 600)
+    seqs = [(n - 1, 1) for n in lens] * 4 + [(0, 150)]
+    page, scale = 8, 1.0 / math.sqrt(hd)
+    case = make_paged_case(seqs, nh, nkv, hd, page, dtype, DEV, seed=hd)
+    T = case.qkv.shape[0]
+    g = torch.Generator().manual_seed(hd)
+    gate = torch.randn(T, nh * hd, generator=g).to(DEV, dtype)
+    pooled = (case.k_pages.nan_to_num(), case.v_pages.nan_to_num(), torch.zeros((len(seqs), 6), dtype=torch.int32, device=DEV), 7)
+    few = o.sm_count() // nh
+    assert few * nh <= o.sm_count() < (T - few) * nh
+    for window, keep, means in ((None, 0, None), (1, 0, None), (33, 0, None), (40, 3, None), (60, 0, pooled), (300, 0, None)):
+        call = lambda a, b: o.attention_generic(
+            case.qkv[a:b], case.k_pages, case.v_pages, case.table, case.seq_of_token[a:b], case.positions[a:b], nh, nkv, hd, page,
+            window, scale, o.AttentionOptions(gate=gate[a:b], gate_wide=True, keep_first=keep) if means is None else None, means)
+        assert torch.equal(call(0, T), torch.cat([call(a, min(T, a + few)) for a in range(0, T, few)]))
