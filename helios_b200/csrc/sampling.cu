@@ -188,6 +188,9 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, int V, in
 // one row 81 / 25; top-p 0.95 of 64 rows N(0, 1), 60,000 tokens kept, 452 / 149.  Eight rows, search of
 // whole keys alone / list tried in vain, then that search / this: top-k 2,000 and top-p 0.9 of N(0, 4)
 // 111 / 141 / 101; top-k 2,000 of whole numbers 48 / 80 / 50; top-k 50 of equal values 39 / 71 / 50.
+// Bound by instructions and barriers: 16 warps a block, three blocks an SM.  So rows come in 16-byte pieces and the argmax
+// with them, fifteen sums of a warp take 16 exchanges, and a value is compared with a level only where it lies
+// above the next lower one: 64 rows N(0, 4) of mixed options 50.8 -> 45.7.
 constexpr int SC_THREADS = 512;
 constexpr int SC_CLUSTER = 8;
 constexpr int SC_MOST = 40;          // elements a thread keeps: rows of up to 8 * 512 * 40 values
@@ -286,12 +289,22 @@ __device__ uint32_t sc_sorted_threshold(uint32_t* list, int count, int k, float 
 __device__ __forceinline__ void sc_sum15(float (&acc)[15], float (*warp_part)[15], float (*block_part)[16],
                                          float* total, int slot) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the trees of `warp_sum`, but of two partners each goes on with half of the sums: 16 exchanges, not 75
+  float v[16];
 #pragma unroll
-  for (int j = 0; j < 15; ++j) acc[j] = warp_sum(acc[j]);
-  if (lane == 0) {
+  for (int j = 0; j < 15; ++j) v[j] = acc[j];
+  v[15] = 0.f;
 #pragma unroll
-    for (int j = 0; j < 15; ++j) warp_part[warp][j] = acc[j];
+  for (int n = 8, o = 16; n > 0; n /= 2, o /= 2) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      const float give = upper ? v[j] : v[j + n], keep = upper ? v[j + n] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
   }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  if ((lane & 1) == 0 && lane < 30) warp_part[warp][lane >> 1] = v[0];     // (bits 16, 8, 4, 2 of the lane: 8, 4, 2, 1 of j)
   __syncthreads();
   if (threadIdx.x < 15) {
     float t = 0.f;
@@ -341,23 +354,34 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
   // of a warp's threads then lie in different banks); 0 where the row has ended (no float
   // has key 0 but one NaN).
   extern __shared__ uint32_t keys[];
+  // ... and the argmax, lowest index among equals
+  uint32_t bk = 0;
+  int bi = 0x7fffffff;
   {
     const int block_first = (int)rank * SC_THREADS * EPT;
-#pragma unroll 8
-    for (int c = tid; c < SC_THREADS * EPT; c += SC_THREADS) {
+    auto take = [&](int c, float v) {                // (a thread's c grow)
       const int owner = c / EPT, i = c - owner * EPT;
-      keys[owner * (EPT + 1) + i] = (block_first + c < V) ? float_key(l[block_first + c]) : 0u;
+      const uint32_t k = block_first + c < V ? float_key(v) : 0u;
+      keys[owner * (EPT + 1) + i] = k;
+      if (k > bk) { bk = k; bi = block_first + c; }
+    };
+    if (((reinterpret_cast<uintptr_t>(logits) & 15) | (uintptr_t)(ld & 3) | (uintptr_t)(V & 3)) == 0) {
+#pragma unroll
+      for (int c = 4 * tid; c < SC_THREADS * EPT; c += 4 * SC_THREADS) {
+        const float4 v = block_first + c < V ? *reinterpret_cast<const float4*>(l + block_first + c)
+                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        take(c, v.x);
+        take(c + 1, v.y);
+        take(c + 2, v.z);
+        take(c + 3, v.w);
+      }
+    } else {
+#pragma unroll 8
+      for (int c = tid; c < SC_THREADS * EPT; c += SC_THREADS) take(c, block_first + c < V ? l[block_first + c] : 0.f);
     }
     __syncthreads();
   }
   const uint32_t* key = keys + tid * (EPT + 1);
-
-  // ---- argmax, lowest index among equals
-  uint32_t bk = 0;
-  int bi = 0x7fffffff;
-#pragma unroll
-  for (int i = 0; i < EPT; ++i)
-    if (key[i] > bk) { bk = key[i]; bi = first + i; }
   auto better = [](uint32_t k1, int i1, uint32_t k2, int i2) { return k1 > k2 || (k1 == k2 && i1 < i2); };
   for (int o = 16; o > 0; o >>= 1) {
     const uint32_t ok = __shfl_xor_sync(0xffffffffu, bk, o);
@@ -410,14 +434,17 @@ sample_cluster_kernel(int* __restrict__ out, const float* __restrict__ logits, i
       const uint32_t c = key[i];
       float e = 0.f;
       if (k_on == 0 && c >= 1u) acc[SC_LEVELS] += e = expf(key_float(c) * inv_t - mx_t);
-      if (c >= level[SC_LEVELS - 1]) {
+      // (the levels lie one above the other, and few warps hold a value above the lower ones)
+      bool in = true;
 #pragma unroll
-        for (int j = 0; j < SC_LEVELS; ++j)
-          if (c >= level[j]) {
+      for (int j = SC_LEVELS - 1; j >= 0; --j)
+        if (in) {
+          in = c >= level[j];
+          if (in) {
             acc[j] += e;
             acc[SC_LEVELS + 1 + j] += 1.f;
           }
-      }
+        }
     }
     sc_sum15(acc, warp_part, block_part, total, slot);
     // lo: the highest level that satisfies the row (holds k values, or more than p of the mass);
