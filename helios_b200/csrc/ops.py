@@ -1021,12 +1021,29 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
                     ("seed", seed), ("offset", offset)):
         if t.numel() != R:
             raise KernelError(f"{name} has {t.numel()} entries for {R} rows")
+    return _sample(logits, _p(temperature), _p(top_k), _p(top_p), _p(seed), _p(offset), kind)
+
+
+def sample_packed(logits: torch.Tensor, options: torch.Tensor, kind: Optional[str] = None) -> torch.Tensor:
+    """``sample`` with the options of its R rows one behind the other in int32 ``options`` [7 R]: seeds
+    and offsets (int64), temperatures, top-p (float32), top-k."""
+    _check(logits, "logits", torch.float32, 2)
+    _check(options, "options", torch.int32, 1)
+    R = logits.shape[0]
+    if options.numel() != 7 * R or options.data_ptr() % 8:
+        raise KernelError(f"options has {options.numel()} words for {R} rows, or its int64 are not aligned")
+    at = options.data_ptr()
+    return _sample(logits, at + 16 * R, at + 24 * R, at + 20 * R, at, at + 8 * R, kind)
+
+
+def _sample(logits, temperature: int, top_k: int, top_p: int, seed: int, offset: int, kind) -> torch.Tensor:
+    R, V = logits.shape
     out = torch.empty((R,), dtype=torch.int32, device=logits.device)
     f = _fn("sampling", "hb_sample",
             [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
              c_void_p, c_int, c_void_p])
-    _run(f(_p(out), _p(logits), R, V, V, _p(temperature), _p(top_k), _p(top_p), _p(seed),
-           _p(offset), _SAMPLE_KINDS[kind], _stream()), "sample")
+    _run(f(_p(out), _p(logits), R, V, V, temperature, top_k, top_p, seed, offset, _SAMPLE_KINDS[kind], _stream()),
+         "sample")
     return out
 
 

@@ -13,8 +13,12 @@ from ..csrc import ops
 
 class _Staging:
     def __init__(self, words: int) -> None:
-        self.host = torch.empty(words, dtype=torch.int32, pin_memory=True)
         self.event = torch.cuda.Event()
+        self.grow(words)
+
+    def grow(self, words: int) -> None:
+        self.host = torch.empty(words, dtype=torch.int32, pin_memory=True)
+        self.words = self.host.numpy()
 
 
 class Sampler:
@@ -35,7 +39,7 @@ class Sampler:
         self._next = (self._next + 1) % self.RING
         st.event.synchronize()                 # its last copy has left the host
         if st.host.numel() < words:
-            st.host = torch.empty(words, dtype=torch.int32, pin_memory=True)
+            st.grow(words)
         return st
 
     def sample(self, logits: torch.Tensor, params: Sequence, seeds: Sequence[int],
@@ -50,26 +54,26 @@ class Sampler:
         R = logits.shape[0]
         if not (len(params) == len(seeds) == len(offsets) == R):
             raise ValueError("one set of sampling options per logits row is required")
-        # int32 words: seeds (int64) | offsets (int64) | temperature | top_p | top_k
+        # (int32 words, laid out as ``ops.sample_packed`` takes them)
         st = self._staging(7 * R)
-        words = st.host.numpy()[:7 * R]
+        words = st.words[:7 * R]
         i64 = words[:4 * R].view(np.int64)
         f32 = words[4 * R:6 * R].view(np.float32)
         top_k = words[6 * R:]
         # whole arrays at once: with hundreds of rows a loop of scalar stores costs a millisecond
         mask = 2**64 - 1
-        i64[:R] = np.fromiter((s & mask for s in seeds), dtype=np.uint64, count=R).view(np.int64)
+        i64[:R] = np.array([s & mask for s in seeds], dtype=np.uint64).view(np.int64)
         i64[R:] = offsets
-        f32[:R] = [p.temperature for p in params]
-        f32[R:] = [p.top_p for p in params]
+        temperature, top_p = f32[:R], f32[R:]
+        temperature[:] = [p.temperature for p in params]
+        top_p[:] = [p.top_p for p in params]
         top_k[:] = [p.top_k for p in params]
-        if any(p.temperature > 0 and (p.top_k > 0 or p.top_p < 1.0) for p in params):
-            kind = "narrow"
+        draws = temperature > 0
+        if not draws.any():
+            kind = "greedy"
         else:
-            kind = "draw" if any(p.temperature > 0 for p in params) else "greedy"
+            kind = "narrow" if (draws & ((top_k > 0) | (top_p < 1.0))).any() else "draw"
         dev = torch.empty(7 * R, dtype=torch.int32, device=logits.device)
         dev.copy_(st.host[:7 * R], non_blocking=True)
         st.event.record()
-        d64 = dev[:4 * R].view(torch.int64)
-        d32 = dev[4 * R:6 * R].view(torch.float32)
-        return ops.sample(logits, d32[:R], dev[6 * R:], d32[R:], d64[:R], d64[R:], kind=kind)
+        return ops.sample_packed(logits, dev, kind)

@@ -796,3 +796,26 @@ def test_generic_attention_of_few_rows_with_all_loads_ahead_is_the_same_bit_for_
             case.qkv[a:b], case.k_pages, case.v_pages, case.table, case.seq_of_token[a:b], case.positions[a:b], nh, nkv, hd, page,
             window, scale, o.AttentionOptions(gate=gate[a:b], gate_wide=True, keep_first=keep) if means is None else None, means)
         assert torch.equal(call(0, T), torch.cat([call(a, min(T, a + few)) for a in range(0, T, few)]))
+
+
+@pytest.mark.parametrize("V", [4096, 4097, 32002, 128256, 128255])
+def test_sampling_with_packed_options_and_rows_that_are_and_are_not_whole_pieces(V):
+    """Options in one tensor are the options in five, and the cluster kernel's ids (rows in 16-byte pieces
+    where their length allows it) those of the kernel with one block a row."""
+    o = ops()
+    g = torch.Generator().manual_seed(V)
+    kinds = [(0.0, 0, 1.0), (0.8, 50, 0.9), (1.0, 0, 1.0), (0.7, 0, 0.95), (1.1, 20, 1.0)]
+    R = 10
+    logits = (torch.randn(R, V, generator=g) * 4).to(DEV)
+    t = torch.tensor([kinds[i % 5][0] for i in range(R)])
+    k = torch.tensor([kinds[i % 5][1] for i in range(R)], dtype=torch.int32)
+    p = torch.tensor([kinds[i % 5][2] for i in range(R)])
+    seed, offset = torch.randint(-2 ** 62, 2 ** 62, (R,), generator=g), torch.arange(R) * 7
+    dev = [x.to(DEV) for x in (t, k, p, seed, offset)]
+    got = o.sample(logits, *dev, kind="narrow")
+    packed = torch.cat([seed.view(torch.int32), offset.view(torch.int32), t.view(torch.int32), p.view(torch.int32), k]).to(DEV)
+    assert torch.equal(o.sample_packed(logits, packed, "narrow"), got)
+    # (a draw that falls on a rounding of the mass may be the neighbour's: none of these does)
+    assert torch.equal(o.sample(logits, *dev, kind="one_block"), got)
+    with pytest.raises(o.KernelError):
+        o.sample_packed(logits, packed[:-1], "narrow")
