@@ -36,7 +36,7 @@ enum { EPI_STORE = 0, EPI_GLU = 1, EPI_GELU = 2 };     // plain | silu(g) u | ge
 
 struct GemmArgs {
   void* out;            // [T, ldo] bfloat16 or float32
-  const float* bias;    // [N] or null
+  const float* bias;    // [N], of a gated unit [2 N] (gate's, then up's; two-SM kernel only), or null
   float* scratch;       // partial sums when the K range is split
   int* tickets;         // one per output tile, zero between launches
   int* error;           // set non-zero when a wait ran out
@@ -726,6 +726,15 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
           tmem_ld16(taddr + c, g);
           tmem_ld16(taddr + 128 + c, u);
           if (t < args.T) {       // rows beyond the last token hold zeros: 0 / x is the division's slow path
+            if (args.bias) {      // gate's, then up's
+              const int n = tile_n * RESULT_COLS + c;
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (n + i < args.N) {
+                  g[i] += args.bias[n + i];
+                  u[i] += args.bias[args.glu_offset + n + i];
+                }
+            }
 #pragma unroll
             for (int i = 0; i < 16; ++i) val[i] = glu_value<EPI>(g[i], u[i]);
           }
@@ -734,7 +743,7 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
         const int n0 = tile_n * RESULT_COLS + c;
         if (t < args.T) {
-          if (args.bias) {
+          if (!GATED && args.bias) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) if (n0 + i < args.N) val[i] += args.bias[n0 + i];
           }
@@ -967,6 +976,7 @@ static int gemm_bf16_call(void* out, const void* x, const void* w, const float* 
   if (k_splits > 1 && !clustered && (scratch == nullptr || tickets == nullptr)) return HB_BAD_ARGUMENT;
   if (k_splits > (K + BK - 1) / BK) return HB_BAD_ARGUMENT;
   if (error == nullptr || glu < 0 || glu > 2) return HB_BAD_ARGUMENT;
+  if (glu && bias && !(swap_bn == 0 && k_splits == 1 && cluster == 2)) return HB_BAD_ARGUMENT;
   if (residual != nullptr || sumsq_in != nullptr) {
     // the epilogues of few-token steps: swapped orientation, one token tile
     if (swap_bn == 0 || T > swap_bn) return HB_BAD_ARGUMENT;

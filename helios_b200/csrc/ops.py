@@ -731,13 +731,14 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
                 plan=None, cluster: Optional[bool] = None, two_sm: Optional[bool] = None,
                 sumsq: Optional[torch.Tensor] = None, eps: float = 0.0,
                 residual: Optional[torch.Tensor] = None, norm_weight: Optional[torch.Tensor] = None,
-                norm_out: Optional[tuple] = None):
+                norm_out: Optional[tuple] = None, glu_bias: Optional[torch.Tensor] = None):
     """y = x W^T (+ bias); bfloat16 operands, float32 accumulate.  On tcgen05 tensor cores, or, for
     one to four tokens and a small weight, on the FMA pipes (``gemv_bf16.cuh``); ``plan``, ``cluster``
     and ``two_sm`` are settings of the tensor-core kernels and choose those.
 
     With ``glu`` (True or "silu", or "gelu_tanh") the weight is [gate rows; up rows] ([2 I, K]) and
-    the result is act(x gate^T) * (x up^T), [T, I].  ``out_dtype`` bfloat16 or float32.  K must be a
+    the result is act(x gate^T) * (x up^T), [T, I], with ``glu_bias`` (float32 [2 I]) added to the two
+    products (more than 128 tokens, two-SM kernel).  ``out_dtype`` bfloat16 or float32.  K must be a
     multiple of 8 (TMA rows are 16-byte aligned); any T and N.
 
     Up to DEFERRED_NORM_MOST tokens there are two more epilogues.  ``sumsq``
@@ -767,6 +768,13 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         _check(bias, "bias", torch.float32, 1)
         if bias.numel() != N:
             raise KernelError(f"bias has {bias.numel()} entries for {N} outputs")
+    if glu_bias is not None:
+        if not glu or T <= 128 or plan is not None or not (GEMM_TWO_SM if two_sm is None else two_sm):
+            raise KernelError("glu_bias goes with a gated unit of more than 128 tokens on the two-SM kernel")
+        _check(glu_bias, "glu_bias", torch.float32, 1)
+        if glu_bias.numel() != rows:
+            raise KernelError(f"glu_bias has {glu_bias.numel()} entries for {rows} rows")
+        bias = glu_bias
     if out_dtype not in (torch.bfloat16, torch.float32):
         raise KernelError(f"out_dtype {out_dtype} is not supported")
     few = sumsq is not None or residual is not None
@@ -962,6 +970,10 @@ def _library_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.
     return torch.nn.functional.linear(rows, weight, bias)[:T]
 
 
+def _library_product(tokens: int, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> bool:
+    return ((bias is None or GEMM_LIBRARY_WITH_BIAS) and _library_range(tokens)) or _small_weight_library(tokens, weight)
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y = x W^T + b.  float32: this package's FMA kernels.  bfloat16: ``linear_bf16`` (tcgen05, or the
     FMA pipes for few tokens and a small weight), or the library for plain products in the token ranges of GEMM_LIBRARY_TOKEN_RANGE and
@@ -972,9 +984,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     _check(x, "x", torch.bfloat16, 2)
     _check(weight, "weight", torch.bfloat16, 2)
     T = x.shape[0]
-    to_library = ((bias is None or GEMM_LIBRARY_WITH_BIAS) and _library_range(T)) \
-        or _small_weight_library(T, weight)
-    if tc_gemm_supported(x, weight) and not to_library:
+    if tc_gemm_supported(x, weight) and not _library_product(T, weight, bias):
         return linear_bf16(x, weight, bias)
     return _library_linear(x, weight, None if bias is None else _bias_bf16(bias))
 
@@ -984,19 +994,25 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor) -> torch.Tensor:
     return linear_glu(x, w_gate_up, "silu")
 
 
-def linear_glu(x: torch.Tensor, w_gate_up: torch.Tensor, kind: str) -> torch.Tensor:
+def linear_glu(x: torch.Tensor, w_gate_up: torch.Tensor, kind: str, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """act(x gate^T) * (x up^T) for ``w_gate_up`` = [gate rows; up rows], ``kind`` "silu" or
-    "gelu_tanh"; fused into the product's epilogue in bfloat16, two kernels otherwise."""
+    "gelu_tanh", ``bias`` (float32, [gate; up]) on the two products; fused into the product's epilogue
+    in bfloat16 (with a bias, where the plain product would run on the two-SM kernel as well), two
+    kernels otherwise."""
     def gate(rows):
         return silu_mul(rows) if kind == "silu" else glu_act(rows, kind)
 
     if x.dtype == torch.bfloat16 and tc_gemm_supported(x, w_gate_up):
         T = x.shape[0]
-        if _small_weight_library(T, w_gate_up, glu=True) or \
+        if bias is not None:
+            if T > 128 and GEMM_TWO_SM and not _library_product(T, w_gate_up, bias):
+                return linear_bf16(x, w_gate_up, glu=kind, glu_bias=bias)
+        elif _small_weight_library(T, w_gate_up, glu=True) or \
                 any(lo <= T <= hi for lo, hi in GEMM_LIBRARY_GLU_TOKENS):
             return gate(_library_linear(x, w_gate_up, None))
-        return linear_bf16(x, w_gate_up, glu=kind)
-    return gate(linear(x, w_gate_up))
+        else:
+            return linear_bf16(x, w_gate_up, glu=kind)
+    return gate(linear(x, w_gate_up, bias))
 
 
 # ------------------------------------------------------------------ sampling

@@ -332,3 +332,23 @@ def test_which_products_the_fma_pipes_take(T, N, K, gated, takes, monkeypatch):
     o = ops()
     monkeypatch.setattr(o, "sm_count", lambda device=None: 148)
     assert o._on_fma_pipes(T, N, K, gated) == takes
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("T,N,K", [(129, 40, 64), (256, 128, 72), (257, 200, 128), (700, 333, 512)])
+def test_gated_unit_with_biases_in_the_epilogue(T, N, K, kind):
+    """The two-SM kernel adds gate's and up's biases to its float32 sums; ragged rows and features."""
+    g = torch.Generator().manual_seed(T + N)
+    x, w = torch.randn(T, K, generator=g).bfloat16(), (torch.randn(2 * N, K, generator=g) * K ** -0.5).bfloat16()
+    b = torch.randn(2 * N, generator=g)
+    got = ops().linear_bf16(x.cuda(), w.cuda(), glu=kind, glu_bias=b.cuda()).cpu().double()
+    y = x.double() @ w.double().T + b.double()
+    act = torch.nn.functional.silu if kind == "silu" else (lambda t: torch.nn.functional.gelu(t, approximate="tanh"))
+    want = act(y[:, :N]) * y[:, N:]
+    # one rounding to eight bits, after sums of 32 bits
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5).all()
+    with pytest.raises(ops().KernelError):
+        ops().linear_bf16(x[:128].cuda(), w.cuda(), glu=kind, glu_bias=b.cuda())
+    with pytest.raises(ops().KernelError):
+        ops().linear_bf16(x.cuda(), w.cuda(), glu=kind, bias=b[:N].cuda())
