@@ -711,6 +711,17 @@ def gemv_features(tokens: int, K: int, gated: bool) -> int:
     return 1536 if tokens in (3, 4) and K <= 1024 else 0
 
 
+def gemv_block_features(tokens: int, features: int, K: int) -> int:
+    """Features a block of a plain product on the FMA pipes: 16, or 8, with twice the warps a row, where that
+    many blocks have an SM each, or, at one token and K up to 2,048, find a place in one round (the slots of
+    the squares, rounded up to 128 features, included).  16 / 8, chains over cold weights, us: 896 x 4,864 at one
+    token 5.1 / 3.6, 1,024 x 4,096 3.7 / 3.0, at two 5.0 / 4.0, 1,152 x 896 at one, two, four 2.2, 2.8, 3.5 / 2.1, 2.6,
+    2.6, 2,048 x 2,048 at one 4.3 / 3.2; but 2,368 x 1,024 at two 2.9 / 4.3, 1,536 x 256 at two 2.5 / 3.0, 2,048 x 8,192
+    at one 8.7 / 9.3, 512 x 512 1.66 / 1.78."""
+    one_round = tokens == 1 and K <= 2048 and 16 * -(-features // 128) <= 2 * sm_count()
+    return 8 if K > 512 and (-(-features // 8) <= sm_count() or one_round) else 16
+
+
 #: tokens -> bytes of a weight matrix up to which plain products run on the FMA pipes; None: what
 #: ``gemv_features`` says
 GEMV_WEIGHT_BYTES = {1: None, 2: None, 3: None, 4: None}
@@ -785,6 +796,9 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         if sumsq.shape[0] != T or not sumsq.is_contiguous():
             raise KernelError(f"sumsq has shape {tuple(sumsq.shape)} for {T} tokens")
     sumsq_out = None
+    on_fma = plan is None and cluster is None and two_sm is None and T <= 4 \
+        and (not glu or out_dtype == torch.bfloat16) and _on_fma_pipes(T, N, K, bool(glu)) \
+        and (x.data_ptr() | weight.data_ptr()) % 16 == 0
     if residual is not None:
         _check(residual, "residual", torch.float32, 2)
         if tuple(residual.shape) != (T, N) or not residual.is_contiguous():
@@ -797,6 +811,8 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
             if norm_weight.numel() != N:
                 raise KernelError(f"norm weight has {norm_weight.numel()} entries for width {N}")
             slots = 8 * -(-N // 128)
+            if norm_out is None and on_fma:
+                slots *= 16 // gemv_block_features(T, N, K)
             if norm_out is not None:
                 out, sumsq_out = norm_out
                 _check(out, "norm_out[0]", torch.bfloat16, 2)
@@ -812,15 +828,15 @@ def linear_bf16(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
         out = torch.empty((T, N), dtype=out_dtype, device=x.device)
     if T == 0:
         return out if residual is None else ((out, sumsq_out) if norm_weight is not None else None)
-    if plan is None and cluster is None and two_sm is None and T <= 4 \
-            and (not glu or out_dtype == torch.bfloat16) and _on_fma_pipes(T, N, K, bool(glu)) \
-            and (x.data_ptr() | weight.data_ptr()) % 16 == 0:
+    if on_fma:
+        # (norm_out's tensors have the slots of the tensor-core kernel: 16 features each)
+        block = 16 if glu or norm_out is not None else gemv_block_features(T, N, K)
         f = _fn("gemm_bf16", "hb_gemv_bf16",
                 [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                 c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p])
+                 c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_void_p])
         _run(f(_p(out), _p(x), _p(weight), _p(bias), T, N, K, K, K, N, glu_code, N if glu else 0, 1 if out_dtype == torch.float32 else 0,
                _p(residual), _p(norm_weight), _p(sumsq_out), _p(sumsq), 0 if sumsq is None else sumsq.shape[1],
-               float(eps), _stream()), "gemv_bf16")
+               float(eps), block, sm_count(x.device), _stream()), "gemv_bf16")
         if residual is not None:
             return (out, sumsq_out) if norm_weight is not None else None
         return out

@@ -352,3 +352,39 @@ def test_gated_unit_with_biases_in_the_epilogue(T, N, K, kind):
         ops().linear_bf16(x[:128].cuda(), w.cuda(), glu=kind, glu_bias=b.cuda())
     with pytest.raises(ops().KernelError):
         ops().linear_bf16(x.cuda(), w.cuda(), glu=kind, bias=b[:N].cuda())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [1, 2, 4])
+@pytest.mark.parametrize("N,K", [(1184, 520), (1185, 520), (2304, 1000), (2305, 1000), (1100, 2056), (1184, 512)])
+def test_products_of_few_tokens_with_blocks_of_eight_and_sixteen_features(T, N, K, monkeypatch):
+    """Both sides of the sizes at which blocks have eight features, and a partial sum of squares each;
+    given tensors keep eight slots to 128 features."""
+    o = ops()
+    monkeypatch.setattr(o, "GEMV_WEIGHT_BYTES", {1: 1 << 30, 2: 1 << 30, 4: 1 << 30})
+    g = torch.Generator().manual_seed(N + K)
+    x, w = torch.randn(T, K, generator=g).bfloat16().cuda(), (torch.randn(N, K, generator=g) * K ** -0.5).bfloat16().cuda()
+    res, nw = torch.randn(T, N, generator=g).cuda(), (torch.rand(N, generator=g) + 0.5).cuda()
+    want = res.double() + x.double() @ w.double().T
+    given = (torch.empty(T, N, dtype=torch.bfloat16, device="cuda"), torch.full((T, 8 * -(-N // 128)), float("nan"), device="cuda"))
+    for out in (None, given):
+        r = res.clone()
+        scaled, squares = o.linear_bf16(x, w, residual=r, norm_weight=nw, norm_out=out)
+        # float32 sums of K products of order 1 / K
+        assert (r.double() - want).abs().max() < 1e-5
+        assert torch.equal(scaled, (r * nw).bfloat16())
+        torch.testing.assert_close(squares.double().sum(-1), (r.double() ** 2).sum(-1), rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [4736, 4737, 5328, 5329, 5921])
+def test_gated_units_of_one_token_with_blocks_of_eight_to_ten_warps(N):
+    """Blocks of 16, 18 and 20 features, whichever need the fewest rounds."""
+    o, K = ops(), 520
+    g = torch.Generator().manual_seed(N)
+    x, w = torch.randn(1, K, generator=g).bfloat16().cuda(), (torch.randn(2 * N, K, generator=g) * K ** -0.5).bfloat16().cuda()
+    slots = torch.rand(1, 24, generator=g).cuda()
+    y = (x.double() @ w.double().T) * torch.rsqrt(slots.double().sum() / K + 1e-5)
+    want = torch.nn.functional.silu(y[:, :N]) * y[:, N:]
+    got = o.linear_bf16(x, w, glu=True, sumsq=slots, eps=1e-5)
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-4).all()
