@@ -788,7 +788,9 @@ def test_generic_attention_of_few_rows_with_all_loads_ahead_is_the_same_bit_for_
     T = case.qkv.shape[0]
     g = torch.Generator().manual_seed(hd)
     gate = torch.randn(T, nh * hd, generator=g).to(DEV, dtype)
-    pooled = (case.k_pages.nan_to_num(), case.v_pages.nan_to_num(), torch.zeros((len(seqs), 6), dtype=torch.int32, device=DEV), 7)
+    # (any pages do as the means of blocks of seven tokens; the table is as wide as the longest request's means)
+    wide = -(-((max(lens) - 60) // 7 + 1) // page)
+    pooled = (case.k_pages.nan_to_num(), case.v_pages.nan_to_num(), torch.zeros((len(seqs), wide), dtype=torch.int32, device=DEV), 7)
     few = o.sm_count() // nh
     assert few * nh <= o.sm_count() < (T - few) * nh
     for window, keep, means in ((None, 0, None), (1, 0, None), (33, 0, None), (40, 3, None), (60, 0, pooled), (300, 0, None)):
