@@ -526,9 +526,12 @@ def silu_mul(gate_up: torch.Tensor) -> torch.Tensor:
 
 # ------------------------------------------------------------------ matrix products
 #: rows of x up to which the float32 product streams the weight through the kernel for few rows
-#: (eight at a time).  Tiles / rows, microseconds, at 16 rows: 9,728 x 896 46 / 35; 896 x 4,864
-#: 59 / 45; 1,152 x 896 14.5 / 8; at 24 rows 46 / 47, 59 / 64 and 14.5 / 14
+#: (eight at a time; of a weight of 2,048 rows or more only up to eight).  Tiles / rows, microseconds, at
+#: 12 rows: 896 x 4,864 32 / 26; 1,152 x 896 9.2 / 7.9; 896 x 896 8.7 / 7.4; at 16 rows 32 / 34, 9.2 / 9.3,
+#: 8.7 / 7.9
 GEMM_F32_FEW_ROWS = 16
+#: the form of those kernels, 0: by size (``hb_gemm_f32_as``); the results are the same
+GEMM_F32_FORM = 0
 
 
 def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -544,11 +547,14 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
         if bias.numel() != N:
             raise KernelError(f"bias has {bias.numel()} entries for {N} outputs")
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    f = _fn("gemm_f32", "hb_gemm_f32",
-            [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-             c_void_p])
-    _run(f(_p(out), _p(x), _p(weight), _p(bias), M, N, K, K, K, N, GEMM_F32_FEW_ROWS, sm_count(x.device), _stream()),
-         "gemm_f32")
+    pointers, sizes = [c_void_p] * 4, [c_int] * 7
+    args = (_p(out), _p(x), _p(weight), _p(bias), M, N, K, K, K, N, GEMM_F32_FEW_ROWS)
+    if GEMM_F32_FORM == 0:
+        f = _fn("gemm_f32", "hb_gemm_f32", pointers + sizes + [c_int, c_void_p])
+        _run(f(*args, sm_count(x.device), _stream()), "gemm_f32")
+    else:
+        f = _fn("gemm_f32", "hb_gemm_f32_as", pointers + sizes + [c_int, c_int, c_void_p])
+        _run(f(*args, GEMM_F32_FORM, sm_count(x.device), _stream()), "gemm_f32")
     return out
 
 

@@ -821,3 +821,24 @@ def test_sampling_with_packed_options_and_rows_that_are_and_are_not_whole_pieces
     assert torch.equal(o.sample(logits, *dev, kind="one_block"), got)
     with pytest.raises(o.KernelError):
         o.sample_packed(logits, packed[:-1], "narrow")
+
+
+@pytest.mark.parametrize("M", [1, 3, 4, 6, 8, 9, 16, 31, 33, 65])
+@pytest.mark.parametrize("N,K", [(1, 4), (7, 68), (65, 132), (130, 516), (2050, 64), (600, 2052), (40, 9000)])
+def test_gemm_f32_in_every_form_is_the_same_bit_for_bit(M, N, K, monkeypatch):
+    """Two and four rows of W a warp, tiles of 4 x 4 and 8 x 4 outputs a thread, and what the sizes choose: rows
+    and columns that end inside all of them, quarters of K that are short or empty."""
+    o = ops()
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
+    xd, wd, bd = x.to(DEV), w.to(DEV), b.to(DEV)
+    got = o.linear_f32(xd, wd, bd)
+    for form in (2, 4, 44, 84):
+        monkeypatch.setattr(o, "GEMM_F32_FORM", form)
+        if form >= 44:
+            monkeypatch.setattr(o, "GEMM_F32_FEW_ROWS", 0)
+        assert torch.equal(o.linear_f32(xd, wd, bd), got), form
+    want = x.double() @ w.double().T + b.double()
+    # runs of 8 + 8, up to K / 64 runs a quarter, four quarters and the bias: as many roundings of a product's size
+    bound = (K / 64 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs())
+    assert ((got.double().cpu() - want).abs() <= bound).all()
