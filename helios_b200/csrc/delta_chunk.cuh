@@ -63,9 +63,11 @@ __host__ __device__ __forceinline__ long dc_chunks(long n_tokens, long n_seqs) {
 
 // One block a (chunk, head).  Bound by its instructions: 256 dot products over dk with a running product of
 // decays each, and the splitting.  Sixteen threads a dot product, the pairs (i, j) of two rows j and 15 - j by the
-// same threads, so that all walk 17.
+// same threads, so that all walk 17; the sums of four rows i go over the lanes together, eight shuffles for 32.  Six
+// blocks an SM (80 registers): with the walk, 2,048 tokens of 16 heads of 128 x 128, 185 -> 178 µs (four 179, eight
+// with their spills 188).
 template <typename T, int DK>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 6)
 delta_chunk_prepare_kernel(uint32_t* __restrict__ chunks, const T* __restrict__ qkv, int qkv_ld, int q_off, int k_off,
                            const T* __restrict__ beta_raw, int beta_ld, const T* __restrict__ a_raw, int a_ld,
                            const float* __restrict__ a_log, const float* __restrict__ dt_bias,
@@ -154,29 +156,39 @@ delta_chunk_prepare_kernel(uint32_t* __restrict__ chunks, const T* __restrict__ 
       float4 w[M];
 #pragma unroll
       for (int m = 0; m < M; ++m) w[m] = *reinterpret_cast<const float4*>(&ks[j][4 * part + 64 * m]);
-#pragma unroll 4
-      for (int i = j; i < N; ++i) {
-        float a = 0.f, b = 0.f;
+#pragma unroll 1
+      for (int i0 = j; i0 < N; i0 += 4) {             // (the two halves of a warp may be at different rows)
+        float sums[8];                                // of k, then of q
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-          if (i > j) {
-            const float4 g = *reinterpret_cast<const float4*>(&gs[i][4 * part + 64 * m]);
-            w[m].x *= g.x; w[m].y *= g.y; w[m].z *= g.z; w[m].w *= g.w;
+        for (int r = 0; r < 4; ++r) {
+          const int i = min(i0 + r, N - 1);
+          float a = 0.f, b = 0.f;
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+            if (i0 + r > j) {
+              const float4 g = *reinterpret_cast<const float4*>(&gs[i][4 * part + 64 * m]);
+              w[m].x *= g.x; w[m].y *= g.y; w[m].z *= g.z; w[m].w *= g.w;
+            }
+            const float4 k = *reinterpret_cast<const float4*>(&ks[i][4 * part + 64 * m]);
+            const float4 q = *reinterpret_cast<const float4*>(&qs[i][4 * part + 64 * m]);
+            a = fmaf(w[m].x, k.x, fmaf(w[m].y, k.y, fmaf(w[m].z, k.z, fmaf(w[m].w, k.w, a))));
+            b = fmaf(w[m].x, q.x, fmaf(w[m].y, q.y, fmaf(w[m].z, q.z, fmaf(w[m].w, q.w, b))));
           }
-          const float4 k = *reinterpret_cast<const float4*>(&ks[i][4 * part + 64 * m]);
-          const float4 q = *reinterpret_cast<const float4*>(&qs[i][4 * part + 64 * m]);
-          a = fmaf(w[m].x, k.x, fmaf(w[m].y, k.y, fmaf(w[m].z, k.z, fmaf(w[m].w, k.w, a))));
-          b = fmaf(w[m].x, q.x, fmaf(w[m].y, q.y, fmaf(w[m].z, q.z, fmaf(w[m].w, q.w, b))));
+          sums[r] = a;
+          sums[4 + r] = b;
         }
+        // eight sums over sixteen lanes: half of them to the other half of the lanes at each step
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {             // (the two halves of a warp may be at different i)
-          a += __shfl_xor_sync(0xffffu << (lane & 16), a, o);
-          b += __shfl_xor_sync(0xffffu << (lane & 16), b, o);
-        }
-        if (part == 0) {
-          am[i][j] = a;
-          bm[i][j] = b;
-        }
+        for (int o = 8, left = 4; o > 1; o /= 2, left /= 2)
+#pragma unroll
+          for (int x = 0; x < left; ++x) {
+            const bool upper = part & o;
+            const float got = __shfl_xor_sync(0xffffu << (lane & 16), upper ? sums[x] : sums[x + left], o);
+            sums[x] = (upper ? sums[x + left] : sums[x]) + got;
+          }
+        sums[0] += __shfl_xor_sync(0xffffu << (lane & 16), sums[0], 1);
+        const int i = i0 + (part >> 1 & 1) + (part >> 1 & 2);
+        if (!(part & 1) && i < N) (part & 8 ? bm : am)[i][j] = sums[0];
       }
     }
   }
@@ -249,17 +261,23 @@ __device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], co
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
 }
-// the six products of two factors of three planes each, by size: sums[0] += a0 b0, ...
-__device__ __forceinline__ void dc_mma_split(float (&sums)[3][4], const uint32_t (&a)[3][4], const uint32_t* frag, int lane) {
-  uint2 b[3];
+// the six products of two factors of three planes each, by size: sums[0] += a0 b0, ...; of two results in turn, so
+// that a product's sums are there when the next one adds to them (one result after the other waited 28 of 79 cycles)
+__device__ __forceinline__ void dc_mma_split(float (&x)[3][4], float (&y)[3][4], const uint32_t (&a)[3][4],
+                                             const uint32_t* frag_x, const uint32_t* frag_y, int lane) {
+  uint2 b[3], c[3];
 #pragma unroll
-  for (int p = 0; p < 3; ++p) b[p] = *reinterpret_cast<const uint2*>(frag + 64 * p + 2 * lane);
-  dc_mma(sums[0], a[0], b[0]);
-  dc_mma(sums[1], a[1], b[0]);
-  dc_mma(sums[2], a[2], b[0]);
-  dc_mma(sums[1], a[0], b[1]);
-  dc_mma(sums[2], a[1], b[1]);
-  dc_mma(sums[2], a[0], b[2]);
+  for (int p = 0; p < 3; ++p) {
+    b[p] = *reinterpret_cast<const uint2*>(frag_x + 64 * p + 2 * lane);
+    c[p] = *reinterpret_cast<const uint2*>(frag_y + 64 * p + 2 * lane);
+  }
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+#pragma unroll
+    for (int q = 0; q + p < 3; ++q) {
+      dc_mma(x[p + q], a[q], b[p]);
+      dc_mma(y[p + q], a[q], c[p]);
+    }
 }
 __device__ __forceinline__ float dc_total(const float (&sums)[3][4], int e) { return sums[0][e] + (sums[1][e] + sums[2][e]); }
 template <int BARRIER, int THREADS>
@@ -285,7 +303,9 @@ struct DeltaChunkSmem {
 // quarter of dk each (columns of S on the rows of the fragment), which are as they stand the A operand of S^T Kc and
 // S^T Qc.  The other four own the solution: four columns each, two tokens of a column a thread.  A chunk's
 // chain is S^T Kc -> barrier -> sums of the four quarters, U = T R -> barrier -> the write into S; S^T Qc runs beside
-// the solution, the outputs and the copies beside the write.  Bound by that chain, 1.05 µs a chunk; eight
+// the solution, the outputs and the copies beside the write.  Bound by that chain, a microsecond
+// a chunk (1.05 before the products of two tiles ran in turn and the next chunk's planes were made beside the
+// write: 185 -> 180 µs of 2,048 tokens); eight
 // warps of 16 dk each instead of four take as long (and 5 % longer where blocks share SMs).
 template <typename T, int DK, int GROUPS, int STAGES>
 __global__ void __launch_bounds__(GROUPS * DC_GROUP_THREADS)
@@ -318,26 +338,30 @@ delta_chunk_kernel(float* __restrict__ o, const uint32_t* __restrict__ chunks, c
         const int d = d0 + 8 * m + 2 * kap + (e & 1), c = row + 8 * (e >> 1);
         S[m][e] = d < dk && col0 + c < dv ? S_g[(size_t)d * dv + c] : 0.f;
       }
-    dc_bar_sync<2, THREADS>();                        // the first chunk is there
-    for (int ch = 0; ch < n_chunks; ++ch) {
-      const uint32_t* st = dc_sm + ch % STAGES * C::WORDS;
-      uint32_t a[ND / 2][3][4];                       // [16 dk][plane]: rows col, col + 8 of two tiles
+    uint32_t a[ND / 2][3][4];                         // [16 dk][plane]: rows col, col + 8 of two tiles
+    auto split_tiles = [&](int m) {                   // tiles m, m + 1
 #pragma unroll
-      for (int m = 0; m < ND; ++m)
+      for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           uint32_t w[3];
-          dc_split(S[m][2 * e], S[m][2 * e + 1], w);
+          dc_split(S[m + t][2 * e], S[m + t][2 * e + 1], w);
 #pragma unroll
-          for (int p = 0; p < 3; ++p) a[m / 2][p][2 * (m % 2) + e] = w[p];
+          for (int p = 0; p < 3; ++p) a[m / 2][p][2 * t + e] = w[p];
         }
+    };
+#pragma unroll
+    for (int m = 0; m < ND; m += 2) split_tiles(m);
+    dc_bar_sync<2, THREADS>();                        // the first chunk is there
+    for (int ch = 0; ch < n_chunks; ++ch) {
+      const uint32_t* st = dc_sm + ch % STAGES * C::WORDS;
       auto product = [&](const uint32_t* frags, float* part) {
         float sums[2][3][4] = {};
 #pragma unroll
-        for (int m = 0; m < ND / 2; ++m)
-#pragma unroll
-          for (int t = 0; t < 2; ++t)
-            dc_mma_split(sums[t], a[m], frags + ((warp * (ND / 2) + m) * 2 + t) * 3 * C::PLANE, lane);
+        for (int m = 0; m < ND / 2; ++m) {
+          const uint32_t* frag = frags + (warp * (ND / 2) + m) * 2 * 3 * C::PLANE;
+          dc_mma_split(sums[0], sums[1], a[m], frag, frag + 3 * C::PLANE, lane);
+        }
         float* p = part + warp * M::PART + row * PLD + 2 * kap;
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
@@ -361,12 +385,17 @@ delta_chunk_kernel(float* __restrict__ o, const uint32_t* __restrict__ chunks, c
         for (int p = 0; p < 3; ++p) u[p][e] = w[p];
       }
 #pragma unroll
-      for (int m = 0; m < ND; ++m) {
-        float sums[3][4] = {};
-        dc_mma_split(sums, u, st + C::E + (warp * ND + m) * 3 * C::PLANE, lane);
-        const float2 g = *reinterpret_cast<const float2*>(st + C::G + d0 + 8 * m + 2 * kap);
+      for (int m = 0; m < ND; m += 2) {
+        float sums[2][3][4] = {};
+        const uint32_t* frag = st + C::E + (warp * ND + m) * 3 * C::PLANE;
+        dc_mma_split(sums[0], sums[1], u, frag, frag + 3 * C::PLANE, lane);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[m][e] = fmaf(S[m][e], (e & 1) ? g.y : g.x, dc_total(sums, e));
+        for (int t = 0; t < 2; ++t) {
+          const float2 g = *reinterpret_cast<const float2*>(st + C::G + d0 + 8 * (m + t) + 2 * kap);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[m + t][e] = fmaf(S[m + t][e], (e & 1) ? g.y : g.x, dc_total(sums[t], e));
+        }
+        split_tiles(m);                               // for the next chunk, beside the other tiles' products
       }
     }
 #pragma unroll

@@ -2285,7 +2285,7 @@ def causal_conv_silu(ctx, x: torch.Tensor, channels: int, weight: torch.Tensor,
 #: Steps whose longest portion may have this many tokens, and that have DELTA_CHUNK_MEAN a request, walk the
 #: delta rule in chunks of 16 tokens (16-bit activations, keys of at most 128 values): keys of more than 64
 #: values | fewer, blocks of 16 columns that all have an SM of their own | fewer, more blocks.
-#: By tokens / by chunks, µs, 16 heads of 128 x 128: one request of 2,048 tokens 448 / 184, of 333 77 / 37, of 64
+#: By tokens / by chunks, µs, 16 heads of 128 x 128: one request of 2,048 tokens 448 / 172, of 333 77 / 37, of 64
 #: 20 / 16; 64 tokens of 32 requests 189 / 171, 32 of 16 53 / 52, 16 of 64 114 / 131; 1,000 beside 24 of one 272 /
 #: 143, 300 90 / 66.  8 heads of 64 x 64: 2,048 297 / 119, 700 of three 110 / 54, 64 13.9 / 12.2, 64 of 32 41 / 44,
 #: 1,000 beside 24 of one 190 / 95.  16 of 24 x 24: 200 29 / 20, 64 of 24 30 / 40.
