@@ -14,11 +14,17 @@
 // The products with S run on mma.sync in bfloat16, each float32 factor as the sum of three bfloat16 values
 // (x = x0 + x1 + x2, exact: 24 bits are 3 x 8), so six products of a pair (those below 2^-24 of the whole
 // are left out), by size in accumulators of their own: the large one holds products of 16 bits, which its
-// 24 take nearly without rounding.  S itself is float32 and takes one fused multiply-add a chunk instead of
-// two roundings a token.  Measured against 64 bits over 17 to 1,500 tokens (relative 2-norm, walk by tokens /
-// this): outputs 1.35e-7 to 1.6e-7 / 1.35e-7 to 1.6e-7, states 1.0e-7 to 1.7e-7 / 0.9e-7 to 1.6e-7 (with TF32
-// and its rest instead, three products, 1.5e-7 to 2.1e-7).  32-bit activations keep the walk by tokens, whose
-// numbers do not depend on how a prompt was cut.
+// 24 take nearly without rounding.  S itself is float32 and takes two fused multiply-adds a chunk instead of
+// two roundings a token.  A sum of a chunk has roundings that the walk by tokens has not, so what costs little is
+// made better than there: 1 / |k|, 1 / |q|, k . q and beta in 64 bits (a unit vector's element is rounded once), the
+// decays' rate as the sum of two, and the term of a token's own write, mostly the largest of its sum, is added last
+// (into o, u and, for a chunk's last token, S): 7 of 180 µs.  Errors against 64 bits, 2,048 tokens of 128 x 128,
+// relative 2-norms in e-7, walk by tokens / this, where the decays are 0.02, 0.46, 0.82, 0.995 and 0.9999 on average:
+// after silu outputs 1.31 / 0.50, 1.30 / 0.63, 1.28 / 0.87, 6.46 / 6.39, 24.1 / 18.9, states 0.73 / 0.50, 0.86 / 0.73,
+// 1.25 / 1.02, 8.69 / 8.29, 30.6 / 23.7; normal inputs, 0.02 and 0.82: outputs 1.46 / 0.51, 1.67 / 1.21, states 0.70 /
+// 0.50, 1.22 / 1.05, and without those measures 1.63, 1.85 and 0.90, 1.21.  Keys that are alike (a cosine of 0.8), dk
+// of 24: 0.98 to 1.06 of the walk's.  TF32 and its rest instead, three products: 1.5 to 2.1.
+// 32-bit activations keep the walk by tokens, whose numbers do not depend on how a prompt was cut.
 #pragma once
 #include "common.cuh"
 
@@ -37,8 +43,8 @@ template <int DK>
 struct DeltaChunk {
   static constexpr int PLANE = 64;                    // words a fragment's plane
   static constexpr int ROWS = 3 * DC_TOKENS * DK / 2; // words of one of the three
-  static constexpr int Q = ROWS, E = 2 * ROWS, G = 3 * ROWS;
-  static constexpr int TI = G + DK, BI = TI + DC_TOKENS * DC_TOKENS;
+  static constexpr int Q = ROWS, E = 2 * ROWS, G = 3 * ROWS, L = G + DK;
+  static constexpr int TI = L + DK, BI = TI + DC_TOKENS * DC_TOKENS;
   static constexpr int WORDS = BI + DC_TOKENS * DC_TOKENS;
   static_assert(WORDS % 4 == 0 && DK % 64 == 0, "");
 };
@@ -61,6 +67,12 @@ __host__ __device__ __forceinline__ long dc_chunks(long n_tokens, long n_seqs) {
   return (n_tokens - 1) / DC_TOKENS + n_seqs;
 }
 
+// g of a raw decay; the rate exp(a_log) as the sum of two
+__device__ __forceinline__ float dc_decay(float a, float rate_hi, float rate_lo) {
+  const float sp = a > 20.f ? a : log1pf(expf(a)), y = rate_hi * sp, g = expf(-y);
+  return g > 0.f ? fmaf(-g, fmaf(rate_lo, sp, fmaf(rate_hi, sp, -y)), g) : g;       // (y may be infinite)
+}
+
 // One block a (chunk, head).  Bound by its instructions: 256 dot products over dk with a running product of
 // decays each, and the splitting.  Sixteen threads a dot product, the pairs (i, j) of two rows j and 15 - j by the
 // same threads, so that all walk 17; the sums of four rows i go over the lanes together, eight shuffles for 32.  Six
@@ -77,7 +89,7 @@ delta_chunk_prepare_kernel(uint32_t* __restrict__ chunks, const T* __restrict__ 
   using C = DeltaChunk<DK>;
   constexpr int N = DC_TOKENS, LD = DK + 4;
   __shared__ __align__(16) float ks[N][LD], qs[N][LD], gs[N][LD];
-  __shared__ float am[N][N + 1], bm[N][N + 1], bs[N];
+  __shared__ float am[N][N + 1], bm[N][N + 1], bs[N], kqs[N];
   const int id = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int lo = 0, hi = n_seqs - 1;                        // the last request whose first chunk is not above id
   while (lo < hi) {
@@ -89,12 +101,11 @@ delta_chunk_prepare_kernel(uint32_t* __restrict__ chunks, const T* __restrict__ 
   const int nc = min(N, cu_tokens[lo + 1] - t_seq - c * N);
   if (c < 0 || nc <= 0) return;
   const int t0 = t_seq + c * N;
-  const float rate = expf(a_log[h]);
   const int kh = h / (heads / kv_heads);
   {
     // a warp's four tokens: everything is asked for before anything is summed
     constexpr int M = DK / 32;
-    float kx[4][M], qx[4][M], ax[4][M], bx[4], kk[4], qq[4], bias[M];
+    float kx[4][M], qx[4][M], ax[4][M], bias[M], beta = 0.f;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const size_t t = t0 + min(warp + 4 * r, nc - 1);
@@ -109,40 +120,64 @@ delta_chunk_prepare_kernel(uint32_t* __restrict__ chunks, const T* __restrict__ 
         qx[r][m] = in ? to_float(qr[d]) : 0.f;
         ax[r][m] = in ? to_float(ar[d]) : 0.f;
       }
-      bx[r] = to_float(beta_raw[t * beta_ld + h]);
     }
+    const int of = lane >> 3, own = warp + 4 * (lane >> 1 & 3);       // what this lane finishes below, and the token
+    if (of == 3) beta = to_float(beta_raw[(size_t)(t0 + min(own, nc - 1)) * beta_ld + h]);
 #pragma unroll
     for (int m = 0; m < M; ++m) bias[m] = lane + 32 * m < dk ? dt_bias[(size_t)h * dk + lane + 32 * m] : 0.f;
+    const double rate = exp((double)a_log[h]);
+    const float rate_hi = (float)rate, rate_lo = (float)(rate - (double)rate_hi);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {                   // (rows behind the last token: k = q = 0, g = 1, beta = 0)
+        const int d = lane + 32 * m;
+        gs[warp + 4 * r][d] = warp + 4 * r < nc && d < dk ? dc_decay(ax[r][m] + bias[m], rate_hi, rate_lo) : 1.f;
+      }
+    // |k|^2, |q|^2 and k . q of the four tokens: a lane's few products in 32 bits, the lanes' in 64; of two partners
+    // each goes on with half of the sums, and lane 8 of + 2 r ends up with sum `of` of token r
+    double sums[16];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      kk[r] = qq[r] = 0.f;
+      float kk = 0.f, qq = 0.f, kq = 0.f;
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        kk[r] = fmaf(kx[r][m], kx[r][m], kk[r]);
-        qq[r] = fmaf(qx[r][m], qx[r][m], qq[r]);
+        kk = fmaf(kx[r][m], kx[r][m], kk);
+        qq = fmaf(qx[r][m], qx[r][m], qq);
+        kq = fmaf(kx[r][m], qx[r][m], kq);
       }
+      sums[r] = kk;
+      sums[4 + r] = qq;
+      sums[8 + r] = kq;
+      sums[12 + r] = 0.;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int left = 8, o = 16; left > 0; left /= 2, o /= 2)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        kk[r] += __shfl_xor_sync(0xffffffffu, kk[r], o);
-        qq[r] += __shfl_xor_sync(0xffffffffu, qq[r], o);
+      for (int x = 0; x < left; ++x) {
+        const bool upper = lane & o;
+        const double got = __shfl_xor_sync(0xffffffffu, upper ? sums[x] : sums[x + left], o);
+        sums[x] = (upper ? sums[x + left] : sums[x]) + got;
       }
-    const float scale = rsqrtf((float)dk);
+    double value = sums[0] + __shfl_xor_sync(0xffffffffu, sums[0], 1);
+    // 1 / |k|, dk^-1/2 / |q|, k . q of the unit vectors, beta
+    if (of < 2) value = rsqrt((value + 1e-6) * (of ? (double)dk : 1.));
+    if (of == 3) value = 1. / (1. + exp(-(double)beta));
+    const double kn = __shfl_sync(0xffffffffu, value, lane & 6), qn = __shfl_sync(0xffffffffu, value, 8 + (lane & 6));
+    if (of == 2) value *= kn * qn;
+    const float hi = (float)value, lo = (float)(value - (double)hi);
+    if (of >= 2 && !(lane & 1)) (of == 2 ? kqs : bs)[own] = own < nc ? hi : 0.f;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int i = warp + 4 * r;
-      const bool token = i < nc;                      // (rows behind the last token: k = q = 0, g = 1, beta = 0)
-      const float kn = rsqrtf(kk[r] + 1e-6f), qn = rsqrtf(qq[r] + 1e-6f) * scale;
+      const float k_hi = __shfl_sync(0xffffffffu, hi, 2 * r), k_lo = __shfl_sync(0xffffffffu, lo, 2 * r);
+      const float q_hi = __shfl_sync(0xffffffffu, hi, 8 + 2 * r), q_lo = __shfl_sync(0xffffffffu, lo, 8 + 2 * r);
 #pragma unroll
       for (int m = 0; m < M; ++m) {
         const int d = lane + 32 * m;
-        ks[i][d] = token ? kx[r][m] * kn : 0.f;
-        qs[i][d] = token ? qx[r][m] * qn : 0.f;
-        gs[i][d] = token && d < dk ? delta_decay(ax[r][m] + bias[m], rate) : 1.f;
+        ks[i][d] = i < nc ? fmaf(kx[r][m], k_hi, kx[r][m] * k_lo) : 0.f;
+        qs[i][d] = i < nc ? fmaf(qx[r][m], q_hi, qx[r][m] * q_lo) : 0.f;
       }
-      if (lane == 0) bs[i] = token ? delta_beta(bx[r]) : 0.f;
     }
   }
   __syncthreads();
@@ -223,9 +258,10 @@ delta_chunk_prepare_kernel(uint32_t* __restrict__ chunks, const T* __restrict__ 
     float p = 1.f, e[N];
 #pragma unroll
     for (int i = N - 1; i >= 0; --i) {
-      e[i] = ks[i][d] * p;
+      e[i] = i == nc - 1 ? 0.f : ks[i][d] * p;        // (the last token's write has no product of decays)
       p *= gs[i][d];
     }
+    reinterpret_cast<float*>(dst)[C::L + d] = ks[nc - 1][d];
     uint32_t* to = dst + C::E + (d / 8) * 3 * C::PLANE + (d % 8) * 8;
     uint32_t w[N / 2][3];                             // [2 kappa + half of the tokens]
 #pragma unroll
@@ -239,7 +275,7 @@ delta_chunk_prepare_kernel(uint32_t* __restrict__ chunks, const T* __restrict__ 
   __syncthreads();
   for (int idx = tid; idx < N * N; idx += 128) {
     const int i = idx / N, j = idx % N;
-    reinterpret_cast<float*>(dst)[C::BI + idx] = j <= i ? bm[i][j] : 0.f;
+    reinterpret_cast<float*>(dst)[C::BI + idx] = j < i ? bm[i][j] : j == i ? kqs[i] : 0.f;
   }
   if (tid < N) {                                      // a column of T a thread
     float x[N];
@@ -373,6 +409,8 @@ delta_chunk_kernel(float* __restrict__ o, const uint32_t* __restrict__ chunks, c
       dc_bar_arrive<1, THREADS>();
       product(st + C::Q, gm + M::PQ + (ch & 1) * 4 * M::PART);
       dc_bar_sync<2, THREADS>();
+      const float* u_last = gm + M::U + (min(N, n - ch * N) - 1) * PLD + row;
+      const float last[2] = {u_last[0], u_last[8]};
       // U^T [columns, tokens]; k = 2 kap, 2 kap + 1 of eight tokens are tokens kap and kap + 4
       uint32_t u[3][4];
       const float* us = gm + M::U + kap * PLD + row;
@@ -392,8 +430,11 @@ delta_chunk_kernel(float* __restrict__ o, const uint32_t* __restrict__ chunks, c
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           const float2 g = *reinterpret_cast<const float2*>(st + C::G + d0 + 8 * (m + t) + 2 * kap);
+          const float2 k = *reinterpret_cast<const float2*>(st + C::L + d0 + 8 * (m + t) + 2 * kap);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) S[m + t][e] = fmaf(S[m + t][e], (e & 1) ? g.y : g.x, dc_total(sums[t], e));
+          for (int e = 0; e < 4; ++e)                 // (the last token's write comes last, with one rounding)
+            S[m + t][e] = fmaf((e & 1) ? k.y : k.x, last[e >> 1],
+                               fmaf(S[m + t][e], (e & 1) ? g.y : g.x, dc_total(sums[t], e)));
         }
         split_tiles(m);                               // for the next chunk, beside the other tiles' products
       }
@@ -435,13 +476,14 @@ delta_chunk_kernel(float* __restrict__ o, const uint32_t* __restrict__ chunks, c
     dc_bar_sync<2, THREADS>();
     float* rs = gm + M::R;
     float* us = gm + M::U;
-    // a row of T or B times a column: it ends at the row's own token (a token that holds NaN must not reach
-    // the ones before it, as zero times NaN would)
-    auto row_sum = [&](const float (&w)[N], const float (&x)[N], int last) {
-      float a[4] = {};
+    // a + the row of T or B left of its own token, times a column (a token that holds NaN must not reach the ones
+    // before it, as zero times NaN would).  The own token's term, mostly the largest, is added last by the callers:
+    // one rounding of its size.
+    auto row_sum = [&](float first, const float (&w)[N], const float (&x)[N], int token) {
+      float a[4] = {first};
 #pragma unroll
-      for (int j = 0; j < N; ++j)
-        if (j <= last) a[j & 3] = fmaf(w[j], x[j], a[j & 3]);
+      for (int j = 0; j < N - 1; ++j)
+        if (j < token) a[(j + 1) & 3] = fmaf(w[j], x[j], a[(j + 1) & 3]);
       return (a[0] + a[1]) + (a[2] + a[3]);
     };
     auto parts_sum = [&](const float* p) { return (p[0] + p[M::PART]) + (p[2 * M::PART] + p[3 * M::PART]); };
@@ -452,24 +494,29 @@ delta_chunk_kernel(float* __restrict__ o, const uint32_t* __restrict__ chunks, c
     for (int ch = 0; ch < n_chunks; ++ch) {
       const float* st = reinterpret_cast<const float*>(dc_sm + ch % STAGES * C::WORDS);
       const int nc = min(N, n - ch * N);
-      float v[2], t_row[2][N];
+      float v[2], t_row[2][N], t_own[2], b_own[2], sum[2];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        v[e] = to_float(v_next[e]);
+        v[e] = tok + 8 * e < nc ? to_float(v_next[e]) : 0.f;
         load_row(t_row[e], st + C::TI + (tok + 8 * e) * N);
+        t_own[e] = st[C::TI + (tok + 8 * e) * (N + 1)];
+        b_own[e] = st[C::BI + (tok + 8 * e) * (N + 1)];
       }
       fetch_v(ch + 1);
       dc_bar_sync<1, THREADS>();
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const float sum = parts_sum(gm + M::PK + own * PLD + tok + 8 * e);
-        rs[own * 20 + tok + 8 * e] = tok + 8 * e < nc ? v[e] - sum : 0.f;
+        sum[e] = tok + 8 * e < nc ? parts_sum(gm + M::PK + own * PLD + tok + 8 * e) : 0.f;
+        rs[own * 20 + tok + 8 * e] = v[e] - sum[e];
       }
       __syncwarp();
       float r[N];
       load_row(r, rs + own * 20);
 #pragma unroll
-      for (int e = 0; e < 2; ++e) us[(tok + 8 * e) * PLD + own] = row_sum(t_row[e], r, tok + 8 * e);
+      for (int e = 0; e < 2; ++e) {
+        sum[e] = fmaf(t_own[e], v[e], row_sum(-t_own[e] * sum[e], t_row[e], r, tok + 8 * e));
+        us[(tok + 8 * e) * PLD + own] = sum[e];
+      }
       asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 3));
       dc_bar_sync<2, THREADS>();
       float u[N];
@@ -480,8 +527,8 @@ delta_chunk_kernel(float* __restrict__ o, const uint32_t* __restrict__ chunks, c
         const int i = tok + 8 * e;
         float b_row[N];
         load_row(b_row, st + C::BI + i * N);
-        const float sum = parts_sum(gm + M::PQ + (ch & 1) * 4 * M::PART + own * PLD + i);
-        if (live && i < nc) o_col[(size_t)(t0 + ch * N + i) * o_step] = sum + row_sum(b_row, u, i);
+        const float before = row_sum(parts_sum(gm + M::PQ + (ch & 1) * 4 * M::PART + own * PLD + i), b_row, u, i);
+        if (live && i < nc) o_col[(size_t)(t0 + ch * N + i) * o_step] = fmaf(b_own[e], sum[e], before);
       }
       // the stage of the chunk before: its last reads were made before this chunk's first barrier
       stage(ch + STAGES - 1);

@@ -817,6 +817,47 @@ def test_delta_rule_by_chunks_of_tokens_is_the_plain_scan(dk, dv, lens, monkeypa
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shift", [4.0, 0.0, -2.0, -10.0])
+@pytest.mark.parametrize("dk,dv", [(64, 64), (128, 128)])
+def test_delta_rule_by_chunks_is_as_near_to_64_bits_as_the_walk_by_tokens(dk, dv, shift, monkeypatch):
+    """Decays from 0.02 to 0.9999 on average: outputs and states of a prompt, both ways, against the scan in 64
+    bits."""
+    from types import SimpleNamespace
+    from helios_b200.csrc import ops
+
+    dev, heads, T = "cuda", 6, 300
+    g = torch.Generator(device=dev).manual_seed(dk)
+    r = lambda *s: torch.randn(*s, generator=g, device=dev)
+    qkv = torch.nn.functional.silu(r(T, heads * (2 * dk + dv))).bfloat16()
+    beta, a = (r(T, heads) + 1).bfloat16(), (r(T, heads * dk) + shift).bfloat16()
+    a_log, dt_bias, before = r(heads) * 0.3, r(heads * dk) * 0.3, r(1, heads * dk * dv) * 0.3
+    ctx = SimpleNamespace(cu_tokens=torch.tensor([0, T], dtype=torch.int32, device=dev),
+                          slots=torch.zeros(1, dtype=torch.int32, device=dev), num_seqs=1)
+    q, k, v = (x.view(T, heads, -1) for x in qkv.double().split([heads * dk, heads * dk, heads * dv], 1))
+    q = q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * dk ** -0.5
+    k = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    gd = torch.exp(-torch.exp(a_log.double())[:, None] * torch.nn.functional.softplus(
+        (a.double() + dt_bias.double()).view(T, heads, dk)))
+    b, S, outs = torch.sigmoid(beta.double()), before.double().view(heads, dk, dv), []
+    for t in range(T):
+        S = gd[t][:, :, None] * S
+        S = S + k[t][:, :, None] * (b[t][:, None] * (v[t] - torch.einsum("hdc,hd->hc", S, k[t])))[:, None, :]
+        outs.append(torch.einsum("hdc,hd->hc", S, q[t]))
+    want = torch.stack(outs).flatten(1), S.flatten()[None]
+
+    def errors(limit):
+        monkeypatch.setattr(ops, "DELTA_CHUNK_TOKENS", (limit,) * 3)
+        state = before.clone()
+        o = ops.delta_rule(ctx, qkv, (0, heads * dk, 2 * heads * dk), beta, a, a_log, dt_bias, state, heads, heads, dk, dv)
+        return [float((x.double() - w).norm() / w.norm()) for x, w in zip((o, state), want)]
+
+    for walk, chunks in zip(errors(T + 1), errors(0)):
+        assert chunks <= walk
+        # (a product that is left out shows at once: roundings of 2^-24, as many as a decay lets pile up)
+        assert chunks < (2.5e-7 if shift > -3 else 3e-6)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("y_dtype", DTYPES)
 @pytest.mark.parametrize("H", [4, 37, 1020, 1024, 1028, 2052, 4100, 8192, 8196])
 def test_norm_on_an_output_at_the_widths_its_rows_are_kept_at(H, y_dtype):
