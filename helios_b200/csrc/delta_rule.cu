@@ -8,7 +8,9 @@
 //
 // The columns of S never mix: eight threads own a column (or two), an eighth of its dk values in
 // registers each, and walk the request's tokens in order, so a request's numbers do not depend on
-// how its tokens were cut into steps or on the rest of the batch.  State, decays, gates, unit norms and
+// how its tokens were cut into steps or on the rest of the batch.  In bfloat16 that holds on each side of one
+// boundary only: long portions go by chunks of tokens (`delta_chunk.cuh`, `delta_rule_by_chunks` in ops.py says
+// which), whose sums have another order.  State, decays, gates, unit norms and
 // the recurrence are float32.
 //
 // Kernels: `causal_conv_silu` (short causal convolution over time per channel + silu, the

@@ -2282,22 +2282,31 @@ def causal_conv_silu(ctx, x: torch.Tensor, channels: int, weight: torch.Tensor,
     return out
 
 
-#: Steps whose longest portion may have this many tokens, and that have DELTA_CHUNK_MEAN a request, walk the
-#: delta rule in chunks of 16 tokens (16-bit activations, keys of at most 128 values): keys of more than 64
-#: values | fewer, blocks of 16 columns that all have an SM of their own | fewer, more blocks.
-#: By tokens / by chunks, µs, 16 heads of 128 x 128: one request of 2,048 tokens 448 / 172, of 333 77 / 37, of 64
-#: 20 / 16; 64 tokens of 32 requests 189 / 171, 32 of 16 53 / 52, 16 of 64 114 / 131; 1,000 beside 24 of one 272 /
-#: 143, 300 90 / 66.  8 heads of 64 x 64: 2,048 297 / 119, 700 of three 110 / 54, 64 13.9 / 12.2, 64 of 32 41 / 44,
-#: 1,000 beside 24 of one 190 / 95.  16 of 24 x 24: 200 29 / 20, 64 of 24 30 / 40.
-DELTA_CHUNK_TOKENS = (64, 128, 512)
+#: Steps whose longest portion has this many tokens walk the delta rule in chunks of 16 tokens (16-bit activations,
+#: keys of at most 128 values, DELTA_CHUNK_MEAN tokens a request; with more than two blocks of 16 columns an SM twice
+#: as many, unless all portions but one have a chunk on average): keys of more than 64 values, or of more than 32 and
+#: no more blocks | of more than 32 otherwise, or of up to 32 (padded to 64) and no more blocks or one long portion | of up
+#: to 32 otherwise.
+#: By tokens / by chunks, µs, 16 heads of 128 x 128: one request of 2,048 tokens 449 / 180, of 64 20.4 / 15.3, of 48
+#: 17.1 / 14.3, of 24 12.3 / 12.4; 32 requests of 128 361 / 312, of 64 190 / 177, of 48 147 / 140, of 24 84 / 104; one of
+#: 1,000 beside 24 of one 275 / 143.  8 heads of 64 x 64: one of 2,048 297 / 127, of 64 14.4 / 12.1, of 48 12.1 / 11.2; 8 of
+#: 64 18.7 / 16.1; 32 of 128 78 / 74, of 96 60 / 59, of 48 33 / 34, of 24 20 / 27; one of 1,000 beside 24 of one 190 / 96.  16
+#: of 24 x 24: one of 64 12.8 / 12.0; 8 of 64 18.5 / 18.1, of 48 15.3 / 15.5; 16 of 256 83 / 94, 32 of 128 71 / 96; one of 1,476
+#: beside 60 of one 300 / 153.
+DELTA_CHUNK_TOKENS = (64, 128, 1 << 30)
 DELTA_CHUNK_MEAN = 24
 
 
 def delta_rule_by_chunks(ctx, dtype: torch.dtype, tokens: int, heads: int, dk: int, dv: int) -> bool:
-    longest = min(getattr(ctx, "max_tokens_per_seq", 0) or tokens, tokens)
-    alone = ctx.num_seqs * heads * -(-dv // 16) <= sm_count()
-    return dtype == torch.bfloat16 and dk <= 128 and tokens >= DELTA_CHUNK_MEAN * ctx.num_seqs \
-        and longest >= DELTA_CHUNK_TOKENS[0 if dk > 64 else 1 if alone else 2]
+    if dtype != torch.bfloat16 or dk > 128 or tokens < DELTA_CHUNK_MEAN * ctx.num_seqs:
+        return False
+    mean = tokens / max(ctx.num_seqs, 1)
+    longest = getattr(ctx, "longest_portion", 0) or mean
+    one_long = tokens - longest <= 16 * (ctx.num_seqs - 1)
+    few = ctx.num_seqs * heads * -(-dv // 16) <= 2 * sm_count()
+    if not few and not one_long and mean < 2 * DELTA_CHUNK_MEAN:
+        return False
+    return longest >= DELTA_CHUNK_TOKENS[0 if dk > (32 if few else 64) else 1 if dk > 32 or few or one_long else 2]
 
 
 def delta_rule(ctx, qkv: torch.Tensor, offsets, beta_raw: torch.Tensor, a_raw: torch.Tensor,

@@ -9,7 +9,8 @@ from typing import Hashable, List, Optional, Sequence
 import torch
 
 from ..cache.manager import KVCacheManager, pool_sizes_for_bytes
-from .batch import MetaLayout, SeqSlice, StepEntry, build_context, context_from_views, fill_meta
+from .batch import (BESIDE_ONE_LONG, MetaLayout, SeqSlice, StepEntry, build_context, context_from_views, fill_meta,
+                    one_long_portion)
 from .model import DecoderModel
 
 
@@ -26,7 +27,7 @@ class _StepGraph:
     Decode steps have one token a request; mixed steps (prompt portions beside decoded
     tokens) are padded to a token count from ``EngineCore.GRAPH_TOKEN_BUCKETS``."""
 
-    def __init__(self, core: "EngineCore", num_seqs: int, num_tokens: int) -> None:
+    def __init__(self, core: "EngineCore", num_seqs: int, num_tokens: int, one_long: bool = False) -> None:
         cache, model = core.cache, core.model
         self.num_seqs, self.num_tokens = num_seqs, num_tokens
         self.decode = num_seqs == num_tokens
@@ -34,9 +35,11 @@ class _StepGraph:
         self.host = torch.empty(self.layout.total, dtype=torch.int32, pin_memory=True)
         self.dev = torch.zeros(self.layout.total, dtype=torch.int32, device=model.device)
         # what kernels are chosen by must not change from step to step: a mixed step always
-        # counts as one with long portions
+        # counts as one with long portions (how long at least, a graph of steps with ``one_long`` portion knows)
         self.ctx = context_from_views(self.layout, self.dev, [], model.dtype, model.device,
-                                      1 if self.decode else num_tokens, core.graph_max_context)
+                                      1 if self.decode else num_tokens, core.graph_max_context,
+                                      num_tokens - BESIDE_ONE_LONG * (num_seqs - 1) if one_long
+                                      else -(-num_tokens // num_seqs))
         from ..csrc import ops
         # the context slices of decode attention over keys and values (a cache with one plane of
         # rows belongs to a part that cuts its key range itself)
@@ -190,6 +193,7 @@ class EngineCore:
                                    for g in range(len(self.cache.groups))]
         self._graphs = {}
         self._bucket_seen = {}
+        self._by_longest_portion = any(getattr(part, "by_longest_portion", False) for _prefix, part in model.plan.named_parts())
         parameters = sum(_numel(spec.shape) for _prefix, part in model.plan.named_parts()
                          for spec in part.weight_specs().values())
         self.graph_token_buckets = self.GRAPH_TOKEN_BUCKETS + (
@@ -307,11 +311,19 @@ class EngineCore:
     def _graph_step(self, entries, token_feed=None):
         """(ran, logits).  A step runs as a captured graph when it fits a shape that has been
         seen before: decode steps by their padded number of requests, mixed steps by their
-        padded numbers of requests and tokens.  The first step of a shape runs kernel by
+        padded numbers of requests and tokens (and, where a part's kernels are chosen by it, whether
+        they are one long portion beside short ones).  The first step of a shape runs kernel by
         kernel; the second runs kernel by kernel on the graph's static buffers (which fixes
         what the graph will need); from the third on the graph is replayed."""
         S = len(entries)
         T = sum(len(e.tokens) for e in entries)
+        longest = max((len(e.tokens) for e in entries), default=0)
+
+        def key_of(num_seqs, num_tokens):
+            if T > S and self._by_longest_portion and one_long_portion(longest, num_tokens, num_seqs):
+                return num_seqs, num_tokens, True
+            return num_seqs, num_tokens
+
         if any(len(e.want) > 1 for e in entries):
             return False, None
         if any(self.cache.length(e.request_id) + len(e.tokens) > self.graph_max_context for e in entries):
@@ -332,13 +344,13 @@ class EngineCore:
                 fits = [b for b in self.GRAPH_FULL_TOKEN_BUCKETS if b >= T and 8 * T >= 7 * b]
                 if fits:
                     num_seqs = S if fits[0] == T else S + 1
-                    if (num_seqs, fits[0]) not in self._graphs and \
-                            sum(t > self.graph_token_buckets[-1] for _s, t in self._graphs) >= self.MAX_FULL_GRAPHS:
+                    if key_of(num_seqs, fits[0]) not in self._graphs and \
+                            sum(k[1] > self.graph_token_buckets[-1] for k in self._graphs) >= self.MAX_FULL_GRAPHS:
                         return False, None
             if not fits or fits[0] > self.graph_max_context:
                 return False, None
             num_tokens = fits[0]
-        key = (num_seqs, num_tokens)
+        key = key_of(num_seqs, num_tokens)
         g = self._graphs.get(key)
         if g is None:
             seen = self._bucket_seen.get(key, 0)
@@ -349,7 +361,7 @@ class EngineCore:
             eager_runs = 1 if num_tokens <= self.graph_token_buckets[-1] else self.FULL_GRAPH_EAGER_RUNS
             if seen < eager_runs:
                 return False, None
-            g = self._graphs[key] = _StepGraph(self, num_seqs, num_tokens)
+            g = self._graphs[key] = _StepGraph(self, *key)
         g.fill(entries, self.cache)
         if token_feed is not None:
             g.ctx.token_ids[:S].copy_(token_feed)

@@ -23,6 +23,9 @@ from .base import Mixer, StateSpec, WeightSpec, register_part
 
 
 class GatedDeltaMixer(Mixer):
+    #: the recurrence's kernel depends on ``StepContext.longest_portion``
+    by_longest_portion = True
+
     def __init__(self, width: int, heads: int, kv_heads: int, dk: int, dv: int, taps: int,
                  decay_rank: int, gate_rank: int, eps: float) -> None:
         """``decay_rank`` / ``gate_rank``: inner sizes of the two-step projections of the decay

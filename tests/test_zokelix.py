@@ -816,6 +816,52 @@ def test_delta_rule_by_chunks_of_tokens_is_the_plain_scan(dk, dv, lens, monkeypa
     assert o2[lens[0] - 1].isnan().all() and torch.equal(state2[:S], state[:S])
 
 
+@pytest.mark.parametrize("heads,dk,portions,takes", [
+    (16, 128, [64], True), (16, 128, [63], False), (16, 128, [64, 40], True), (16, 128, [47] * 8, False),
+    (16, 128, [64] + [24] * 7, False), (16, 128, [64] * 32, True), (16, 128, [1000] + [1] * 24, True),
+    (16, 128, [300] + [1] * 24, False), (16, 129, [2048], False), (8, 64, [64] * 8, True), (8, 64, [64] * 32, False),
+    (8, 64, [128] * 32, True), (8, 64, [1476] + [1] * 60, True), (16, 24, [64], False), (16, 24, [128] * 4, True),
+    (16, 24, [2048] * 20, False), (16, 24, [1000] + [1] * 24, True)])
+def test_which_portions_the_delta_rule_takes_by_chunks(heads, dk, portions, takes, monkeypatch):
+    """Eagerly, and in a captured step, which knows only whether there is one long portion beside short ones."""
+    from types import SimpleNamespace
+    from helios_b200.csrc import ops
+    from helios_b200.engine.batch import one_long_portion
+
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    T, S = sum(portions), len(portions)
+    for dtype in (torch.bfloat16, torch.float32):
+        ctx = SimpleNamespace(num_seqs=S, longest_portion=max(portions))
+        assert ops.delta_rule_by_chunks(ctx, dtype, T, heads, dk, dk) == (takes and dtype == torch.bfloat16)
+    known = T - 16 * (S - 1) if one_long_portion(max(portions), T, S) else -(-T // S)
+    ctx = SimpleNamespace(num_seqs=S, longest_portion=known)
+    assert ops.delta_rule_by_chunks(ctx, torch.bfloat16, T, heads, dk, dk) == (takes and portions != [64, 40])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("portions", [[70, 1, 1, 1], [24, 24, 24, 24]])
+def test_captured_steps_take_the_delta_rule_as_the_same_steps_run_kernel_by_kernel(zk_folders, portions, monkeypatch):
+    from helios_b200.csrc import ops
+    from helios_b200.engine.batch import StepEntry
+
+    rule, routes = ops.delta_rule_by_chunks, []
+    monkeypatch.setattr(ops, "DELTA_CHUNK_TOKENS", (50, 50, 50))
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MEAN", 16)
+
+    def noted(*args):
+        routes.append(rule(*args))
+        return routes[-1]
+
+    monkeypatch.setattr(ops, "delta_rule_by_chunks", noted)
+    core = _core(zk_folders["zk_a"], "bfloat16", 600, max_slots=5)
+    for i in range(4):
+        core.step([StepEntry((i, j), tuple(k % 20 for k in range(n)), (n - 1,)) for j, n in enumerate(portions)])
+        for j in range(len(portions)):
+            core.end((i, j))
+    assert any(g.graph is not None for g in core._graphs.values())
+    assert set(routes) == {portions[0] == 70}
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("shift", [4.0, 0.0, -2.0, -10.0])
 @pytest.mark.parametrize("dk,dv", [(64, 64), (128, 128)])
