@@ -816,6 +816,61 @@ def test_delta_rule_by_chunks_of_tokens_is_the_plain_scan(dk, dv, lens, monkeypa
     assert o2[lens[0] - 1].isnan().all() and torch.equal(state2[:S], state[:S])
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[300, 0, 130, 17], [17, 64, 0, 65, 130, 300]], ids=["one_group", "two_groups"])
+@pytest.mark.parametrize("dk,dv", [(64, 128), (40, 116), (128, 128), (100, 116)])
+def test_delta_rule_by_chunks_walks_its_ring_of_chunks_around(dk, dv, lens, monkeypatch):
+    """More chunks than stages, with blocks of one and of two column groups; requests without tokens; q, k, v, beta, a
+    and the states as columns of wider rows, as a model passes them; the same bits twice."""
+    from types import SimpleNamespace
+    from helios_b200.csrc import ops
+
+    monkeypatch.setattr(ops, "DELTA_CHUNK_TOKENS", (0, 0, 0))
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MEAN", 0)
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    dev, heads, S, T = "cuda", 4, len(lens), sum(lens)
+    assert (S * heads * -(-dv // 16) <= 148) == (S == 4)
+    g = torch.Generator(device=dev).manual_seed(dk + dv + S)
+    r = lambda *s: torch.randn(*s, generator=g, device=dev)
+    qkv = torch.nn.functional.silu(r(T, 24 + heads * (2 * dk + dv))).bfloat16()
+    wide = (r(T, heads * dk + 40) - 1).bfloat16()
+    beta, a = wide[:, 3:3 + heads], wide[:, 17:17 + heads * dk]
+    a_log, dt_bias, rows = r(heads) * 0.3, r(heads * dk) * 0.3, r(S + 2, heads * dk * dv + 12) * 0.3
+    slots = list(range(S, 0, -1))
+    ctx = SimpleNamespace(cu_tokens=torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).int().to(dev),
+                          slots=torch.tensor(slots, dtype=torch.int32, device=dev), num_seqs=S)
+    at = (8, 8 + heads * dk, 24 + 2 * heads * dk)
+
+    def run():
+        kept = rows.clone()
+        return ops.delta_rule(ctx, qkv, at, beta, a, a_log, dt_bias, kept[:, :heads * dk * dv], heads, heads, dk, dv), kept
+
+    (got, kept), again = run(), run()
+    assert torch.equal(got, again[0]) and torch.equal(kept, again[1])
+    idle = [0, S + 1] + [slots[i] for i in range(S) if lens[i] == 0]
+    assert torch.equal(kept[idle], rows[idle]) and torch.equal(kept[:, heads * dk * dv:], rows[:, heads * dk * dv:])
+    q, k, v = (qkv.double()[:, c:c + heads * n].view(T, heads, n) for c, n in zip(at, (dk, dk, dv)))
+    q = q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * dk ** -0.5
+    k = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    gd = torch.exp(-torch.exp(a_log.double())[:, None] * torch.nn.functional.softplus(
+        (a.double() + dt_bias.double()).view(T, heads, dk)))
+    b, first = torch.sigmoid(beta.double()), 0
+    for n, slot in zip(lens, slots):
+        state, outs = rows[slot, :heads * dk * dv].double().view(heads, dk, dv), []
+        for t in range(first, first + n):
+            state = gd[t][:, :, None] * state
+            u = b[t][:, None] * (v[t] - torch.einsum("hdc,hd->hc", state, k[t]))
+            state = state + k[t][:, :, None] * u[:, None, :]
+            outs.append(torch.einsum("hdc,hd->hc", state, q[t]).flatten())
+        # relative 2-norms: some roundings of 2^-24 a token, which decays of 0.8 forget
+        bound = 3e-7
+        if n:
+            o = torch.stack(outs)
+            assert (got[first:first + n].double() - o).norm() < bound * o.norm()
+        assert (kept[slot, :heads * dk * dv].double() - state.flatten()).norm() < bound * state.norm()
+        first += n
+
+
 @pytest.mark.parametrize("heads,dk,portions,takes", [
     (16, 128, [64], True), (16, 128, [63], False), (16, 128, [64, 40], True), (16, 128, [47] * 8, False),
     (16, 128, [64] + [24] * 7, False), (16, 128, [64] * 32, True), (16, 128, [1000] + [1] * 24, True),
