@@ -526,9 +526,9 @@ def silu_mul(gate_up: torch.Tensor) -> torch.Tensor:
 
 # ------------------------------------------------------------------ matrix products
 #: rows of x up to which the float32 product streams the weight through the kernel for few rows
-#: (eight at a time; of a weight of 2,048 rows or more only up to eight).  Tiles / rows, microseconds, at
-#: 12 rows: 896 x 4,864 32 / 26; 1,152 x 896 9.2 / 7.9; 896 x 896 8.7 / 7.4; at 16 rows 32 / 34, 9.2 / 9.3,
-#: 8.7 / 7.9
+#: (six or eight at a time; of a weight of 2,048 rows or more only up to eight, of more than 1,024 up to twelve).
+#: Tiles / rows, microseconds, at 12 rows: 896 x 4,864 32 / 19; 1,152 x 896 9.0 / 8.3; 896 x 896 8.9 / 6.9; at 16 rows
+#: 896 x 4,864 32 / 26, 896 x 896 8.9 / 7.9, 1,024 x 4,096 27 / 23
 GEMM_F32_FEW_ROWS = 16
 #: the form of those kernels, 0: by size (``hb_gemm_f32_as``); the results are the same
 GEMM_F32_FORM = 0

@@ -842,3 +842,26 @@ def test_gemm_f32_in_every_form_is_the_same_bit_for_bit(M, N, K, monkeypatch):
     # runs of 8 + 8, up to K / 64 runs a quarter, four quarters and the bias: as many roundings of a product's size
     bound = (K / 64 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs())
     assert ((got.double().cpu() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("M", [1, 9, 33, 65, 200])
+@pytest.mark.parametrize("N,K", [(65, 4), (100, 32), (130, 64), (65, 96), (70, 128), (64, 516), (65, 17), (130, 50), (70, 333), (64, 1001)])
+def test_gemm_f32_tiles_with_a_quarter_and_with_all_of_k_a_block(M, N, K, monkeypatch):
+    """One to four quarters that are not empty, rows in 16-byte pieces and not, ends inside both tiles; zeros with
+    their sign."""
+    o = ops()
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g), torch.randn(N, generator=g)
+    x[0], w[1], b[2:9] = -0.0, w[1].abs(), -0.0
+    xd, wd, bd = x.to(DEV), w.to(DEV), b.to(DEV)
+    want = x.double() @ w.double().T + b.double()
+    bound = (K / 64 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs())
+    for bias in (bd, None):
+        few = o.linear_f32(xd, wd, bias)
+        monkeypatch.setattr(o, "GEMM_F32_FEW_ROWS", 0)
+        for form in (0, 44, 84, 441, 444, 841, 844):
+            monkeypatch.setattr(o, "GEMM_F32_FORM", form)
+            assert torch.equal(o.linear_f32(xd, wd, bias).view(torch.int32), few.view(torch.int32)), form
+        monkeypatch.undo()
+        if bias is bd:
+            assert ((few.double().cpu() - want).abs() <= bound).all()
