@@ -76,8 +76,8 @@ __device__ __forceinline__ float dc_decay(float a, float rate_hi, float rate_lo)
 // One block a (chunk, head).  Bound by its instructions: 256 dot products over dk with a running product of
 // decays each, and the splitting.  Sixteen threads a dot product, the pairs (i, j) of two rows j and 15 - j by the
 // same threads, so that all walk 17; the sums of four rows i go over the lanes together, eight shuffles for 32.  Six
-// blocks an SM (80 registers): with the walk, 2,048 tokens of 16 heads of 128 x 128, 185 -> 178 µs (four 179, eight
-// with their spills 188).
+// blocks an SM (80 registers; four 1 % slower with the walk, eight, with their spills, 6 %).  Under ncu, 2,048 tokens of 16
+// heads of 128 x 128: 51 µs, issue slots 65 % busy, the way from shared memory 64 %, the 64-bit pipe 2 %.
 template <typename T, int DK>
 __global__ void __launch_bounds__(128, 6)
 delta_chunk_prepare_kernel(uint32_t* __restrict__ chunks, const T* __restrict__ qkv, int qkv_ld, int q_off, int k_off,
@@ -298,7 +298,7 @@ __device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], co
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
 }
 // the six products of two factors of three planes each, by size: sums[0] += a0 b0, ...; of two results in turn, so
-// that a product's sums are there when the next one adds to them (one result after the other waited 28 of 79 cycles)
+// that a product's sums are there when the next one adds to them
 __device__ __forceinline__ void dc_mma_split(float (&x)[3][4], float (&y)[3][4], const uint32_t (&a)[3][4],
                                              const uint32_t* frag_x, const uint32_t* frag_y, int lane) {
   uint2 b[3], c[3];
@@ -339,10 +339,9 @@ struct DeltaChunkSmem {
 // quarter of dk each (columns of S on the rows of the fragment), which are as they stand the A operand of S^T Kc and
 // S^T Qc.  The other four own the solution: four columns each, two tokens of a column a thread.  A chunk's
 // chain is S^T Kc -> barrier -> sums of the four quarters, U = T R -> barrier -> the write into S; S^T Qc runs beside
-// the solution, the outputs and the copies beside the write.  Bound by that chain, a microsecond
-// a chunk (1.05 before the products of two tiles ran in turn and the next chunk's planes were made beside the
-// write: 185 -> 180 µs of 2,048 tokens); eight
-// warps of 16 dk each instead of four take as long (and 5 % longer where blocks share SMs).
+// the solution, the outputs and the copies beside the write.  Bound by that chain, 1,880 cycles
+// a chunk under ncu (2,048 tokens, 16 heads of 128 x 128: 143 µs, issue slots 47 % busy, tensor pipe 31 %, the way from
+// shared memory 49 %); eight warps of 16 dk each instead of four take as long (and 5 % longer where blocks share SMs).
 template <typename T, int DK, int GROUPS, int STAGES>
 __global__ void __launch_bounds__(GROUPS * DC_GROUP_THREADS)
 delta_chunk_kernel(float* __restrict__ o, const uint32_t* __restrict__ chunks, const T* __restrict__ qkv, int qkv_ld,

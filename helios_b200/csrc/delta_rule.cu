@@ -859,7 +859,9 @@ HB_EXPORT int hb_delta_chunk_words(int dk) {
   return dk <= 0 || dk > 128 ? 0 : dk <= 64 ? DeltaChunk<64>::WORDS : DeltaChunk<128>::WORDS;
 }
 
-// scratch: dc_chunks(n_tokens, n_seqs) * heads * hb_delta_chunk_words(dk) words, 16-byte aligned
+// scratch: dc_chunks(n_tokens, n_seqs) * heads * hb_delta_chunk_words(dk) words, 16-byte aligned.  39,936 bytes a chunk and
+// head of 128 values, 2,496 a token where `hb_delta_rule` takes 1,544; a request of one token takes a whole chunk, so the
+// callers ask for 24 tokens a request (at most 4.2 KB a token and head).
 HB_EXPORT int hb_delta_chunk(float* o, uint32_t* scratch, const void* qkv, int qkv_ld, int q_off, int k_off,
                              int v_off, const void* beta_raw, int beta_ld, const void* a_raw, int a_ld,
                              const float* a_log, const float* dt_bias, float* state,

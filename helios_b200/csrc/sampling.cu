@@ -188,7 +188,8 @@ sample_kernel(int* __restrict__ out, const float* __restrict__ logits, int V, in
 // one row 81 / 25; top-p 0.95 of 64 rows N(0, 1), 60,000 tokens kept, 452 / 149.  Eight rows, search of
 // whole keys alone / list tried in vain, then that search / this: top-k 2,000 and top-p 0.9 of N(0, 4)
 // 111 / 141 / 101; top-k 2,000 of whole numbers 48 / 80 / 50; top-k 50 of equal values 39 / 71 / 50.
-// Bound by instructions and barriers: 16 warps a block, three blocks an SM.  So rows come in 16-byte pieces and the argmax
+// Bound by instructions and barriers: 16 warps a block, three blocks an SM (two for rows of more than 131,072 values,
+// which take 84 KB a block).  So rows come in 16-byte pieces and the argmax
 // with them, fifteen sums of a warp take 16 exchanges, and a value is compared with a level only where it lies
 // above the next lower one: 64 rows N(0, 4) of mixed options 50.8 -> 45.7.
 constexpr int SC_THREADS = 512;
