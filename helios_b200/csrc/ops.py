@@ -2302,7 +2302,7 @@ def delta_rule_by_chunks(ctx, dtype: torch.dtype, tokens: int, heads: int, dk: i
         return False
     mean = tokens / max(ctx.num_seqs, 1)
     longest = getattr(ctx, "longest_portion", 0) or mean
-    one_long = tokens - longest <= 16 * (ctx.num_seqs - 1)
+    one_long = getattr(ctx, "one_long", ctx.num_seqs == 1)
     few = ctx.num_seqs * heads * -(-dv // 16) <= 2 * sm_count()
     if not few and not one_long and mean < 2 * DELTA_CHUNK_MEAN:
         return False

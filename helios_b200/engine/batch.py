@@ -55,8 +55,10 @@ class StepContext:
     decode_only: bool = False
     max_tokens_per_seq: int = 0
     max_context_len: int = 0
-    # tokens that the longest portion has at least, in every run of a captured step
+    # tokens that the longest portion has at least, in every run of a captured step, and whether the
+    # others are short beside it
     longest_portion: int = 0
+    one_long: bool = False
     # left by the plan's position encoding for the mixers that were given none of their own
     rotary_cos: Optional[torch.Tensor] = None
     rotary_sin: Optional[torch.Tensor] = None
@@ -227,18 +229,23 @@ def fill_meta(layout: MetaLayout, host: np.ndarray, entries: Sequence[StepEntry]
     return seqs
 
 
-#: tokens that the portions beside ONE long one have on average at most
-BESIDE_ONE_LONG = 16
-
-
 def one_long_portion(longest: int, tokens: int, requests: int) -> bool:
-    """Whether a step is one long portion beside short ones (decoding requests, mostly)."""
-    return tokens - longest <= BESIDE_ONE_LONG * (requests - 1)
+    """Whether a step is one long portion beside short ones (decoding requests, mostly): at most 16
+    tokens on average."""
+    return tokens - longest <= 16 * (requests - 1)
+
+
+def long_class(longest: int, tokens: int, requests: int) -> int:
+    """What a captured step may know of its one long portion: 128 tokens at least, or 64; 0: there is
+    none."""
+    if not one_long_portion(longest, tokens, requests):
+        return 0
+    return 128 if longest >= 128 else 64 if longest >= 64 else 0
 
 
 def context_from_views(layout: MetaLayout, dev: torch.Tensor, seqs: List[SeqSlice],
                        act_dtype: torch.dtype, device: torch.device, max_tokens_per_seq: int,
-                       max_context_len: int, longest_portion: int) -> StepContext:
+                       max_context_len: int, longest_portion: int, one_long: bool) -> StepContext:
     v = layout.device_views(dev)
     return StepContext(
         act_dtype=act_dtype, device=device, num_tokens=layout.T, num_seqs=layout.S,
@@ -246,7 +253,8 @@ def context_from_views(layout: MetaLayout, dev: torch.Tensor, seqs: List[SeqSlic
         cu_tokens=v[3], start_pos=v[4], context_len=v[5], slots=v[6], want_rows=v[7],
         block_tables=[t.view(layout.S, w) for t, w in zip(v[8:], layout.widths)],
         decode_only=(max_tokens_per_seq == 1), max_tokens_per_seq=max_tokens_per_seq,
-        max_context_len=max_context_len, longest_portion=longest_portion)
+        max_context_len=max_context_len, longest_portion=longest_portion,
+        one_long=one_long)
 
 
 def build_context(entries: Sequence[StepEntry], cache, act_dtype: torch.dtype,
@@ -264,4 +272,5 @@ def build_context(entries: Sequence[StepEntry], cache, act_dtype: torch.dtype,
     dev = host.to(device, non_blocking=True)
     n_max = max((len(e.tokens) for e in entries), default=0)
     max_ctx = max((s.start_pos + s.num_tokens for s in seqs), default=0)
-    return context_from_views(layout, dev, seqs, act_dtype, device, n_max, max_ctx, n_max)
+    return context_from_views(layout, dev, seqs, act_dtype, device, n_max, max_ctx, n_max,
+                              one_long_portion(n_max, T, S))

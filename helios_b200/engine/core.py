@@ -9,8 +9,7 @@ from typing import Hashable, List, Optional, Sequence
 import torch
 
 from ..cache.manager import KVCacheManager, pool_sizes_for_bytes
-from .batch import (BESIDE_ONE_LONG, MetaLayout, SeqSlice, StepEntry, build_context, context_from_views, fill_meta,
-                    one_long_portion)
+from .batch import MetaLayout, SeqSlice, StepEntry, build_context, context_from_views, fill_meta, long_class
 from .model import DecoderModel
 
 
@@ -27,7 +26,7 @@ class _StepGraph:
     Decode steps have one token a request; mixed steps (prompt portions beside decoded
     tokens) are padded to a token count from ``EngineCore.GRAPH_TOKEN_BUCKETS``."""
 
-    def __init__(self, core: "EngineCore", num_seqs: int, num_tokens: int, one_long: bool = False) -> None:
+    def __init__(self, core: "EngineCore", num_seqs: int, num_tokens: int, one_long: int = 0) -> None:
         cache, model = core.cache, core.model
         self.num_seqs, self.num_tokens = num_seqs, num_tokens
         self.decode = num_seqs == num_tokens
@@ -35,11 +34,10 @@ class _StepGraph:
         self.host = torch.empty(self.layout.total, dtype=torch.int32, pin_memory=True)
         self.dev = torch.zeros(self.layout.total, dtype=torch.int32, device=model.device)
         # what kernels are chosen by must not change from step to step: a mixed step always
-        # counts as one with long portions (how long at least, a graph of steps with ``one_long`` portion knows)
+        # counts as one with long portions (``one_long``: `long_class` of its steps)
         self.ctx = context_from_views(self.layout, self.dev, [], model.dtype, model.device,
                                       1 if self.decode else num_tokens, core.graph_max_context,
-                                      num_tokens - BESIDE_ONE_LONG * (num_seqs - 1) if one_long
-                                      else -(-num_tokens // num_seqs))
+                                      one_long or -(-num_tokens // num_seqs), one_long > 0)
         from ..csrc import ops
         # the context slices of decode attention over keys and values (a cache with one plane of
         # rows belongs to a part that cuts its key range itself)
@@ -320,9 +318,9 @@ class EngineCore:
         longest = max((len(e.tokens) for e in entries), default=0)
 
         def key_of(num_seqs, num_tokens):
-            if T > S and self._by_longest_portion and one_long_portion(longest, num_tokens, num_seqs):
-                return num_seqs, num_tokens, True
-            return num_seqs, num_tokens
+            # (the padding requests count as short ones, whatever the last of them is given)
+            long = long_class(longest, T, num_seqs) if T > S and self._by_longest_portion else 0
+            return (num_seqs, num_tokens, long) if long else (num_seqs, num_tokens)
 
         if any(len(e.want) > 1 for e in entries):
             return False, None
